@@ -64,37 +64,45 @@ void launch_p2m_tc(Ctx& c, const DevPlan& p, const int32_t* slot, const float* W
 // FP64 M2L of one level with CUDA-core FMAs (dense operators).
 void launch_m2l64(Ctx& c, const DevPlan& p, int b0, int nb, double* L, const double* E, int R, double scale);
 
-// Factored M2L data (orders 4-6, ranks <= kFacMaxRank): low-rank factors of
-// every offset, per-source column lists for phase 1 and per-target B-row lists
-// for phase 2.
+// Factored M2L data (ranks <= kFacMaxRank): low-rank factors of every offset
+// and, per box pair, its place in the source's and the target's columns
+// (m2l_fac.cu).
 constexpr int kFacMaxRank = 32;
+// Phase-1 work items: a source box and a run of its outgoing pairs with at
+// most kFacItemCols summed ranks.
+constexpr int kFacItemCols = 512;
+struct FacItem {
+    int32_t src;
+    int32_t p0, p1;  // pairs [p0, p1) of the source-major list
+};
 template <class T>
 struct FacM2L {
     int ns = 64;                        // node stride
+    int nitems = 0;
+    int max_cols = 0;                   // largest summed rank of a target box
+    const FacItem* items = nullptr;
     const T* Vt = nullptr;              // 343 x 32 x ns, row k of slot o = Vt_o[k][:]
     const T* Ut = nullptr;              // 343 x 32 x ns, row k of slot o = U_o[:][k]
-    const int64_t* src_col_off = nullptr;  // nbox + 1: phase-1 columns of each source box
-    const int64_t* col_vt = nullptr;    // per column: offset of its Vt row
-    const int32_t* col_tgt = nullptr;   // per column: target box
-    const int32_t* col_pos = nullptr;   // per column: column in the target's T block
-    const int64_t* tgt_col_off = nullptr;  // nbox + 1: phase-2 contraction range of each target
-    const int64_t* tgt_ut = nullptr;    // per contraction index: offset of its Ut row
-    const int64_t* tgt_base = nullptr;  // nbox: sum of padded block widths of earlier boxes
-    T* Tm = nullptr;                    // target-major intermediate (Kp columns of R values per target)
-    const double* box_scale = nullptr;  // per box: 1 / half-width of its level (all-levels launches)
+    const int32_t* rank = nullptr;      // per slot
+    const int32_t* src_slot = nullptr;  // source-major pair list: operator slot,
+    const int64_t* src_col = nullptr;   // summed ranks of the pairs before it (one more entry than pairs),
+    const int64_t* src_trow = nullptr;  // and the T row of its first column
+    const int64_t* m2l_off = nullptr;   // nbox + 1: pairs of each target box (the plan's list)
+    const int32_t* m2l_slot = nullptr;  // per pair
+    const int32_t* tgt_col = nullptr;   // per pair: its first column within the target
+    const int64_t* tgt_col_off = nullptr;  // nbox + 1: summed ranks of the targets before
+    const int64_t* tgt_base = nullptr;  // nbox: first T row (each target's columns rounded up to 4)
+    T* Tm = nullptr;                    // target-major intermediate (R values per column)
+    const double* box_scale = nullptr;  // per box: 1 / half-width of its level
 };
-// Phase-1 work items of one level: (source box, first column, column count <= kFacItemCols).
-constexpr int kFacItemCols = 512;
-struct FacLevel {
-    int nitems = 0;
-    const int32_t* item_src = nullptr;
-    const int64_t* item_c0 = nullptr;
-    const int32_t* item_cnt = nullptr;
-};
-// M2L of one level with the factored operators (two kernels).
+// L of the boxes [b0, b0 + nb), levels 2 and deeper, = M2L of E (two kernels);
+// boxes without pairs get zero.  n3: nodes of an expansion (<= ns).
 template <class T>
-void launch_m2l_fac(Ctx& c, const FacM2L<T>& f, const FacLevel& lv, int b0, int nb, T* L, const T* E, int R,
-                    double scale);
+void launch_m2l_fac(Ctx& c, const FacM2L<T>& f, int b0, int nb, T* L, const T* E, int R, int n3);
+template <>
+void launch_m2l_fac<double>(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, const double* E, int R, int n3);
+template <>
+void launch_m2l_fac<float>(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const float* E, int R, int n3);
 
 // Tensor-core (tcgen05, TF32 inputs, FP32 accumulation) M2L work list of one
 // level: pairs of target boxes sharing one offset loop.

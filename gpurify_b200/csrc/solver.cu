@@ -135,7 +135,7 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
     }
     d->d_rank.upload(host.rank, ctx.stream);
     for (int32_t r : host.rank) d->max_rank = std::max(d->max_rank, (int)r);
-    if (mode == GPX_M2L_COMPRESSED && n >= 4 && n <= 6 && d->max_rank <= kFacMaxRank) {
+    if (mode == GPX_M2L_COMPRESSED && d->max_rank <= kFacMaxRank) {
         // factored tables: Vt rows and transposed U rows, kFacMaxRank rows of
         // node stride ns per slot (rows beyond the rank and padding nodes zero)
         const int n3 = n * n * n, ns = node_stride(n), KR = kFacMaxRank;
@@ -153,8 +153,10 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
                 }
         d->Ut64.upload(ut, ctx.stream);
         d->Vt64.upload(vt, ctx.stream);
-        d->Ut32.upload(ut32, ctx.stream);
-        d->Vt32.upload(vt32, ctx.stream);
+        if (n >= 4) {  // the mixed path runs orders 4 to 6
+            d->Ut32.upload(ut32, ctx.stream);
+            d->Vt32.upload(vt32, ctx.stream);
+        }
         d->factored_ok = true;
     }
     if (n == 4 || n == 5) {
@@ -451,15 +453,12 @@ struct Operator {
     DBuf<float> Eh32, Lh32; // compressed expansions, nbox x Rb32 x kShared
     FacM2L<double> fac64;
     FacM2L<float> fac32;
-    DBuf<int64_t> src_col_off, col_vt, tgt_col_off, tgt_ut, tgt_base;
-    DBuf<int32_t> col_tgt, col_pos;
+    DBuf<int64_t> src_col, src_trow, tgt_col_off, tgt_base;
+    DBuf<int32_t> src_slot, tgt_col;
+    DBuf<FacItem> fac_items;
     DBuf<double> T64;
     DBuf<float> T32;
-    std::vector<FacLevel> fac_level;
-    FacLevel fac_all;
     DBuf<double> box_scale;
-    DBuf<int32_t> fi_src, fi_cnt;
-    DBuf<int64_t> fi_c0;
     int Rb32 = 0;
     double t_assembly_s = 0.0;
     int64_t applies = 0, applies32 = 0;
@@ -674,112 +673,83 @@ struct Operator {
         finish();
     }
 
-    // Column lists of the factored M2L: phase 1 per source box, phase 2 per
-    // target box (see farfield.cu).
+    // Pair lists of the factored M2L (see m2l_fac.cu): phase 1 by source box,
+    // phase 2 by target box.
     void setup_factored() {
         const int64_t np = pl.m2l_pairs(), nb = pl.nbox();
-        const int ns = node_stride(pl.n);
         const std::vector<int32_t>& rank = m2l->rank;  // host copy: no device round trip
-        std::vector<int64_t> tcol(nb + 1, 0), base(nb, 0), pos_of_pair(np);
-        std::vector<int32_t> tgt_of_pair(np);
-        int64_t acc = 0;
+        std::vector<int64_t> tcol(nb + 1, 0), base(nb, 0), first(nb + 1, 0);
+        std::vector<int32_t> tc_e(np);
+        int64_t acc = 0, max_cols = 0;
         for (int64_t b = 0; b < nb; ++b) {
-            int64_t k = 0;
+            int32_t k = 0;
             for (int64_t e = pl.m2l_off[b]; e < pl.m2l_off[b + 1]; ++e) {
-                pos_of_pair[e] = k;
-                tgt_of_pair[e] = (int32_t)b;
+                tc_e[e] = k;
                 k += rank[pl.m2l_slot[e]];
+                first[pl.m2l_src[e] + 1] += 1;
             }
             tcol[b + 1] = tcol[b] + k;
             base[b] = acc;
-            acc += (k + 3) & ~int64_t(3);
+            acc += (k + 3) & ~3;
+            max_cols = std::max<int64_t>(max_cols, k);
         }
-        std::vector<int64_t> ut(tcol[nb]);
-        for (int64_t b = 0; b < nb; ++b) {
-            int64_t j = tcol[b];
-            for (int64_t e = pl.m2l_off[b]; e < pl.m2l_off[b + 1]; ++e)
-                for (int k = 0; k < rank[pl.m2l_slot[e]]; ++k)
-                    ut[j++] = ((int64_t)pl.m2l_slot[e] * kFacMaxRank + k) * ns;
-        }
-        // phase-1 columns grouped by source box
-        std::vector<int64_t> scol(nb + 1, 0);
-        for (int64_t e = 0; e < np; ++e) scol[pl.m2l_src[e] + 1] += rank[pl.m2l_slot[e]];
-        for (int64_t b = 0; b < nb; ++b) scol[b + 1] += scol[b];
-        std::vector<int64_t> cvt(scol[nb]), fill(scol.begin(), scol.end() - 1);
-        std::vector<int32_t> ctg(scol[nb]), cps(scol[nb]);
-        for (int64_t e = 0; e < np; ++e) {
-            const int s = pl.m2l_src[e], slot = pl.m2l_slot[e];
-            for (int k = 0; k < rank[slot]; ++k) {
-                const int64_t c = fill[s]++;
-                cvt[c] = ((int64_t)slot * kFacMaxRank + k) * ns;
-                ctg[c] = tgt_of_pair[e];
-                cps[c] = (int32_t)(pos_of_pair[e] + k);
+        for (int64_t b = 0; b < nb; ++b) first[b + 1] += first[b];
+        // the same pairs by source box
+        std::vector<int32_t> sslot(np);
+        std::vector<int64_t> scol(np + 1), strow(np), fill(first.begin(), first.end() - 1);
+        for (int64_t b = 0; b < nb; ++b)
+            for (int64_t e = pl.m2l_off[b]; e < pl.m2l_off[b + 1]; ++e) {
+                const int64_t q = fill[pl.m2l_src[e]]++;
+                sslot[q] = pl.m2l_slot[e];
+                strow[q] = base[b] + tc_e[e];
             }
-        }
-        // phase-1 work items per level: each source box's columns in pieces of
-        // at most kFacItemCols (one CTA stages the source expansion once per piece)
-        std::vector<int32_t> isrc, icnt;
-        std::vector<int64_t> ic0;
-        std::vector<int> lvl_first(pl.L + 2, 0);
-        for (int l = 0; l <= pl.L; ++l) {
-            lvl_first[l] = (int)isrc.size();
-            for (int32_t b = pl.lvl_off[l]; b < pl.lvl_off[l + 1]; ++b)
-                for (int64_t c = scol[b]; c < scol[b + 1]; c += kFacItemCols) {
-                    isrc.push_back(b);
-                    ic0.push_back(c);
-                    icnt.push_back((int32_t)std::min<int64_t>(kFacItemCols, scol[b + 1] - c));
-                }
-        }
-        lvl_first[pl.L + 1] = (int)isrc.size();
+        scol[0] = 0;
+        for (int64_t q = 0; q < np; ++q) scol[q + 1] = scol[q] + rank[sslot[q]];
+        // Phase-1 items: runs of a source's pairs of at most `cap` columns.  A
+        // run of 512 stages the source's expansion once for 16 blocks of 32
+        // columns; where that would leave SMs idle (fewer than eight CTAs
+        // each), shorter runs spread the work.
+        const int64_t cap = scol[np] / kFacItemCols >= 8 * 148 ? kFacItemCols : 128;
+        std::vector<FacItem> items;
+        for (int64_t b = 0; b < nb; ++b)
+            for (int64_t p = first[b]; p < first[b + 1];) {
+                const int64_t p0 = p;
+                while (p < first[b + 1] && scol[p + 1] - scol[p0] <= cap) ++p;
+                items.push_back({(int32_t)b, (int32_t)p0, (int32_t)p});
+            }
         cudaStream_t s = ctx.stream;
-        fi_src.upload(isrc, s);
-        fi_cnt.upload(icnt, s);
-        fi_c0.upload(ic0, s);
-        fac_level.assign(pl.L + 1, FacLevel());
-        for (int l = 0; l <= pl.L; ++l) {
-            FacLevel& fl = fac_level[l];
-            fl.nitems = lvl_first[l + 1] - lvl_first[l];
-            fl.item_src = fi_src.p + lvl_first[l];
-            fl.item_c0 = fi_c0.p + lvl_first[l];
-            fl.item_cnt = fi_cnt.p + lvl_first[l];
-        }
-        // all levels in one launch: the phase-1 items of levels 2..L, and the
-        // M2L scale 1/half of each box's level
-        const int lf = std::min(2, pl.L + 1);
-        fac_all.nitems = lvl_first[pl.L + 1] - lvl_first[lf];
-        fac_all.item_src = fi_src.p + lvl_first[lf];
-        fac_all.item_c0 = fi_c0.p + lvl_first[lf];
-        fac_all.item_cnt = fi_cnt.p + lvl_first[lf];
-
-        src_col_off.upload(scol, s);
-        col_vt.upload(cvt, s);
-        col_tgt.upload(ctg, s);
-        col_pos.upload(cps, s);
+        fac_items.upload(items, s);
+        src_slot.upload(sslot, s);
+        src_col.upload(scol, s);
+        src_trow.upload(strow, s);
+        tgt_col.upload(tc_e, s);
         tgt_col_off.upload(tcol, s);
-        tgt_ut.upload(ut, s);
         tgt_base.upload(base, s);
         auto wire = [&](auto& f) {
-            f.ns = ns;
-            f.box_scale = box_scale.p;
-            f.src_col_off = src_col_off.p;
-            f.col_vt = col_vt.p;
-            f.col_tgt = col_tgt.p;
-            f.col_pos = col_pos.p;
+            f.ns = node_stride(pl.n);
+            f.nitems = (int)items.size();
+            f.max_cols = (int)max_cols;
+            f.items = fac_items.p;
+            f.rank = m2l->d_rank.p;
+            f.src_slot = src_slot.p;
+            f.src_col = src_col.p;
+            f.src_trow = src_trow.p;
+            f.m2l_off = d.v.m2l_off;
+            f.m2l_slot = d.v.m2l_slot;
+            f.tgt_col = tgt_col.p;
             f.tgt_col_off = tgt_col_off.p;
-            f.tgt_ut = tgt_ut.p;
             f.tgt_base = tgt_base.p;
+            f.box_scale = box_scale.p;
         };
         wire(fac64);
         wire(fac32);
         T64.alloc((size_t)acc * R, s);
-        T64.zero();  // padding columns stay zero
         fac64.Tm = T64.p;
         fac64.Ut = m2l->Ut64.p;
         fac64.Vt = m2l->Vt64.p;
         if (mixed) {  // also with the tensor-core M2L: the stall guard may switch to this form
             Rb32 = (R + 63) / 64 * 64;
             T32.alloc((size_t)acc * Rb32, s);
-            T32.zero();
             fac32.Tm = T32.p;
             fac32.Ut = m2l->Ut32.p;
             fac32.Vt = m2l->Vt32.p;
@@ -795,28 +765,26 @@ struct Operator {
     void apply_direct(const double* X, double* Y) {
         launch_near_apply(ctx, d.v, pl.nnz(), P.p, X, Y, R);
         if (has_far()) {
-            M2LLevelFn<double> m2l_fn = [&](int level, int b0, int nb, double scale) {
-                if (factored)
-                    launch_m2l_fac<double>(ctx, fac64, level < 0 ? fac_all : fac_level[level], b0, nb, L64.p, E64.p,
-                                           R, scale);
-                else
-                    launch_m2l64(ctx, d.v, b0, nb, L64.p, E64.p, R, scale);
-            };
-            launch_far_field<double>(ctx, d.v, d.far, X, w64, Y, R, R, E64.p, L64.p, kCoulomb, m2l_fn, factored);
+            M2LLevelFn<double> m2l_fn = [&](int, int b0, int nb, double scale) { m2l64(b0, nb, scale); };
+            launch_far_field<double>(ctx, d.v, d.far, X, w64, Y, R, R, E64.p, L64.p, kCoulomb, m2l_fn, factored, nullptr,
+                                     factored);
         }
+    }
+    // FP64 M2L: the factored form covers every level at once and overwrites L;
+    // the dense form (exact operators) runs per level and adds to it.
+    void m2l64(int b0, int nb, double scale) {
+        if (factored)
+            launch_m2l_fac<double>(ctx, fac64, b0, nb, L64.p, E64.p, R, pl.n3);
+        else
+            launch_m2l64(ctx, d.v, b0, nb, L64.p, E64.p, R, scale);
     }
 
     // Y += far field of X with the given end weights (FP64).
     void apply_far_with(const double* X, double* Y, const FarWeights<double>& w) {
         if (!has_far()) return;
-        M2LLevelFn<double> m2l_fn = [&](int level, int b0, int nb, double scale) {
-            if (factored)
-                launch_m2l_fac<double>(ctx, fac64, level < 0 ? fac_all : fac_level[level], b0, nb, L64.p, E64.p, R,
-                                       scale);
-            else
-                launch_m2l64(ctx, d.v, b0, nb, L64.p, E64.p, R, scale);
-        };
-        launch_far_field<double>(ctx, d.v, d.far, X, w, Y, R, R, E64.p, L64.p, kCoulomb, m2l_fn, factored);
+        M2LLevelFn<double> m2l_fn = [&](int, int b0, int nb, double scale) { m2l64(b0, nb, scale); };
+        launch_far_field<double>(ctx, d.v, d.far, X, w, Y, R, R, E64.p, L64.p, kCoulomb, m2l_fn, factored, nullptr,
+                                 factored);
     }
 
     // Y = A32 X: FP32 near field, FP32 far field with TF32 tensor-core M2L.
@@ -858,15 +826,15 @@ struct Operator {
                     launch_m2l_tc(ctx, level < 0 ? tc.all : tc.level[level], node_stride(pl.n), E32.p, L32.p,
                                   m2l->K32.p, Rb32, (float)scale, level < 0 ? box_scale.p : nullptr, tc_err.p);
                 else
-                    launch_m2l_fac<float>(ctx, fac32, level < 0 ? fac_all : fac_level[level], b0, nb, L32.p, E32.p,
-                                          Rb32, scale);
+                    launch_m2l_fac<float>(ctx, fac32, b0, nb, L32.p, E32.p, Rb32, pl.n3);
             };
             const P2MSplit sp{Whi32.p, Wlo32.p, Xhi32.p, Xlo32.p, tc_err.p, l2p_tc ? Shi32.p : nullptr,
                               l2p_tc ? Slo32.p : nullptr};
-            // the shared-basis decompression overwrites every local expansion of
-            // levels 2 and deeper (L and L^ were cleared once, when allocated)
+            // the shared-basis decompression and the factored form overwrite
+            // every local expansion of levels 2 and deeper (L^ was cleared once,
+            // when allocated); the tensor-core form those of boxes with pairs
             launch_far_field<float>(ctx, d.v, d.far, X32.p, w32, Y, R, Rb32, E32.p, L32.p, kCoulomb, m2l_fn, true,
-                                    p2m_tc ? &sp : nullptr, shared);
+                                    p2m_tc ? &sp : nullptr, !tc32);
         }
     }
 

@@ -1,0 +1,31 @@
+"""Operator applies at right-hand-side counts around the kernels' column tiles
+(multiples of 8 up to 64, chunks beyond) against the oracle's apply: the same
+tree and the same compressed operators, FP64 reassociation only (1e-11, the bar
+of the operator parity tests)."""
+import numpy as np
+import pytest
+
+from gpurify_b200 import _lib, layouts
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = _lib.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("order,nrhs", [(2, 8), (3, 20), (4, 9), (4, 16), (4, 64), (5, 17), (5, 33), (5, 40), (5, 56),
+                                        (5, 65), (5, 130), (6, 24), (6, 33), (6, 64), (6, 256)])
+def test_apply_at_column_tile_edges(ctx, orc, order, nrhs):
+    lay = layouts.two_wires(length_nm=6000)
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, mesh_max_edge_m=0.3e-6,
+                             max_panels=-1)
+    sig = np.random.default_rng(order * 1000 + nrhs).standard_normal((len(p["verts"]), nrhs))
+    y, rep = ctx.operator_apply(p["verts"], sig, order=order, max_level=4, dense_below=-1)
+    assert rep["m2l_pairs"] > 0 and rep["dense"] == 0
+    for j in sorted({0, nrhs // 2, 7, 8, 63, 64, nrhs - 1} & set(range(nrhs))):
+        yo, _ = orc.fmm_cap_apply(p["verts"], sig[:, j], order, 4)
+        assert np.linalg.norm(y[:, j] - yo) / np.linalg.norm(yo) < 1e-11
