@@ -94,8 +94,7 @@ constexpr int kDTile = 64;
 __global__ void __launch_bounds__(kDThreads) k_near_assemble_dual(DevPlan p, const double* __restrict__ V,
                                                                   const double* __restrict__ dcent,
                                                                   double* __restrict__ dP, double coef) {
-    const int t = p.item_leaf[blockIdx.x];
-    const int r0 = p.item_row0[blockIdx.x];
+    const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int64_t tb = p.leaf_begin[t];
     const int m = min((int)(p.leaf_begin[t + 1] - tb), r0 + 64);
     const int S = p.near_S[t];

@@ -4,11 +4,12 @@
 //    source panel (integrals/panel.rs:147-208), one CTA per target leaf, one
 //    warp per group of target rows, lanes over source panels staged in shared
 //    memory (source geometry is prepared once per lane and reused across rows);
-//  * near-field apply: dense leaf blocks times R right-hand sides, source
-//    columns of X staged in shared memory, block rows broadcast by shuffle;
+//  * near-field apply: dense leaf blocks times R right-hand sides on FP64
+//    matrix instructions (FP32 on the CUDA cores);
 //  * far field: Chebyshev P2M, M2M, M2L, L2L, L2P (fmm/bbfmm.rs:209-448).
 #include <algorithm>
 
+#include "dmma.cuh"
 #include "gpx_common.h"
 #include "kernels.cuh"
 #include "wilton.cuh"
@@ -23,8 +24,7 @@ constexpr int kAsmTile = 64;
 // One CTA per work item (target leaf, <= 64 rows): rows of the leaf's
 // P block m_t x S_t, row-major.
 __global__ void __launch_bounds__(kAsmThreads, 2) k_near_assemble(DevPlan p, double* __restrict__ P, double coef) {
-    const int t = p.item_leaf[blockIdx.x];
-    const int r0 = p.item_row0[blockIdx.x];
+    const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int64_t tb = p.leaf_begin[t];
     const int m = min((int)(p.leaf_begin[t + 1] - tb), r0 + 64);
     const int S = p.near_S[t];
@@ -67,45 +67,174 @@ __global__ void k_diag_inv(DevPlan p, const double* __restrict__ P, double* __re
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// FP64 near apply: per work item (target leaf, <= 64 rows) and chunk of 8 NT
+// right-hand sides, Y[rows][.] = P_t[rows][0:S] X[src(0:S)][.] on FP64 matrix
+// instructions.  KC source panels per stage go through a three-stage cp.async
+// ring: the item's P rows (contiguous along the contraction) and the gathered
+// X rows (contiguous along the right-hand sides).  Four warps: NT / NTW of
+// them side by side over the columns, the others (WK in all) over the
+// contraction, their partial tiles added in a fixed order at the end.  Narrow
+// chunks thus split the contraction instead of leaving warps without columns.
+// Row tiles past the item's rows are skipped, so a 12-row leaf costs 16 rows.
+// Pitches of 4 more than a multiple of 8 doubles keep fragment reads free of
+// bank conflicts.  P rows are padded to a multiple of 4 entries and R is a
+// multiple of 4, so every 16-byte copy is aligned.
+// Bound: the FP64 rate from R = 32 up (2 R flop per 8-byte entry), below it
+// the stream of P and the gathers of X from L2.  Per apply, against 64 x 64
+// FMA tiles of 64 threads: 147.8 M entries, R = 64 1.01 ms (1.56 before; 0.51
+// at the FP64 rate); 7.5 M entries in 12-row leaves, R = 24 74 us (297);
+// 470 panels all pairs, R = 4 18 us (70).  The items run largest first: that
+// alone took the 12-row leaves from 106 to 74 us.
+template <int NT>
+struct NearMma {
+    static constexpr int NTW = NT % 3 == 0 ? 3 : NT == 1 ? 1 : 2;  // column tiles per warp
+    static constexpr int WN = NT / NTW, WK = 4 / WN;
+    static constexpr int KC = NT <= 3 ? 32 : 16, S = 3;
+    static constexpr int PP = KC + 4, XP = 8 * NT + 4;
+};
+template <int NT>
+__global__ void __launch_bounds__(128) k_near_apply_mma(DevPlan p, const double* __restrict__ P,
+                                                        const double* __restrict__ X, double* __restrict__ Y, int R,
+                                                        int tile_rows) {
+    using C = NearMma<NT>;
+    constexpr int NTW = C::NTW, WK = C::WK, KC = C::KC, S = C::S, PP = C::PP, XP = C::XP;
+    const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
+    const int rc = blockIdx.y * (8 * NT);
+    const int64_t tb = p.leaf_begin[t] + r0;
+    const int m = min((int)(p.leaf_begin[t + 1] - p.leaf_begin[t]) - r0, 64);
+    const int cols = min(8 * NT, R - rc);
+    const int nsrc = p.near_S[t], Sp = (nsrc + 3) & ~3;
+    const double* Pi = P + p.nval_off[t] + (int64_t)r0 * Sp;
+    __shared__ int64_t s_beg[28];
+    __shared__ int32_t s_pre[29];
+    extern __shared__ __align__(16) double near_smem[];
+    double* Ps = near_smem;                       // [S][tile_rows][PP]
+    double* Xs = Ps + S * tile_rows * PP;         // [S][KC][XP]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    if (warp == 0) near_ranges_warp(p, t, lane, s_beg, s_pre);
+    __syncthreads();
+    const int nst = (Sp + KC - 1) / KC, mt = (m + 7) >> 3;
+    int e = 0;  // near leaf of this thread's next X row (rows only grow)
+    auto issue = [&](int st) {
+        if (st < nst) {
+            const int k0 = st * KC;
+            double* ps = Ps + (st % S) * tile_rows * PP;
+            double* xs = Xs + (st % S) * KC * XP;
+            for (int id = tid; id < m * (KC / 2); id += 128) {
+                const int row = id / (KC / 2), k = 2 * (id % (KC / 2));
+                const bool ok = k0 + k < Sp;
+                cp_async_16(ps + row * PP + k, ok ? Pi + (int64_t)row * Sp + k0 + k : P, ok);
+            }
+#pragma unroll
+            for (int id = tid; id < KC * 4 * NT; id += 128) {
+                const int kk = id / (4 * NT), c = 2 * (id % (4 * NT)), k = k0 + kk;
+                const bool ok = k < nsrc && c < cols;
+                int64_t gid = 0;
+                if (k < nsrc) {
+                    while (s_pre[e + 1] <= k) ++e;
+                    gid = s_beg[e] + (k - s_pre[e]);
+                }
+                cp_async_16(xs + kk * XP + c, ok ? X + gid * R + rc + c : X, ok);
+            }
+        }
+        cp_async_fence();
+    };
+    const int wn = warp % C::WN, wk = warp / C::WN;
+    double acc[8][NTW][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll
+    for (int st = 0; st < S - 1; ++st) issue(st);
+    for (int st = 0; st < nst; ++st) {
+        cp_async_wait_for<S - 2>();
+        __syncthreads();
+        issue(st + S - 1);
+        const double* ps = Ps + (st % S) * tile_rows * PP + g * PP + q;
+        const double* xs = Xs + (st % S) * KC * XP + q * XP + 8 * NTW * wn + g;
+#pragma unroll
+        for (int k = 4 * wk; k < KC; k += 4 * WK) {
+            double b[NTW];
+#pragma unroll
+            for (int j = 0; j < NTW; ++j) b[j] = xs[k * XP + 8 * j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < mt) {
+                    // rows m .. 8 mt - 1 of the last tile hold leftovers of
+                    // other stages or items: their outputs are never stored
+                    const double a = ps[8 * i * PP + k];
+#pragma unroll
+                    for (int j = 0; j < NTW; ++j) dmma(acc[i][j], a, b[j]);
+                }
+        }
+    }
+    cp_async_wait_for<0>();
+    if constexpr (WK > 1) {
+        // partial tiles of the warps wk >= 1 through shared memory
+        __syncthreads();
+        double2* red = reinterpret_cast<double2*>(near_smem);  // [(WK - 1) WN][mt][NTW][32]
+        if (wk > 0)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < mt)
+#pragma unroll
+                    for (int j = 0; j < NTW; ++j)
+                        red[((((wk - 1) * C::WN + wn) * mt + i) * NTW + j) * 32 + lane] =
+                            make_double2(acc[i][j][0], acc[i][j][1]);
+        __syncthreads();
+        if (wk > 0) return;
+#pragma unroll
+        for (int w = 0; w < WK - 1; ++w)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < mt)
+#pragma unroll
+                    for (int j = 0; j < NTW; ++j) {
+                        const double2 v = red[(((w * C::WN + wn) * mt + i) * NTW + j) * 32 + lane];
+                        acc[i][j][0] += v.x;
+                        acc[i][j][1] += v.y;
+                    }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = 8 * i + g;
+        if (row >= m) continue;
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) {
+            const int c = 8 * (NTW * wn + j) + 2 * q;
+            if (c < cols)
+                *reinterpret_cast<double2*>(Y + (tb + row) * R + rc + c) = make_double2(acc[i][j][0], acc[i][j][1]);
+        }
+    }
 }
 
-// Near apply as a register-tiled GEMM per work item (target leaf, <= 64 rows)
-// and 64-wide chunk of right-hand sides:
-//     Y[rows][0:64] = P_t[rows][0:S] X[src(0:S)][0:64],
-// 64 threads, 8 x 8 outputs per thread (rows ty+8i, columns tx+8j: every
-// shared-memory read is a broadcast or conflict-free), the contraction
-// staged 32 source panels at a time with cp.async into a double buffer so the
-// next tile's loads overlap this tile's FMAs.  T = double (plain path) or
-// float (mixed path); rows of P are padded to a multiple of 4 entries and R
-// is a multiple of 4, so every 16-byte copy is aligned.
-template <class T>
-__global__ void __launch_bounds__(64) k_near_apply(DevPlan p, const T* __restrict__ P, const T* __restrict__ X,
-                                                   double* __restrict__ Y, int R) {
-    constexpr int V = 16 / sizeof(T);        // elements per 16-byte copy
-    constexpr int KC = 128 / sizeof(T);      // contraction chunk: 32 floats / 16 doubles
-    constexpr int PP = KC + V;               // Ps row pitch (16-byte multiple, conflict-free)
-    constexpr int XP = 64 + V;               // Xs row pitch
-    const int t = p.item_leaf[blockIdx.x];
-    const int r0 = p.item_row0[blockIdx.x];
+// FP32 near apply on the CUDA cores (the mixed path's mixed_near 1) as a
+// register-tiled GEMM per work item (target leaf, <= 64 rows) and 64-wide
+// chunk of right-hand sides: 64 threads, 8 x 8 outputs per thread (rows
+// ty+8i, columns tx+8j: every shared-memory read is a broadcast or
+// conflict-free), the contraction staged 32 source panels at a time with
+// cp.async into a double buffer so the next tile's loads overlap this tile's
+// FMAs.  Rows of P are padded to a multiple of 4 entries and R is a multiple
+// of 4, so every 16-byte copy is aligned.
+__global__ void __launch_bounds__(64) k_near_apply32(DevPlan p, const float* __restrict__ P,
+                                                     const float* __restrict__ X, double* __restrict__ Y, int R) {
+    constexpr int V = 4;        // elements per 16-byte copy
+    constexpr int KC = 32;      // contraction chunk
+    constexpr int PP = KC + V;  // Ps row pitch (16-byte multiple, conflict-free)
+    constexpr int XP = 64 + V;  // Xs row pitch
+    const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int rc = blockIdx.y * 64;
     const int64_t tb = p.leaf_begin[t] + r0;
     const int m = min((int)(p.leaf_begin[t + 1] - p.leaf_begin[t]) - r0, 64);
     const int S = p.near_S[t];
     const int Sp = (S + 3) & ~3;
-    const T* Pi = P + p.nval_off[t] + (int64_t)r0 * Sp;
+    const float* Pi = P + p.nval_off[t] + (int64_t)r0 * Sp;
     __shared__ int64_t s_beg[28];
     __shared__ int32_t s_pre[29];
     __shared__ int64_t s_gid[2][KC];
-    __shared__ __align__(16) T Ps[2][64][PP];  // [row][k]
-    __shared__ __align__(16) T Xs[2][KC][XP];  // [k][col]
+    __shared__ __align__(16) float Ps[2][64][PP];  // [row][k]
+    __shared__ __align__(16) float Xs[2][KC][XP];  // [k][col]
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
     if (tid < 32) near_ranges_warp(p, t, tid, s_beg, s_pre);
     __syncthreads();
@@ -128,21 +257,21 @@ __global__ void __launch_bounds__(64) k_near_apply(DevPlan p, const T* __restric
         for (int q = 0; q < KC / V; ++q) {  // P tile: 64 rows x KC
             const int id = tid + 64 * q, row = id / (KC / V), kc = (id % (KC / V)) * V;
             const bool ok = row < m && k0 + kc < Sp;
-            cp_async16(&Ps[buf][row][kc], ok ? (const void*)(Pi + (int64_t)row * Sp + k0 + kc) : (const void*)P, ok);
+            cp_async_16(&Ps[buf][row][kc], ok ? Pi + (int64_t)row * Sp + k0 + kc : P, ok);
         }
 #pragma unroll
         for (int q = 0; q < KC / V; ++q) {  // X tile: KC x 64 columns
             const int id = tid + 64 * q, kk = id / (64 / V), cc = (id % (64 / V)) * V;
             const bool ok = k0 + kk < S && rc + cc < R;
-            cp_async16(&Xs[buf][kk][cc], ok ? (const void*)(X + s_gid[buf][kk] * R + rc + cc) : (const void*)X, ok);
+            cp_async_16(&Xs[buf][kk][cc], ok ? X + s_gid[buf][kk] * R + rc + cc : X, ok);
         }
-        cp_async_commit();
+        cp_async_fence();
     };
-    T acc[8][8];
+    float acc[8][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = (T)0;
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     gather_ids(0);
     __syncthreads();
     issue(0);
@@ -151,15 +280,15 @@ __global__ void __launch_bounds__(64) k_near_apply(DevPlan p, const T* __restric
         __syncthreads();
         if (c + 1 < nchunk) {
             issue(c + 1);
-            cp_async_wait<1>();
+            cp_async_wait_for<1>();
         } else {
-            cp_async_wait<0>();
+            cp_async_wait_for<0>();
         }
         __syncthreads();
         const int buf = c & 1;
 #pragma unroll 4
         for (int kk = 0; kk < KC; ++kk) {
-            T a[8], b[8];
+            float a[8], b[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) a[i] = Ps[buf][ty + 8 * i][kk];
 #pragma unroll
@@ -289,18 +418,35 @@ void launch_diag_inv(Ctx& c, const DevPlan& p, const double* P, double* inv) {
     c.launches += 1;
 }
 
+template <int NT>
+static void near_mma(Ctx& c, const DevPlan& p, const double* P, const double* X, double* Y, int R) {
+    using C = NearMma<NT>;
+    const int tile_rows = std::min(64, (p.max_leaf + 7) & ~7);
+    const int smem = (int)sizeof(double) * C::S * (tile_rows * C::PP + C::KC * C::XP);
+    set_smem_once(k_near_apply_mma<NT>, smem);
+    k_near_apply_mma<NT><<<dim3(p.nitems, (R + 8 * NT - 1) / (8 * NT)), 128, smem, c.stream>>>(p, P, X, Y, R, tile_rows);
+    GPX_LAUNCH_CHECK();
+}
+
 void launch_near_apply(Ctx& c, const DevPlan& p, int64_t nnz, const double* P, const double* X, double* Y, int R) {
     if (p.nleaf == 0) return;
     KTimer t(c, K_NEAR_APPLY64, 8.0 * nnz + 16.0 * (double)p.N * R, 2.0 * (double)nnz * R);
-    k_near_apply<double><<<dim3(p.nitems, (R + 63) / 64), 64, 0, c.stream>>>(p, P, X, Y, R);
-    GPX_LAUNCH_CHECK();
+    switch (rhs_chunk(R, 64) / 8) {  // tiles of 5 and 7 would leave warps without columns
+        case 1: near_mma<1>(c, p, P, X, Y, R); break;
+        case 2: near_mma<2>(c, p, P, X, Y, R); break;
+        case 3: near_mma<3>(c, p, P, X, Y, R); break;
+        case 4: near_mma<4>(c, p, P, X, Y, R); break;
+        case 5:
+        case 6: near_mma<6>(c, p, P, X, Y, R); break;
+        default: near_mma<8>(c, p, P, X, Y, R); break;
+    }
     c.launches += 1;
 }
 
 void launch_near_apply32(Ctx& c, const DevPlan& p, int64_t nnz, const float* P, const float* X, double* Y, int R) {
     if (p.nleaf == 0) return;
     KTimer t(c, K_NEAR_APPLY, 4.0 * nnz + 12.0 * (double)p.N * R, 2.0 * (double)nnz * R);
-    k_near_apply<float><<<dim3(p.nitems, (R + 63) / 64), 64, 0, c.stream>>>(p, P, X, Y, R);
+    k_near_apply32<<<dim3(p.nitems, (R + 63) / 64), 64, 0, c.stream>>>(p, P, X, Y, R);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }

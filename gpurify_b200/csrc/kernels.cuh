@@ -14,6 +14,7 @@ struct DevPlan {
     int ns;                   // node stride of one expansion row: n3 rounded up to a multiple of 32
     int64_t N;
     int32_t nleaf, nbox, leaf_box0, nitems;
+    int32_t max_leaf;         // panels of the largest leaf
     const double* verts;      // 12 per panel
     const double* cent;       // 3 per panel
     const double* area;
@@ -26,6 +27,8 @@ struct DevPlan {
     const int64_t* nval_off;
     const int32_t* item_leaf;  // near-field work items (leaf, first row), <= 64 rows each
     const int32_t* item_row0;
+    const int32_t* item_order;  // the items by falling rows x sources: with thousands of uneven items on a few
+                                // hundred CTA slots, the largest must not start last
     const int32_t* box_parent;
     const int32_t* box_octant;
     const int64_t* m2l_off;

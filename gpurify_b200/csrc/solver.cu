@@ -184,7 +184,7 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
 struct DevPlanBufs {
     DBuf<double> verts, cent, area, w1d, m2m1d;
     DBuf<int32_t> cond, near_off, near_src, near_S, box_parent, box_octant, m2l_src, m2l_slot, child_first,
-        child_count, leaf_of, item_leaf, item_row0, item128_leaf, item128_row0, near_rev, near_pre, p2m_slot,
+        child_count, leaf_of, item_leaf, item_row0, item_order, item128_leaf, item128_row0, near_rev, near_pre, p2m_slot,
         fix_leaf, fix_first, fix_cnt;
     DBuf<int64_t> leaf_begin, nval_off, m2l_off;
     DBuf<double> leaf_ctr, wsrc;
@@ -225,6 +225,18 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
     }
     d.item_leaf.upload(p.item_leaf, s);
     d.item_row0.upload(p.item_row0, s);
+    {
+        std::vector<std::pair<int64_t, int32_t>> by(p.item_leaf.size());
+        for (size_t i = 0; i < by.size(); ++i) {
+            const int32_t k = p.item_leaf[i];
+            const int64_t rows = std::min<int64_t>(64, p.leaf_begin[k + 1] - p.leaf_begin[k] - p.item_row0[i]);
+            by[i] = {-rows * p.near_S[k], (int32_t)i};
+        }
+        std::sort(by.begin(), by.end());
+        std::vector<int32_t> order(by.size());
+        for (size_t i = 0; i < by.size(); ++i) order[i] = by[i].second;
+        d.item_order.upload(order, s);
+    }
     {
         // P2M runs over the near items: the first item of a leaf writes the
         // leaf's expansion, further items write partials that k_p2m_fix adds
@@ -273,6 +285,7 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
     }
     DevPlan& v = d.v;
     v.nitems = (int32_t)p.item_leaf.size();
+    v.max_leaf = p.max_leaf;
     v.item_leaf = d.item_leaf.p;
     v.leaf_ctr = d.leaf_ctr.p;
     v.leaf_of = d.leaf_of.p;
@@ -282,6 +295,7 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
         for (int k = 0; k < p.n && k < 8; ++k) v.roots[k] = roots[k];
     }
     v.item_row0 = d.item_row0.p;
+    v.item_order = d.item_order.p;
     {
         // 128-row work items of the tensor-core near apply, largest first so
         // the last wave of CTAs holds the short items
