@@ -14,10 +14,10 @@
 // FP64 runs on mma.sync (dmma.cuh) with column tiles that follow R, FP32 on
 // the CUDA cores.  One FP64 apply (both phases), against the 64-column
 // FMA tiles it replaced:
-//   order 5, R = 64, 62,802 box pairs:  1.20 ms (1.98 before; 0.8 at the FP64 rate)
-//   order 6, R = 24, 96,750 box pairs:  1.63 ms (6.23)
-//   order 5, R = 16, 31,940 box pairs:  0.28 ms (0.95)
-//   order 4, R = 4, 4,528 box pairs:    44 us (135)
+//   order 5, R = 64, 62,802 box pairs:  1.04 ms (1.98 before; 0.8 at the FP64 rate)
+//   order 6, R = 24, 96,750 box pairs:  1.35 ms (6.23)
+//   order 5, R = 16, 31,940 box pairs:  0.21 ms (0.95)
+//   order 4, R = 4, 4,528 box pairs:    32 us (135)
 #include "dmma.cuh"
 #include "farfield.cuh"
 
@@ -140,16 +140,23 @@ __global__ void __launch_bounds__(128) k_fac_v64(FacM2L<double> f, const FacItem
 // keep the four contraction rows of a fragment read in distinct banks.  L is
 // written, not added to (boxes without pairs get zero), so the caller clears
 // nothing.  Bound: FP64 tensor rate at R = 64, L2 (Ut rows) at R <= 16.
-template <int NT>
+template <int NT, int NS>
 struct FacU64 {
     static constexpr int KC = NT >= 3 ? 8 : 16;  // short tiles: fewer barriers per flop
     static constexpr int kStages = 4;
+    static constexpr int TP = 8 * NT + 4, UP = NS + 4;
+    static constexpr int kSmem = (int)sizeof(double) * kStages * KC * (TP + UP);  // + the column list
+    // 64-column tiles would take 183 registers and leave two CTAs an SM at
+    // order 5; three need at most 168 (707 us of phase 2 down to 540)
+    static constexpr int kMinCtas = NS == 128 ? 3 : NS < 128 ? 4 : 1;
 };
-template <int NT>
-__global__ void __launch_bounds__(224) k_fac_u64(FacM2L<double> f, int b0, double* __restrict__ L, int R) {
-    constexpr int KC = FacU64<NT>::KC, S = FacU64<NT>::kStages, TP = 8 * NT + 4;
+template <int NT, int NS>
+__global__ void __launch_bounds__(NS, (FacU64<NT, NS>::kMinCtas))
+    k_fac_u64(FacM2L<double> f, int b0, double* __restrict__ L, int R) {
+    using C = FacU64<NT, NS>;
+    constexpr int KC = C::KC, S = C::kStages, TP = C::TP, UP = C::UP, ns = NS;
     const int t = b0 + blockIdx.x, rc = blockIdx.y * (8 * NT);
-    const int ns = f.ns, rows = min(8 * NT, R - rc), UP = ns + 4;
+    const int rows = min(8 * NT, R - rc);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
     const int K = (int)(f.tgt_col_off[t + 1] - f.tgt_col_off[t]);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -167,18 +174,20 @@ __global__ void __launch_bounds__(224) k_fac_u64(FacM2L<double> f, int b0, doubl
         __syncthreads();
         const double* Tt = f.Tm + f.tgt_base[t] * R + rc;
         const int nst = (K + KC - 1) / KC;
-        const int tp = 4 * NT, up = ns / 2;  // 16-byte pieces of a T row and a Ut row
+        constexpr int tp = 4 * NT, up = ns / 2;  // 16-byte pieces of a T row and a Ut row
         auto issue = [&](int s) {
             if (s < nst) {
                 const int k0 = s * KC;
                 double* ts = Ts + (s % S) * KC * TP;
                 double* us = Us + (s % S) * KC * UP;
-                for (int e = threadIdx.x; e < KC * tp; e += blockDim.x) {
+#pragma unroll
+                for (int e = threadIdx.x; e < KC * tp; e += NS) {
                     const int k = e / tp, r = 2 * (e - k * tp);
                     const bool ok = k0 + k < K && r < rows;
                     cp_async_16(ts + k * TP + r, ok ? Tt + (int64_t)(k0 + k) * R + r : f.Tm, ok);
                 }
-                for (int e = threadIdx.x; e < KC * up; e += blockDim.x) {
+#pragma unroll
+                for (int e = threadIdx.x; e < KC * up; e += NS) {
                     const int k = e / up, m = 2 * (e - k * up);
                     const bool ok = k0 + k < K;
                     cp_async_16(us + k * UP + m, ok ? f.Ut + (int64_t)col[k0 + k] * ns + m : f.Ut, ok);
@@ -393,21 +402,30 @@ __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* 
     }
 }
 
+template <int NT, int NS>
+void run_fac_u64(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, int R) {
+    const int smem = FacU64<NT, NS>::kSmem + 2 * ((f.max_cols + 7) & ~7);
+    set_smem_once(k_fac_u64<NT, NS>, smem);
+    k_fac_u64<NT, NS><<<dim3(nb, cdiv(R, 8 * NT)), NS, smem, c.stream>>>(f, b0, L, R);
+    GPX_LAUNCH_CHECK();
+}
+
 template <int NT>
 void run_fac64(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, const double* E, int R, int n3) {
     constexpr int MT = NT >= 6 ? 2 : NT == 5 ? 3 : 4;  // at most 16 accumulator tiles a warp
-    const unsigned chunks = cdiv(R, 8 * NT);
     if (f.nitems > 0) {
         const int smem = (int)(sizeof(double) * 8 * NT * (f.ns + 8) + 12 * kFacItemCols);
         set_smem_once(k_fac_v64<NT, MT>, smem);
-        k_fac_v64<NT, MT><<<dim3(f.nitems, chunks), 128, smem, c.stream>>>(f, f.items, E, R, (n3 + 7) / 8);
+        k_fac_v64<NT, MT><<<dim3(f.nitems, cdiv(R, 8 * NT)), 128, smem, c.stream>>>(f, f.items, E, R, (n3 + 7) / 8);
         GPX_LAUNCH_CHECK();
     }
-    using U = FacU64<NT>;
-    const int smem = (int)(sizeof(double) * U::kStages * U::KC * (8 * NT + 4 + f.ns + 4)) + 2 * ((f.max_cols + 7) & ~7);
-    set_smem_once(k_fac_u64<NT>, smem);
-    k_fac_u64<NT><<<dim3(nb, chunks), f.ns, smem, c.stream>>>(f, b0, L, R);
-    GPX_LAUNCH_CHECK();
+    switch (f.ns) {
+        case 32: run_fac_u64<NT, 32>(c, f, b0, nb, L, R); break;
+        case 64: run_fac_u64<NT, 64>(c, f, b0, nb, L, R); break;
+        case 128: run_fac_u64<NT, 128>(c, f, b0, nb, L, R); break;
+        default:
+            if constexpr (NT <= 4) run_fac_u64<NT, 224>(c, f, b0, nb, L, R);
+    }
 }
 
 }  // namespace
