@@ -142,10 +142,11 @@ __global__ void __launch_bounds__(kDThreads) k_near_assemble_dual(DevPlan p, con
 __global__ void k_dsrc_weights(DevPlan p, int quad, const double* __restrict__ V, double* __restrict__ dW) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= p.N) return;
-    const int n = p.n, n3 = p.n3;
+    const int n = p.n, ns = p.ns;
     const double* ctr = p.leaf_ctr + 3 * p.leaf_of[j];
     const double ih = 1.0 / p.leaf_half;
-    double* out = dW + j * n3;
+    double* out = dW + j * ns;
+    for (int m = 0; m < ns; ++m) out[m] = 0.0;
     Dual cen[3], area;
     panel_props_dual(p.verts + 12 * j, V + 12 * j, cen, area);
     Dual w[3][8];
@@ -181,7 +182,6 @@ __global__ void k_dsrc_weights(DevPlan p, int quad, const double* __restrict__ V
         jw[q] = sqrt(cx * cx + cy * cy + cz * cz);
         jsum += jw[q];
     }
-    for (int m = 0; m < n3; ++m) out[m] = 0.0;
     for (int q = 0; q < 4; ++q) {
         const Dual wq = jsum > 0.0 ? jw[q] / jsum : Dual(0.25);
         for (int d = 0; d < 3; ++d) cheb_w_t<Dual>((pts[q][d] - ctr[d]) * ih, n, p.roots, w[d]);
@@ -193,19 +193,21 @@ __global__ void k_dsrc_weights(DevPlan p, int quad, const double* __restrict__ V
     }
 }
 
-// Chebyshev weights of the collocation point (centroid) as an N x n3 array:
+// Chebyshev weights of the collocation point (centroid) as an N x ns array
+// (node stride, padding zero):
 // the value (dcent == null) or its derivative along dcent.
 __global__ void k_centroid_weights(DevPlan p, const double* __restrict__ dcent, double* __restrict__ out) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= p.N) return;
-    const int n = p.n, n3 = p.n3;
+    const int n = p.n, n3 = p.n3, ns = p.ns;
     const double* ctr = p.leaf_ctr + 3 * p.leaf_of[j];
     const double ih = 1.0 / p.leaf_half;
     Dual w[3][8];
     for (int d = 0; d < 3; ++d)
         cheb_w_t<Dual>(Dual((p.cent[3 * j + d] - ctr[d]) * ih, dcent ? dcent[3 * j + d] * ih : 0.0), n, p.roots,
                        w[d]);
-    double* o = out + j * n3;
+    double* o = out + j * ns;
+    for (int m = n3; m < ns; ++m) o[m] = 0.0;
     for (int a = 0; a < n; ++a)
         for (int b = 0; b < n; ++b)
             for (int c = 0; c < n; ++c) {

@@ -18,6 +18,7 @@
 // contractions share partial sums along a binary tree (z, then y, then x for
 // M2M; the reverse for L2L): 14 n^4 multiply-adds per parent and right-hand
 // side instead of 24 n^4.
+#include "dmma.cuh"
 #include "farfield.cuh"
 #include "krylov.cuh"
 
@@ -57,6 +58,221 @@ constexpr int kMinCtas() {
     return sizeof(T) == 4 && N <= 5 ? 4 : 1;
 }
 
+// FP64 P2M and L2P on FP64 matrix instructions, one CTA per (work item = leaf
+// and <= 64 of its panels, chunk of 8 NT right-hand sides).  Both are bound by
+// latency and L2 at the leaves' sizes (12 to 64 panels): each stages what its
+// warps share once and has no stage loop.
+//
+// P2M: E[leaf][r][m] = sum_j W[j][m] (a_j X[j][r]).  One warp per 32 nodes;
+// the item's X rows are staged (zero past the item), the W rows, which each
+// warp reads in its own columns only, go from L2 straight to registers, four
+// panels ahead.  The weights have the node stride (padding zero).
+template <int N, int NT>
+__global__ void __launch_bounds__(Ord<N>::ns) k_p2m_mma(DevPlan p, const int32_t* __restrict__ slot,
+                                                        const double* __restrict__ X, const double* __restrict__ W,
+                                                        bool mul_area, double* __restrict__ E, int R) {
+    constexpr int NS = Ord<N>::ns, XP = 8 * NT + 4;
+    const int it = blockIdx.x, t = p.item_leaf[it], r0 = p.item_row0[it];
+    const int rc = blockIdx.y * (8 * NT), cols = min(8 * NT, R - rc);
+    const int64_t j0 = p.leaf_begin[t] + r0;
+    const int cnt = (int)min((int64_t)kItemPanels, p.leaf_begin[t + 1] - j0), cnt4 = (cnt + 3) & ~3;
+    extern __shared__ __align__(16) unsigned char far_smem[];
+    double* Xs = reinterpret_cast<double*>(far_smem);  // [kItemPanels][XP]
+    double* as = Xs + kItemPanels * XP;                // [kItemPanels]
+    for (int e = threadIdx.x; e < cnt4 * 4 * NT; e += NS) {
+        const int k = e / (4 * NT), c = 2 * (e % (4 * NT));
+        const bool ok = k < cnt && c < cols;
+        cp_async_16(Xs + k * XP + c, ok ? X + (j0 + k) * R + rc + c : X, ok);
+    }
+    cp_async_fence();
+    for (int k = threadIdx.x; k < cnt4; k += NS) as[k] = mul_area && k < cnt ? p.area[j0 + k] : 1.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const double* w = W + j0 * NS + 32 * warp + g;
+    double acc[NT][4][2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    double nx[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) nx[j] = __ldg(w + (int64_t)min(q, cnt - 1) * NS + 8 * j);
+    cp_async_wait_for<0>();
+    __syncthreads();
+    for (int k = 0; k < cnt4; k += 4) {
+        double b[4];
+        const double* wn = w + (int64_t)min(k + 4 + q, cnt - 1) * NS;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            b[j] = nx[j];
+            nx[j] = __ldg(wn + 8 * j);
+        }
+        const double ar = as[k + q];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const double a = ar * Xs[(k + q) * XP + 8 * i + g];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dmma(acc[i][j], a, b[j]);
+        }
+    }
+    const int64_t box = slot[it] < 0 ? (int64_t)p.leaf_box0 + t : (int64_t)p.nbox + slot[it];
+    double* out = E + (box * R + rc + g) * NS + 32 * warp + 2 * q;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        if (8 * i + g >= cols) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<double2*>(out + (int64_t)(8 * i) * NS + 8 * j) =
+                make_double2(acc[i][j][0], acc[i][j][1]);
+    }
+}
+
+// L2P: Y[j][r] += coef sum_m S_j[m] L[leaf][r][m].  The leaf's local rows are
+// staged; four warps share the item as tasks of 16 panels x 8 NTW columns.
+// The separable weights S_j[m] = (wx[a] wy[b]) wz[c] are formed in registers
+// from the panel's n^2 products and n values in shared memory; explicit
+// weights (WT) come from L2 with the node stride, times a_j if mul_area.
+template <int N, int NT, bool WT>
+__global__ void __launch_bounds__(128) k_l2p_mma(DevPlan p, const double* __restrict__ L,
+                                                 const double* __restrict__ Wt, bool mul_area, double* __restrict__ Y,
+                                                 int R, double coef) {
+    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, LP = NS + 8, NN = N * N;
+    constexpr int NTW = NT % 2 == 0 ? 2 : NT == 1 ? 1 : 3, NG = NT / NTW;
+    const int it = blockIdx.x, t = p.item_leaf[it], r0 = p.item_row0[it];
+    const int rc = blockIdx.y * (8 * NT), cols = min(8 * NT, R - rc);
+    const int64_t j0 = p.leaf_begin[t] + r0;
+    const int cnt = (int)min((int64_t)kItemPanels, p.leaf_begin[t + 1] - j0);
+    extern __shared__ __align__(16) unsigned char far_smem[];
+    double* Ls = reinterpret_cast<double*>(far_smem);      // [8 NT][LP]
+    double* wz = Ls + 8 * NT * LP;                         // [kItemPanels][N]
+    double* wxy = wz + kItemPanels * N;                    // [kItemPanels][NN]
+    uint16_t* tab = reinterpret_cast<uint16_t*>(wxy + kItemPanels * NN);  // per node: xy pair << 4 | z
+    const double* src = L + ((int64_t)(p.leaf_box0 + t) * R + rc) * NS;
+    for (int e = threadIdx.x; e < 8 * NT * (NS / 2); e += 128) {
+        const int r = e / (NS / 2), m = 2 * (e % (NS / 2));
+        cp_async_16(Ls + r * LP + m, r < cols ? src + (int64_t)r * NS + m : L, r < cols);
+    }
+    cp_async_fence();
+    if constexpr (!WT) {
+        const double* w = p.w1d + j0 * 3 * N;
+        for (int e = threadIdx.x; e < kItemPanels * NN; e += 128) {
+            const int j = e / NN, ab = e % NN;
+            wxy[e] = j < cnt ? w[j * 3 * N + ab / N] * w[j * 3 * N + N + ab % N] : 0.0;
+        }
+        for (int e = threadIdx.x; e < kItemPanels * N; e += 128) {
+            const int j = e / N;
+            wz[e] = j < cnt ? w[j * 3 * N + 2 * N + e % N] : 0.0;
+        }
+        // padding nodes: any weight does, their local expansion is zero
+        for (int m = threadIdx.x; m < NS; m += 128) tab[m] = m < N3 ? (uint16_t)((m / N) << 4 | (m % N)) : 0;
+    }
+    cp_async_wait_for<0>();
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int ntask = ((cnt + 15) >> 4) * NG;
+    for (int task = warp; task < ntask; task += 4) {
+        const int p0 = (task / NG) * 16, c0 = (task % NG) * 8 * NTW;
+        double acc[2][NTW][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < NTW; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        const double* lb = Ls + (c0 + g) * LP + 2 * q;
+        const double* wrow[2];
+        double ar[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = min(p0 + 8 * i + g, cnt - 1);
+            wrow[i] = WT ? Wt + (j0 + j) * NS + 2 * q : nullptr;
+            ar[i] = WT && mul_area ? p.area[j0 + j] : 1.0;
+        }
+#pragma unroll 4
+        for (int s = 0; s < (N3 + 7) / 8; ++s) {
+            double2 a[2];
+            if constexpr (WT) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const double2 v = __ldg(reinterpret_cast<const double2*>(wrow[i] + 8 * s));
+                    a[i] = make_double2(v.x * ar[i], v.y * ar[i]);
+                }
+            } else {
+                const int t0 = tab[8 * s + 2 * q], t1 = tab[8 * s + 2 * q + 1];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int j = p0 + 8 * i + g;
+                    a[i].x = wxy[j * NN + (t0 >> 4)] * wz[j * N + (t0 & 15)];
+                    a[i].y = wxy[j * NN + (t1 >> 4)] * wz[j * N + (t1 & 15)];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NTW; ++j) {
+                const double2 b = *reinterpret_cast<const double2*>(lb + 8 * j * LP + 8 * s);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].x, b.x);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].y, b.y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = p0 + 8 * i + g;
+            if (j >= cnt) continue;
+#pragma unroll
+            for (int n = 0; n < NTW; ++n) {
+                const int c = c0 + 8 * n + 2 * q;
+                if (c >= cols) continue;
+                double2* y = reinterpret_cast<double2*>(Y + (j0 + j) * R + rc + c);
+                double2 v = *y;
+                v.x += coef * acc[i][n][0];
+                v.y += coef * acc[i][n][1];
+                *y = v;
+            }
+        }
+    }
+}
+
+template <int N, int NT>
+void run_p2m64(Ctx& c, const DevPlan& p, const int32_t* slot, const double* X, const FarWeights<double>& w, double* E,
+               int R) {
+    const int smem = (int)sizeof(double) * (kItemPanels * (8 * NT + 4) + kItemPanels);
+    set_smem_once(k_p2m_mma<N, NT>, smem);
+    k_p2m_mma<N, NT><<<dim3(p.nitems, (R + 8 * NT - 1) / (8 * NT)), Ord<N>::ns, smem, c.stream>>>(
+        p, slot, X, w.src, w.src_area, E, R);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+}
+
+template <int N, int NT>
+void run_l2p64(Ctx& c, const DevPlan& p, const double* L, const FarWeights<double>& w, double* Y, int R, double coef) {
+    const int smem = (int)sizeof(double) * (8 * NT * (Ord<N>::ns + 8) + kItemPanels * (N + N * N)) + 2 * Ord<N>::ns;
+    const dim3 grid(p.nitems, (R + 8 * NT - 1) / (8 * NT));
+    if (w.tgt) {
+        set_smem_once(k_l2p_mma<N, NT, true>, smem);
+        k_l2p_mma<N, NT, true><<<grid, 128, smem, c.stream>>>(p, L, w.tgt, w.tgt_area, Y, R, coef);
+    } else {
+        set_smem_once(k_l2p_mma<N, NT, false>, smem);
+        k_l2p_mma<N, NT, false><<<grid, 128, smem, c.stream>>>(p, L, nullptr, false, Y, R, coef);
+    }
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+}
+
+// Column chunks as in the M2L (m2l_fac.cu), widths of 5 and 7 tiles rounded up.
+template <int N, class F>
+void by_chunk(int R, F&& run) {
+    switch (rhs_chunk(R, Ord<N>::ns > 128 ? 32 : 64) / 8) {
+        case 1: run(std::integral_constant<int, 1>()); break;
+        case 2: run(std::integral_constant<int, 2>()); break;
+        case 3: run(std::integral_constant<int, 3>()); break;
+        case 4: run(std::integral_constant<int, 4>()); break;
+        case 5:
+        case 6:
+            if constexpr (Ord<N>::ns <= 128) run(std::integral_constant<int, 6>());
+            break;
+        default:
+            if constexpr (Ord<N>::ns <= 128) run(std::integral_constant<int, 8>());
+    }
+}
+
 // P2M as a GEMM per (work item = leaf and <= 64 of its panels, 64-wide chunk
 // of rows r):  E[leaf][r][m] = sum_j W[j][m] * (a_j X[j][r]).
 // The work items are the near-field items (64 panels each), so a leaf of a few
@@ -92,7 +308,7 @@ __global__ void __launch_bounds__(256, kMinCtas<T, N>())
         __syncthreads();
         for (int e = tid; e < KP * NS; e += 256) {
             const int k = e / NS, m = e % NS;
-            Ws[k][m] = (k < cnt && m < N3) ? W[(jb + k) * N3 + m] : (T)0;
+            Ws[k][m] = k < cnt ? W[(jb + k) * NS + m] : (T)0;
         }
         for (int e = tid; e < KP * 64; e += 256) {
             const int k = e >> 6, r = e & 63;
@@ -194,7 +410,7 @@ __global__ void __launch_bounds__(256, kMinCtas<T, N>())
             const int jj = e / MK, mm = e % MK, m = m0 + mm;
             T v = (T)0;
             if (m < N3 && jj < cnt) {
-                v = Wt ? Wt[(jb + jj) * N3 + m] : wv[jj][m / (N * N)] * wv[jj][N + (m / N) % N] * wv[jj][2 * N + m % N];
+                v = Wt ? Wt[(jb + jj) * NS + m] : wv[jj][m / (N * N)] * wv[jj][N + (m / N) % N] * wv[jj][2 * N + m % N];
                 if (mul_area) v *= (T)p.area[jb + jj];
             }
             Ss[mm][jj] = v;
@@ -642,9 +858,13 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
                 c.launches += 1;
             }
         } else {
-            k_p2m<T, N><<<dim3(p.nitems, rchunks64), 256, 0, s>>>(p, f.p2m_slot, X, w.src, w.src_area, E, R, Rb);
-            GPX_LAUNCH_CHECK();
-            c.launches += 1;
+            if constexpr (sizeof(T) == 8) {
+                by_chunk<N>(R, [&](auto nt) { run_p2m64<N, nt>(c, p, f.p2m_slot, X, w, E, R); });
+            } else {
+                k_p2m<T, N><<<dim3(p.nitems, rchunks64), 256, 0, s>>>(p, f.p2m_slot, X, w.src, w.src_area, E, R, Rb);
+                GPX_LAUNCH_CHECK();
+                c.launches += 1;
+            }
         }
         if (f.nfix > 0) {
             const int64_t block = (int64_t)Rb * NS;
@@ -708,7 +928,9 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
                 done = true;
             }
         }
-        if (!done) {
+        if constexpr (sizeof(T) == 8) {
+            by_chunk<N>(R, [&](auto nt) { run_l2p64<N, nt>(c, p, L, w, Y, R, coef); });
+        } else if (!done) {
             k_l2p<T, N><<<dim3(p.nitems, cdiv(R, 64)), 256, 0, s>>>(p, L, w.tgt, w.tgt_area, Y, R, Rb, coef);
             GPX_LAUNCH_CHECK();
             c.launches += 1;

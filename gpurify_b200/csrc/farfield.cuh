@@ -18,9 +18,9 @@ using M2LLevelFn = std::function<void(int, int, int, double)>;
 // (S(c) as an array, none) at P2M and (W, area) at L2P.
 template <class T>
 struct FarWeights {
-    const T* src = nullptr;  // N x n3
+    const T* src = nullptr;  // N x ns (node stride, padding zero)
     bool src_area = true;
-    const T* tgt = nullptr;  // N x n3 or null
+    const T* tgt = nullptr;  // N x ns or null
     bool tgt_area = false;
 };
 
@@ -51,8 +51,8 @@ void launch_far_field(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, 
 // l_written: the M2L callback overwrites every local-expansion row of levels
 // 2 and deeper (the shared-basis decompression does), and L's rows of levels
 // 0 and 1 are zero: L is then not cleared before the M2L.
-// Whi / Wlo [N][128] = TF32 split of (area if mul_area) x W[N][n3] (n3 <= 128).
-void launch_split_weights(Ctx& c, const double* W, int n3, const double* area, bool mul_area, float* Whi, float* Wlo,
+// Whi / Wlo [N][128] = TF32 split of (area if mul_area) x W[N][ns] (ns <= 128).
+void launch_split_weights(Ctx& c, const double* W, int ns, const double* area, bool mul_area, float* Whi, float* Wlo,
                           int64_t N);
 // Y += coef L2P of the far-field locals L with split target weights (orders 4 and 5).
 void launch_l2p_tc(Ctx& c, const DevPlan& p, const float* L, const float* Shi, const float* Slo, double* Y, int R,

@@ -89,11 +89,12 @@ template <int NT>
 struct NearMma {
     static constexpr int NTW = NT % 3 == 0 ? 3 : NT == 1 ? 1 : 2;  // column tiles per warp
     static constexpr int WN = NT / NTW, WK = 4 / WN;
-    static constexpr int KC = NT <= 3 ? 32 : 16, S = 3;
+    static constexpr int KC = NT <= 3 ? 32 : 16, S = NT == 8 ? 2 : 3;
+    static constexpr int kMinCtas = NT == 8 ? 4 : 2;
     static constexpr int PP = KC + 4, XP = 8 * NT + 4;
 };
 template <int NT>
-__global__ void __launch_bounds__(128) k_near_apply_mma(DevPlan p, const double* __restrict__ P,
+__global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(DevPlan p, const double* __restrict__ P,
                                                         const double* __restrict__ X, double* __restrict__ Y, int R,
                                                         int tile_rows) {
     using C = NearMma<NT>;
@@ -336,15 +337,15 @@ __device__ __forceinline__ void cheb_w(double x, int n, const double* roots, dou
     }
 }
 
-// One thread per panel: W[j][m] for all n^3 nodes.
+// One thread per panel: W[j][m] for all n^3 nodes (node stride, padding zero).
 __global__ void k_src_weights(DevPlan p, int quad, double* __restrict__ W) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= p.N) return;
-    const int n = p.n, n3 = p.n3;
+    const int n = p.n, ns = p.ns;
     const double* ctr = p.leaf_ctr + 3 * p.leaf_of[j];
     const double ih = 1.0 / p.leaf_half;
-    double* out = W + j * n3;
-    for (int m = 0; m < n3; ++m) out[m] = 0.0;
+    double* out = W + j * ns;
+    for (int m = 0; m < ns; ++m) out[m] = 0.0;
     double w[3][8];
     if (quad == 0) {
         for (int d = 0; d < 3; ++d) cheb_w((p.cent[3 * j + d] - ctr[d]) * ih, n, p.roots, w[d]);

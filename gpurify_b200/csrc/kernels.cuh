@@ -40,7 +40,7 @@ struct DevPlan {
     const int32_t* leaf_of;   // per panel: its leaf
     double leaf_half;
     double roots[8];          // Chebyshev roots of order n
-    const double* wsrc;       // N x n3 far-field source weights (P2M), set by launch_src_weights
+    const double* wsrc;       // N x ns far-field source weights (P2M), set by launch_src_weights
 };
 
 // Source ranges of target leaf t's near list, read by the 32 lanes of one

@@ -198,15 +198,15 @@ __global__ void __launch_bounds__(kThreads) k_p2m_tc(DevPlan p, const int32_t* _
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// Whi / Wlo [N][kWS] = TF32 split of (area if mul_area) x W[N][n3], nodes past n3 zero.
-__global__ void k_split_weights(const double* __restrict__ W, int n3, const double* __restrict__ area, int mul_area,
+// Whi / Wlo [N][kWS] = TF32 split of (area if mul_area) x W[N][ns], nodes past ns zero.
+__global__ void k_split_weights(const double* __restrict__ W, int ns, const double* __restrict__ area, int mul_area,
                                 float* __restrict__ Whi, float* __restrict__ Wlo, int64_t N) {
     const int64_t n = N * kWS;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = i / kWS;
         const int m = (int)(i % kWS);
         double w = 0.0;
-        if (m < n3) w = W[j * n3 + m] * (mul_area ? area[j] : 1.0);
+        if (m < ns) w = W[j * ns + m] * (mul_area ? area[j] : 1.0);
         const float hi = to_tf32((float)w);
         Whi[i] = hi;
         Wlo[i] = to_tf32((float)(w - (double)hi));
@@ -215,12 +215,12 @@ __global__ void k_split_weights(const double* __restrict__ W, int n3, const doub
 
 }  // namespace
 
-void launch_split_weights(Ctx& c, const double* W, int n3, const double* area, bool mul_area, float* Whi, float* Wlo,
+void launch_split_weights(Ctx& c, const double* W, int ns, const double* area, bool mul_area, float* Whi, float* Wlo,
                           int64_t N) {
-    if (n3 > kWS) throw Error(GPX_ERR_INTERNAL, "split far-field weights take at most 128 nodes");
+    if (ns > kWS) throw Error(GPX_ERR_INTERNAL, "split far-field weights take at most 128 nodes");
     const int64_t n = N * kWS;
     KTimer t(c, K_VEC, 16.0 * n, 0.0);
-    k_split_weights<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 16), 256, 0, c.stream>>>(W, n3, area,
+    k_split_weights<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 16), 256, 0, c.stream>>>(W, ns, area,
                                                                                                  mul_area ? 1 : 0,
                                                                                                  Whi, Wlo, N);
     GPX_LAUNCH_CHECK();

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "dmma.cuh"
 #include "precond.cuh"
 
 namespace gpx {
@@ -84,58 +85,79 @@ __global__ void __launch_bounds__(256) k_block_invert(DevPlan p, const double* _
     for (int e = threadIdx.x; e < kB * kB; e += blockDim.x) out[e] = I[e / kB][e % kB];
 }
 
-// One CTA per (block, 64-column chunk): Z[rows] = Minv V[rows].  256
-// threads; thread (ty, tx) holds rows ty + 16 a (a < KB/16) and columns
-// tx + 16 q (q < 4) in registers, so each shared-memory read feeds several
-// multiply-adds.
-template <int kB>
-__global__ void __launch_bounds__(256) k_block_apply(const double* __restrict__ Minv,
+// Z[rows] = Minv V[rows] on FP64 matrix instructions, one CTA per (block,
+// chunk of 8 NT columns).  The block's V rows are staged; each warp takes 16
+// rows of the inverse at a time, read once, straight into registers (a lane's
+// 16 bytes hold columns k + 2q and k + 2q + 1, q = lane % 4, for two
+// instructions).  The pitch 8 NT + 2 puts V rows k, k + 2, k + 4, k + 6 in
+// distinct banks.  Only the block's own rows and columns are read and
+// multiplied (a 12-panel leaf costs 16 x 16, not 96 x 96).
+template <int kB, int NT>
+__global__ void __launch_bounds__(128) k_block_apply(const double* __restrict__ Minv,
                                                      const int64_t* __restrict__ blk_start,
                                                      const int32_t* __restrict__ blk_size, const double* __restrict__ V,
                                                      DevIndex di, double* __restrict__ Z, int R, int add) {
-    constexpr int RA = kB / 16;
+    constexpr int VP = 8 * NT + 2;
     V = dev_offset(V, di);
     const int bi = blockIdx.x;
-    const int rc = blockIdx.y * 64;
+    const int rc = blockIdx.y * (8 * NT), cols = min(8 * NT, R - rc);
     const int64_t s0 = blk_start[bi];
-    const int b = blk_size[bi];
-    extern __shared__ double bj_smem[];
-    double(*Ms)[kB + 1] = reinterpret_cast<double(*)[kB + 1]>(bj_smem);
-    double(*Vs)[65] = reinterpret_cast<double(*)[65]>(bj_smem + kB * (kB + 1));
-    const double* M = Minv + (int64_t)bi * kB * kB;
-    for (int e = threadIdx.x; e < kB * kB; e += blockDim.x) Ms[e / kB][e % kB] = M[e];
-    for (int e = threadIdx.x; e < kB * 64; e += blockDim.x) {
-        const int i = e >> 6, c = e & 63;
-        Vs[i][c] = (i < b && rc + c < R) ? V[(s0 + i) * R + rc + c] : 0.0;
+    const int b = blk_size[bi], b8 = (b + 7) & ~7;
+    extern __shared__ __align__(16) double bj_smem[];
+    double* Vs = bj_smem;  // [b8][VP]
+    for (int e = threadIdx.x; e < b8 * 4 * NT; e += 128) {
+        const int i = e / (4 * NT), c = 2 * (e % (4 * NT));
+        const bool ok = i < b && c < cols;
+        cp_async_16(Vs + i * VP + c, ok ? V + (s0 + i) * R + rc + c : V, ok);
     }
+    cp_async_fence();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const double* M = Minv + (int64_t)bi * kB * kB + 2 * q;
+    cp_async_wait_for<0>();
     __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[RA][4];
+    for (int i0 = 16 * warp; i0 < b; i0 += 64) {
+        const double* m0 = M + (int64_t)(i0 + g) * kB;  // rows past b (inside the kB x kB block) are never stored
+        double acc[2][NT][2];
 #pragma unroll
-    for (int a = 0; a < RA; ++a)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[a][q] = 0.0;
-    for (int k = 0; k < b; ++k) {
-        double m[RA], v[4];
+            for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        double2 nx[2];
 #pragma unroll
-        for (int a = 0; a < RA; ++a) m[a] = Ms[ty + 16 * a][k];
+        for (int i = 0; i < 2; ++i) nx[i] = __ldg(reinterpret_cast<const double2*>(m0 + 8 * i * kB));
+        for (int k = 0; k < b8; k += 8) {
+            double2 a[2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = Vs[k][tx + 16 * q];
+            for (int i = 0; i < 2; ++i) {
+                a[i] = nx[i];
+                nx[i] = __ldg(reinterpret_cast<const double2*>(m0 + 8 * i * kB + min(k + 8, kB - 8)));
+            }
 #pragma unroll
-        for (int a = 0; a < RA; ++a)
+            for (int j = 0; j < NT; ++j) {
+                const double v0 = Vs[(k + 2 * q) * VP + 8 * j + g], v1 = Vs[(k + 2 * q + 1) * VP + 8 * j + g];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[a][q] += m[a] * v[q];
-    }
+                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].x, v0);
 #pragma unroll
-    for (int a = 0; a < RA; ++a) {
-        const int i = ty + 16 * a;
-        if (i >= b) continue;
+                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].y, v1);
+            }
+        }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = tx + 16 * q;
-            if (rc + c >= R) continue;
-            double* z = Z + (s0 + i) * R + rc + c;
-            *z = add ? *z + acc[a][q] : acc[a][q];
+        for (int i = 0; i < 2; ++i) {
+            const int row = i0 + 8 * i + g;
+            if (row >= b) continue;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const int c = 8 * j + 2 * q;
+                if (c >= cols) continue;
+                double2* z = reinterpret_cast<double2*>(Z + (s0 + row) * R + rc + c);
+                double2 v = make_double2(acc[i][j][0], acc[i][j][1]);
+                if (add) {
+                    const double2 o = *z;
+                    v.x += o.x;
+                    v.y += o.y;
+                }
+                *z = v;
+            }
         }
     }
 }
@@ -295,21 +317,37 @@ void BlockJacobi::check(Ctx& c) const {
     if (sing) throw Error(GPX_ERR_CAPACITANCE, "singular near-field block in the block-Jacobi preconditioner");
 }
 
-void BlockJacobi::apply(Ctx& c, const double* V, double* Z, int64_t N, int R, bool add, const DevIndex& di) const {
-    const int kB = block;
-    KTimer t(c, K_VEC, 8.0 * (2.0 * N * R + (double)nblk * kB * kB), 2.0 * (double)N * kB * R);
-    const int smem = (int)(sizeof(double) * (kB * (kB + 1) + kB * 65));
-    const dim3 g(nblk, (R + 63) / 64);
-    if (kB == 96) {
-        set_smem_once(k_block_apply<96>, smem);
-        k_block_apply<96><<<g, 256, smem, c.stream>>>(Minv.p, d_start.p, d_size.p, V, di, Z, R, add ? 1 : 0);
-    } else {
-        set_smem_once(k_block_apply<48>, smem);
-        k_block_apply<48><<<g, 256, smem, c.stream>>>(Minv.p, d_start.p, d_size.p, V, di, Z, R, add ? 1 : 0);
-    }
+template <int kB, int NT>
+static void block_apply(Ctx& c, const BlockJacobi& bj, const double* V, double* Z, int R, bool add, const DevIndex& di) {
+    const int smem = (int)sizeof(double) * kB * (8 * NT + 2);
+    set_smem_once(k_block_apply<kB, NT>, smem);
+    k_block_apply<kB, NT><<<dim3(bj.nblk, (R + 8 * NT - 1) / (8 * NT)), 128, smem, c.stream>>>(
+        bj.Minv.p, bj.d_start.p, bj.d_size.p, V, di, Z, R, add ? 1 : 0);
     GPX_LAUNCH_CHECK();
+}
+
+template <int kB>
+static void block_apply_by_chunk(Ctx& c, const BlockJacobi& bj, const double* V, double* Z, int R, bool add,
+                                 const DevIndex& di) {
+    switch (rhs_chunk(R, 64) / 8) {
+        case 1: block_apply<kB, 1>(c, bj, V, Z, R, add, di); break;
+        case 2: block_apply<kB, 2>(c, bj, V, Z, R, add, di); break;
+        case 3: block_apply<kB, 3>(c, bj, V, Z, R, add, di); break;
+        case 4: block_apply<kB, 4>(c, bj, V, Z, R, add, di); break;
+        case 5:
+        case 6: block_apply<kB, 6>(c, bj, V, Z, R, add, di); break;
+        default: block_apply<kB, 8>(c, bj, V, Z, R, add, di); break;
+    }
+}
+
+void BlockJacobi::apply(Ctx& c, const double* V, double* Z, int64_t N, int R, bool add, const DevIndex& di) const {
+    if (R % 4 != 0) throw Error(GPX_ERR_INTERNAL, "block-Jacobi apply needs R % 4 == 0");
+    KTimer t(c, K_VEC, 8.0 * (2.0 * N * R + (double)nblk * block * block), 2.0 * (double)N * block * R);
+    if (block == 96)
+        block_apply_by_chunk<96>(c, *this, V, Z, R, add, di);
+    else
+        block_apply_by_chunk<48>(c, *this, V, Z, R, add, di);
     c.launches += 1;
-    (void)N;
 }
 
 }  // namespace gpx

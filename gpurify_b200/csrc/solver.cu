@@ -610,12 +610,12 @@ struct Operator {
         if (has_far()) {
             const int ns = node_stride(pl.n);
             if (!transposed) {
-                d.wsrc.alloc((size_t)pl.N * pl.n3, s);
+                d.wsrc.alloc((size_t)pl.N * node_stride(pl.n), s);
                 launch_src_weights(ctx, d.v, far_quad, d.wsrc.p);
                 d.v.wsrc = d.wsrc.p;
                 w64 = FarWeights<double>{d.wsrc.p, true, nullptr, false};
             } else {
-                Sc.alloc((size_t)pl.N * pl.n3, s);
+                Sc.alloc((size_t)pl.N * node_stride(pl.n), s);
                 launch_centroid_weights(ctx, d.v, nullptr, Sc.p);
                 w64 = FarWeights<double>{Sc.p, false, d.wsrc.p, true};
             }
@@ -648,13 +648,13 @@ struct Operator {
                 Rb32 = (R + 63) / 64 * 64;
                 E32.alloc((size_t)(pl.nbox() + d.far.npart) * ns * Rb32, s);
                 L32.alloc((size_t)pl.nbox() * ns * Rb32, s);
-                W32.alloc((size_t)pl.N * pl.n3, s);
-                launch_to_f32(ctx, d.wsrc.p, W32.p, pl.N * pl.n3);
+                W32.alloc((size_t)pl.N * node_stride(pl.n), s);
+                launch_to_f32(ctx, d.wsrc.p, W32.p, pl.N * node_stride(pl.n));
                 if (!transposed) {
                     w32 = FarWeights<float>{W32.p, true, nullptr, false};
                 } else {
-                    Sc32.alloc((size_t)pl.N * pl.n3, s);
-                    launch_to_f32(ctx, Sc.p, Sc32.p, pl.N * pl.n3);
+                    Sc32.alloc((size_t)pl.N * node_stride(pl.n), s);
+                    launch_to_f32(ctx, Sc.p, Sc32.p, pl.N * node_stride(pl.n));
                     w32 = FarWeights<float>{Sc32.p, false, W32.p, true};
                 }
                 if (p2m_tc) {
@@ -664,14 +664,14 @@ struct Operator {
                     Slo32.alloc((size_t)pl.N * 128, s);
                     if (!transposed) {
                         // P2M: source weights with the area; L2P: collocation weights at the centroids
-                        launch_split_weights(ctx, d.wsrc.p, pl.n3, d.area.p, true, Whi32.p, Wlo32.p, pl.N);
+                        launch_split_weights(ctx, d.wsrc.p, ns, d.area.p, true, Whi32.p, Wlo32.p, pl.N);
                         DBuf<double> S64;
-                        S64.alloc((size_t)pl.N * pl.n3, s);
+                        S64.alloc((size_t)pl.N * node_stride(pl.n), s);
                         launch_centroid_weights(ctx, d.v, nullptr, S64.p);
-                        launch_split_weights(ctx, S64.p, pl.n3, d.area.p, false, Shi32.p, Slo32.p, pl.N);
+                        launch_split_weights(ctx, S64.p, ns, d.area.p, false, Shi32.p, Slo32.p, pl.N);
                     } else {
-                        launch_split_weights(ctx, Sc.p, pl.n3, d.area.p, false, Whi32.p, Wlo32.p, pl.N);
-                        launch_split_weights(ctx, d.wsrc.p, pl.n3, d.area.p, true, Shi32.p, Slo32.p, pl.N);
+                        launch_split_weights(ctx, Sc.p, ns, d.area.p, false, Whi32.p, Wlo32.p, pl.N);
+                        launch_split_weights(ctx, d.wsrc.p, ns, d.area.p, true, Shi32.p, Slo32.p, pl.N);
                     }
                 }
                 if (tc32 || shared) build_tc_lists(ctx, pl, tc);
@@ -1754,8 +1754,8 @@ void cap_sensitivity(Ctx& ctx, int64_t n, const double* verts, const int32_t* co
     G.alloc((size_t)Ra * R, s);
     Gp.alloc((size_t)grad_contract_splits(Ra) * Ra * R, s);
     if (op.has_far()) {
-        dW.alloc((size_t)n * pl.n3, s);
-        dS.alloc((size_t)n * pl.n3, s);
+        dW.alloc((size_t)n * node_stride(pl.n), s);
+        dS.alloc((size_t)n * node_stride(pl.n), s);
     }
     std::vector<double> vs((size_t)n * 12), hg((size_t)Ra * R);
     for (size_t e = 0; e < (size_t)np * ncond * ncond; ++e) dCdp[e] = std::nan("");
