@@ -50,14 +50,6 @@ struct Ord {
     static constexpr int ns = (n3 + 31) & ~31;
 };
 
-// CTAs per SM the FP32 P2M and L2P are compiled for at orders <= 5: four
-// (64 registers, no spills) instead of the two that 90 registers allowed, so
-// more warps hide the latency of each staged slice's global loads.
-template <class T, int N>
-constexpr int kMinCtas() {
-    return sizeof(T) == 4 && N <= 5 ? 4 : 1;
-}
-
 // FP64 P2M and L2P on FP64 matrix instructions, one CTA per (work item = leaf
 // and <= 64 of its panels, chunk of 8 NT right-hand sides).  Both are bound by
 // latency and L2 at the leaves' sizes (12 to 64 panels): each stages what its
@@ -135,7 +127,7 @@ template <int N, int NT, bool WT>
 __global__ void __launch_bounds__(128) k_l2p_mma(DevPlan p, const double* __restrict__ L,
                                                  const double* __restrict__ Wt, bool mul_area, double* __restrict__ Y,
                                                  int R, double coef) {
-    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, LP = NS + 8, NN = N * N;
+    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, LP = NS + 4, NN = N * N;
     constexpr int NTW = NT % 2 == 0 ? 2 : NT == 1 ? 1 : 3, NG = NT / NTW;
     const int it = blockIdx.x, t = p.item_leaf[it], r0 = p.item_row0[it];
     const int rc = blockIdx.y * (8 * NT), cols = min(8 * NT, R - rc);
@@ -176,40 +168,37 @@ __global__ void __launch_bounds__(128) k_l2p_mma(DevPlan p, const double* __rest
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < NTW; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-        const double* lb = Ls + (c0 + g) * LP + 2 * q;
+        const double* lb = Ls + (c0 + g) * LP + q;
         const double* wrow[2];
         double ar[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int j = min(p0 + 8 * i + g, cnt - 1);
-            wrow[i] = WT ? Wt + (j0 + j) * NS + 2 * q : nullptr;
+            wrow[i] = WT ? Wt + (j0 + j) * NS + q : nullptr;
             ar[i] = WT && mul_area ? p.area[j0 + j] : 1.0;
         }
 #pragma unroll 4
         for (int s = 0; s < (N3 + 7) / 8; ++s) {
-            double2 a[2];
-            if constexpr (WT) {
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const double2 v = __ldg(reinterpret_cast<const double2*>(wrow[i] + 8 * s));
-                    a[i] = make_double2(v.x * ar[i], v.y * ar[i]);
+            for (int h = 0; h < 2; ++h) {  // nodes 8 s + 4 h .. + 3, ascending
+                double a[2];
+                if constexpr (WT) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) a[i] = __ldg(wrow[i] + 8 * s + 4 * h) * ar[i];
+                } else {
+                    const int tn = tab[8 * s + 4 * h + q];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int j = p0 + 8 * i + g;
+                        a[i] = wxy[j * NN + (tn >> 4)] * wz[j * N + (tn & 15)];
+                    }
                 }
-            } else {
-                const int t0 = tab[8 * s + 2 * q], t1 = tab[8 * s + 2 * q + 1];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int j = p0 + 8 * i + g;
-                    a[i].x = wxy[j * NN + (t0 >> 4)] * wz[j * N + (t0 & 15)];
-                    a[i].y = wxy[j * NN + (t1 >> 4)] * wz[j * N + (t1 & 15)];
+                for (int j = 0; j < NTW; ++j) {
+                    const double b = lb[8 * j * LP + 8 * s + 4 * h];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i], b);
                 }
-            }
-#pragma unroll
-            for (int j = 0; j < NTW; ++j) {
-                const double2 b = *reinterpret_cast<const double2*>(lb + 8 * j * LP + 8 * s);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].x, b.x);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].y, b.y);
             }
         }
 #pragma unroll
@@ -243,7 +232,7 @@ void run_p2m64(Ctx& c, const DevPlan& p, const int32_t* slot, const double* X, c
 
 template <int N, int NT>
 void run_l2p64(Ctx& c, const DevPlan& p, const double* L, const FarWeights<double>& w, double* Y, int R, double coef) {
-    const int smem = (int)sizeof(double) * (8 * NT * (Ord<N>::ns + 8) + kItemPanels * (N + N * N)) + 2 * Ord<N>::ns;
+    const int smem = (int)sizeof(double) * (8 * NT * (Ord<N>::ns + 4) + kItemPanels * (N + N * N)) + 2 * Ord<N>::ns;
     const dim3 grid(p.nitems, (R + 8 * NT - 1) / (8 * NT));
     if (w.tgt) {
         set_smem_once(k_l2p_mma<N, NT, true>, smem);
@@ -273,80 +262,82 @@ void by_chunk(int R, F&& run) {
     }
 }
 
-// P2M as a GEMM per (work item = leaf and <= 64 of its panels, 64-wide chunk
-// of rows r):  E[leaf][r][m] = sum_j W[j][m] * (a_j X[j][r]).
+// CTAs per SM the FP32 P2M and L2P are compiled for at orders <= 5: four
+// (64 registers, no spills) instead of the two that 90 registers allowed, so
+// more warps hide the latency of each staged slice's global loads.
+template <int N>
+constexpr int kMinCtas() {
+    return N <= 5 ? 4 : 1;
+}
+
+// FP32 P2M as a GEMM per (work item = leaf and <= 64 of its panels, chunk of
+// RW = 16, 32 or 64 rows r): E[leaf][r][m] = sum_j W[j][m] * (a_j X[j][r]).
 // The work items are the near-field items (64 panels each), so a leaf of a few
 // hundred panels spreads over several CTAs instead of serialising one: the
 // first item of a leaf writes E[leaf], each further item writes a partial
 // expansion at box index nbox + slot, and k_p2m_fix adds the partials in item
 // order (deterministic).
 // 256 threads; thread (tm, tr) holds nodes MI tm .. MI tm + MI - 1 and rows
-// 8 tr .. 8 tr + 7.  Panels are staged KP at a time.  Every row r < Rb and node
-// m < ns of the chunk is written (zeros outside r < R, m < n3).
-template <class T, int N>
-__global__ void __launch_bounds__(256, kMinCtas<T, N>())
-    k_p2m(DevPlan p, const int32_t* __restrict__ slot, const T* __restrict__ X, const T* __restrict__ W,
-          bool mul_area, T* __restrict__ E, int R, int Rb) {
-    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, MI = NS / 32;
-    constexpr int KP = sizeof(T) == 8 ? 16 : 32;  // panels per staged chunk (static shared memory <= 48 KB)
-    constexpr int QW = 64 + 16 / (int)sizeof(T);  // Qs row stride: 16-byte aligned rows
+// RT tr .. RT tr + RT - 1, RT = RW / 8.  Panels are staged 32 at a time.  Every
+// row r < Rb and node m < ns of the chunk is written (zeros outside r < R, m < n3).
+template <int N, int RW>
+__global__ void __launch_bounds__(256, kMinCtas<N>())
+    k_p2m32(DevPlan p, const int32_t* __restrict__ slot, const float* __restrict__ X, const float* __restrict__ W,
+            bool mul_area, float* __restrict__ E, int R, int Rb) {
+    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, MI = NS / 32, RT = RW / 8;
+    constexpr int KP = 32;       // panels per staged chunk
+    constexpr int QW = RW + 4;   // Qs row stride: 16-byte aligned rows
     const int it = blockIdx.x;
     const int t = p.item_leaf[it], r0 = p.item_row0[it];
-    const int rc = blockIdx.y * 64;
+    const int rc = blockIdx.y * RW;
     const int64_t lb = p.leaf_begin[t];
     const int64_t j0 = lb + r0, j1 = min(lb + r0 + kItemPanels, p.leaf_begin[t + 1]);
-    __shared__ T Ws[KP][NS + 1];
-    __shared__ __align__(16) T Qs[KP][QW];
+    __shared__ float Ws[KP][NS + 1];
+    __shared__ __align__(16) float Qs[KP][QW];
     const int tid = threadIdx.x, tm = tid >> 3, tr = tid & 7;
-    T acc[MI][8];
+    float acc[MI][RT];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = (T)0;
+        for (int j = 0; j < RT; ++j) acc[i][j] = 0.f;
     for (int64_t jb = j0; jb < j1; jb += KP) {
         const int cnt = (int)min((int64_t)KP, j1 - jb);
         __syncthreads();
         for (int e = tid; e < KP * NS; e += 256) {
             const int k = e / NS, m = e % NS;
-            Ws[k][m] = k < cnt ? W[(jb + k) * NS + m] : (T)0;
+            Ws[k][m] = k < cnt ? W[(jb + k) * NS + m] : 0.f;
         }
-        for (int e = tid; e < KP * 64; e += 256) {
-            const int k = e >> 6, r = e & 63;
-            Qs[k][r] = (k < cnt && rc + r < R) ? (mul_area ? (T)p.area[jb + k] : (T)1) * X[(jb + k) * R + rc + r]
-                                               : (T)0;
+        for (int e = tid; e < KP * RW; e += 256) {
+            const int k = e / RW, r = e % RW;
+            Qs[k][r] = (k < cnt && rc + r < R) ? (mul_area ? (float)p.area[jb + k] : 1.f) * X[(jb + k) * R + rc + r]
+                                               : 0.f;
         }
         __syncthreads();
         for (int k = 0; k < cnt; ++k) {
-            T a[MI], b[8];
+            float a[MI], b[RT];
 #pragma unroll
             for (int i = 0; i < MI; ++i) a[i] = Ws[k][MI * tm + i];
-            if constexpr (sizeof(T) == 4) {
-                const float4 b0 = *reinterpret_cast<const float4*>(&Qs[k][8 * tr]);
-                const float4 b1 = *reinterpret_cast<const float4*>(&Qs[k][8 * tr + 4]);
-                b[0] = b0.x, b[1] = b0.y, b[2] = b0.z, b[3] = b0.w, b[4] = b1.x, b[5] = b1.y, b[6] = b1.z, b[7] = b1.w;
-            } else {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const double2 v = *reinterpret_cast<const double2*>(&Qs[k][8 * tr + 2 * q]);
-                    b[2 * q] = v.x, b[2 * q + 1] = v.y;
-                }
+            for (int j = 0; j < RT; j += 2) {
+                const float2 v = *reinterpret_cast<const float2*>(&Qs[k][RT * tr + j]);
+                b[j] = v.x, b[j + 1] = v.y;
             }
 #pragma unroll
             for (int i = 0; i < MI; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
+                for (int j = 0; j < RT; ++j) acc[i][j] += a[i] * b[j];
         }
     }
     const int64_t box = slot[it] < 0 ? (int64_t)p.leaf_box0 + t : (int64_t)p.nbox + slot[it];
-    T* out = E + (box * Rb + rc) * NS;
+    float* out = E + (box * Rb + rc) * NS;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int r = 8 * tr + j;
+    for (int j = 0; j < RT; ++j) {
+        const int r = RT * tr + j;
         if (rc + r >= Rb) continue;
 #pragma unroll
         for (int i = 0; i < MI; ++i) {
             const int m = MI * tm + i;
-            out[(int64_t)r * NS + m] = (m < N3 && rc + r < R) ? acc[i][j] : (T)0;
+            out[(int64_t)r * NS + m] = (m < N3 && rc + r < R) ? acc[i][j] : 0.f;
         }
     }
 }
@@ -371,94 +362,112 @@ __global__ void __launch_bounds__(256) k_p2m_fix(int nbox, int leaf_box0, const 
     dst[0] = v0, dst[1] = v1, dst[2] = v2, dst[3] = v3;
 }
 
-// L2P as a GEMM per (work item = leaf and <= 64 of its panels, 64-wide chunk
-// of r):  Y[j][r] += coef * sum_m S_j[m] L[leaf][r][m],  S_j[m] = wx[a] wy[b]
-// wz[c] (the centroid's separable weights), or S_j = Wt[j] (times a_j if
-// mul_area) when explicit weights are given.
+// FP32 L2P as a GEMM per (work item = leaf and <= 64 of its panels, chunk of
+// RW = 16, 32 or 64 rows r): Y[j][r] += coef * sum_m S_j[m] L[leaf][r][m],
+// S_j[m] = wx[a] wy[b] wz[c] (the centroid's separable weights), or S_j = Wt[j]
+// (times a_j if mul_area) when explicit weights are given.
 // 256 threads; thread (tj, tr) holds panels 4 tj .. 4 tj + 3 and rows
-// 4 tr .. 4 tr + 3; nodes are staged 32 at a time.
-template <class T, int N>
-__global__ void __launch_bounds__(256, kMinCtas<T, N>())
-    k_l2p(DevPlan p, const T* __restrict__ L, const T* __restrict__ Wt, bool mul_area, double* __restrict__ Y, int R,
-          int Rb, double coef) {
-    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns;
-    constexpr int JP = kItemPanels, MK = 32, SW = 64 + 16 / (int)sizeof(T);
+// RT tr .. RT tr + RT - 1, RT = RW / 16; nodes are staged 32 at a time.
+template <int N, int RW>
+__global__ void __launch_bounds__(256, kMinCtas<N>())
+    k_l2p32(DevPlan p, const float* __restrict__ L, const float* __restrict__ Wt, bool mul_area,
+            double* __restrict__ Y, int R, int Rb, double coef) {
+    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, RT = RW / 16;
+    constexpr int JP = kItemPanels, MK = 32, SW = 64 + 4, LW = RW + 4;
     const int it = blockIdx.x;
     const int t = p.item_leaf[it], r0 = p.item_row0[it];
-    const int rc = blockIdx.y * 64;
+    const int rc = blockIdx.y * RW;
     const int64_t lb = p.leaf_begin[t];
     const int64_t jb = lb + r0;
     const int cnt = (int)min((int64_t)JP, p.leaf_begin[t + 1] - jb);
-    const T* src = L + ((int64_t)(p.leaf_box0 + t) * Rb + rc) * NS;
-    __shared__ T wv[JP][3 * N];
-    __shared__ __align__(16) T Ss[MK][SW];  // [node][panel]
-    __shared__ __align__(16) T Ls[MK][SW];  // [node][row]
+    const float* src = L + ((int64_t)(p.leaf_box0 + t) * Rb + rc) * NS;
+    __shared__ float wv[JP][3 * N];
+    __shared__ __align__(16) float Ss[MK][SW];  // [node][panel]
+    __shared__ __align__(16) float Ls[MK][LW];  // [node][row]
     const int tid = threadIdx.x, tj = tid >> 4, tr = tid & 15;
     if (!Wt)
         for (int e = tid; e < JP * 3 * N; e += 256) {
             const int jj = e / (3 * N);
-            wv[jj][e % (3 * N)] = jj < cnt ? (T)p.w1d[jb * 3 * N + e] : (T)0;
+            wv[jj][e % (3 * N)] = jj < cnt ? (float)p.w1d[jb * 3 * N + e] : 0.f;
         }
-    T acc[4][4];
+    float acc[4][RT];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[i][q] = (T)0;
+        for (int q = 0; q < RT; ++q) acc[i][q] = 0.f;
     for (int m0 = 0; m0 < N3; m0 += MK) {
         __syncthreads();
         for (int e = tid; e < JP * MK; e += 256) {
             const int jj = e / MK, mm = e % MK, m = m0 + mm;
-            T v = (T)0;
+            float v = 0.f;
             if (m < N3 && jj < cnt) {
                 v = Wt ? Wt[(jb + jj) * NS + m] : wv[jj][m / (N * N)] * wv[jj][N + (m / N) % N] * wv[jj][2 * N + m % N];
-                if (mul_area) v *= (T)p.area[jb + jj];
+                if (mul_area) v *= (float)p.area[jb + jj];
             }
             Ss[mm][jj] = v;
         }
-        for (int e = tid; e < 64 * MK; e += 256) {
+        for (int e = tid; e < RW * MK; e += 256) {
             const int mm = e % MK, r = e / MK;
-            Ls[mm][r] = (m0 + mm < N3 && rc + r < R) ? src[(int64_t)r * NS + m0 + mm] : (T)0;
+            Ls[mm][r] = (m0 + mm < N3 && rc + r < R) ? src[(int64_t)r * NS + m0 + mm] : 0.f;
         }
         __syncthreads();
 #pragma unroll 8
         for (int k = 0; k < MK; ++k) {
-            T a[4], b[4];
-            if constexpr (sizeof(T) == 4) {
-                const float4 av = *reinterpret_cast<const float4*>(&Ss[k][4 * tj]);
-                const float4 bv = *reinterpret_cast<const float4*>(&Ls[k][4 * tr]);
-                a[0] = av.x, a[1] = av.y, a[2] = av.z, a[3] = av.w;
-                b[0] = bv.x, b[1] = bv.y, b[2] = bv.z, b[3] = bv.w;
-            } else {
+            const float4 av = *reinterpret_cast<const float4*>(&Ss[k][4 * tj]);
+            const float a[4] = {av.x, av.y, av.z, av.w};
+            float b[RT];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const double2 av = *reinterpret_cast<const double2*>(&Ss[k][4 * tj + 2 * h]);
-                    const double2 bv = *reinterpret_cast<const double2*>(&Ls[k][4 * tr + 2 * h]);
-                    a[2 * h] = av.x, a[2 * h + 1] = av.y, b[2 * h] = bv.x, b[2 * h + 1] = bv.y;
-                }
-            }
+            for (int q = 0; q < RT; ++q) b[q] = Ls[k][RT * tr + q];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[i][q] += a[i] * b[q];
+                for (int q = 0; q < RT; ++q) acc[i][q] += a[i] * b[q];
         }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int jj = 4 * tj + i;
         if (jj >= cnt) continue;
-        double* y = Y + (jb + jj) * R + rc + 4 * tr;
-        if ((R & 1) == 0 && rc + 4 * tr + 3 < R) {  // 16-byte aligned pairs
+        double* y = Y + (jb + jj) * R + rc + RT * tr;
+        if (RT == 4 && rc + RT * tr + 3 < R) {  // R is a multiple of 4: 16-byte aligned pairs
             double2 y0 = *reinterpret_cast<double2*>(y), y1 = *reinterpret_cast<double2*>(y + 2);
-            y0.x += coef * (double)acc[i][0], y0.y += coef * (double)acc[i][1];
-            y1.x += coef * (double)acc[i][2], y1.y += coef * (double)acc[i][3];
+            y0.x += coef * (double)acc[i][0], y0.y += coef * (double)acc[i][RT > 1 ? 1 : 0];
+            y1.x += coef * (double)acc[i][RT > 2 ? 2 : 0], y1.y += coef * (double)acc[i][RT > 3 ? 3 : 0];
             *reinterpret_cast<double2*>(y) = y0;
             *reinterpret_cast<double2*>(y + 2) = y1;
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (rc + 4 * tr + q < R) y[q] += coef * (double)acc[i][q];
+            for (int q = 0; q < RT; ++q)
+                if (rc + RT * tr + q < R) y[q] += coef * (double)acc[i][q];
         }
     }
+}
+
+template <int N, int RW>
+void run_p2m32(Ctx& c, const DevPlan& p, const int32_t* slot, const float* X, const FarWeights<float>& w, float* E,
+               int R, int Rb) {
+    k_p2m32<N, RW><<<dim3(p.nitems, (Rb + RW - 1) / RW), 256, 0, c.stream>>>(p, slot, X, w.src, w.src_area, E, R, Rb);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+}
+
+template <int N, int RW>
+void run_l2p32(Ctx& c, const DevPlan& p, const float* L, const FarWeights<float>& w, double* Y, int R, int Rb,
+               double coef) {
+    k_l2p32<N, RW><<<dim3(p.nitems, (R + RW - 1) / RW), 256, 0, c.stream>>>(p, L, w.tgt, w.tgt_area, Y, R, Rb, coef);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+}
+
+// Column tile of the FP32 kernels for Rb = rhs_pad32(R) rows.
+template <class F>
+void by_rows32(int Rb, F&& run) {
+    if (Rb == 16)
+        run(std::integral_constant<int, 16>());
+    else if (Rb == 32)
+        run(std::integral_constant<int, 32>());
+    else
+        run(std::integral_constant<int, 64>());
 }
 
 // Rows of right-hand sides per M2M / L2L block.
@@ -842,29 +851,18 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
     const int Lv = p.L;
     const double wb = (double)sizeof(T);
     const double box_bytes = wb * N3 * R;
-    const unsigned rchunks64 = cdiv(Rb, 64), rchunks_tree = cdiv(Rb, RC);
+    const unsigned rchunks_tree = cdiv(Rb, RC);
     if (!l_written)
         launch_zero(c, L, (size_t)p.nbox * NS * Rb * sizeof(T));  // a kernel: also valid inside a device-side loop
     {
         KTimer t(c, prec_tag<T>(K_P2M), (double)p.N * (wb * R + wb * N3 + 8.0) + (p.nleaf + 2.0 * f.npart) * box_bytes,
                  2.0 * (double)p.N * N3 * R);
-        if constexpr (sizeof(T) == 4 && (N == 4 || N == 5)) {
-            if (p2m_tc) {
-                launch_p2m_tc(c, p, f.p2m_slot, p2m_tc->whi, p2m_tc->wlo, p2m_tc->xhi, p2m_tc->xlo,
-                              reinterpret_cast<float*>(E), R, Rb, p2m_tc->err);
-            } else {
-                k_p2m<T, N><<<dim3(p.nitems, rchunks64), 256, 0, s>>>(p, f.p2m_slot, X, w.src, w.src_area, E, R, Rb);
-                GPX_LAUNCH_CHECK();
-                c.launches += 1;
-            }
+        if constexpr (sizeof(T) == 8) {
+            by_chunk<N>(R, [&](auto nt) { run_p2m64<N, nt>(c, p, f.p2m_slot, X, w, E, R); });
+        } else if (p2m_tc && (N == 4 || N == 5)) {
+            launch_p2m_tc(c, p, f.p2m_slot, p2m_tc->whi, p2m_tc->wlo, p2m_tc->xhi, p2m_tc->xlo, E, R, Rb, p2m_tc->err);
         } else {
-            if constexpr (sizeof(T) == 8) {
-                by_chunk<N>(R, [&](auto nt) { run_p2m64<N, nt>(c, p, f.p2m_slot, X, w, E, R); });
-            } else {
-                k_p2m<T, N><<<dim3(p.nitems, rchunks64), 256, 0, s>>>(p, f.p2m_slot, X, w.src, w.src_area, E, R, Rb);
-                GPX_LAUNCH_CHECK();
-                c.launches += 1;
-            }
+            by_rows32(Rb, [&](auto rw) { run_p2m32<N, rw>(c, p, f.p2m_slot, X, w, E, R, Rb); });
         }
         if (f.nfix > 0) {
             const int64_t block = (int64_t)Rb * NS;
@@ -920,20 +918,12 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
     }
     {
         KTimer t(c, prec_tag<T>(K_L2P), (double)p.N * (16.0 * R + 24.0 * N) + p.nleaf * box_bytes, 2.0 * (double)p.N * N3 * R);
-        bool done = false;
-        if constexpr (sizeof(T) == 4 && (N == 4 || N == 5)) {
-            if (p2m_tc && p2m_tc->shi) {
-                launch_l2p_tc(c, p, reinterpret_cast<const float*>(L), p2m_tc->shi, p2m_tc->slo, Y, R, Rb, coef,
-                              p2m_tc->err);
-                done = true;
-            }
-        }
         if constexpr (sizeof(T) == 8) {
             by_chunk<N>(R, [&](auto nt) { run_l2p64<N, nt>(c, p, L, w, Y, R, coef); });
-        } else if (!done) {
-            k_l2p<T, N><<<dim3(p.nitems, cdiv(R, 64)), 256, 0, s>>>(p, L, w.tgt, w.tgt_area, Y, R, Rb, coef);
-            GPX_LAUNCH_CHECK();
-            c.launches += 1;
+        } else if (p2m_tc && p2m_tc->shi && (N == 4 || N == 5)) {
+            launch_l2p_tc(c, p, L, p2m_tc->shi, p2m_tc->slo, Y, R, Rb, coef, p2m_tc->err);
+        } else {
+            by_rows32(Rb, [&](auto rw) { run_l2p32<N, rw>(c, p, L, w, Y, R, Rb, coef); });
         }
     }
 }

@@ -105,24 +105,30 @@ template <>
 void launch_m2l_fac<float>(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const float* E, int R, int n3);
 
 // Tensor-core (tcgen05, TF32 inputs, FP32 accumulation) M2L work list of one
-// level: pairs of target boxes sharing one offset loop.
-// Target boxes per tensor-core M2L work item (of one octant class, so that
-// their interaction lists use the same offsets): 2, one TMEM accumulator.
-// Four boxes with two accumulators sharing each operator tile measured
-// slower on the bench window (0.385 against 0.309 ms per launch: half the
-// CTAs per SM by shared memory, and more zero-filled rows in the union of
-// four boxes' offsets).
-constexpr int kGroup = 2;
+// level: groups of target boxes sharing one offset loop.
+// An item holds 128 operand rows: 128 / Rb target boxes of one octant class
+// (so that their interaction lists use the same offsets) with Rb right-hand
+// sides each, Rb = 16, 32 or 64 (two boxes for a multiple of 64).  Four boxes
+// of 64 with two accumulators sharing each operator tile measured slower on
+// the bench window (0.385 against 0.309 ms per launch: half the CTAs per SM by
+// shared memory, and more zero-filled rows in the union of four boxes' offsets).
+inline int tc_group(int Rb) { return Rb >= 64 ? 2 : 128 / Rb; }
 struct TcLevel {
     int nitems = 0;
-    const int32_t* item_t = nullptr;    // kGroup per item: target boxes (trailing ones may be -1)
+    const int32_t* item_t = nullptr;    // tc_group per item: target boxes (trailing ones may be -1)
     const int32_t* item_off = nullptr;  // nitems + 1: entry ranges
     const int32_t* slot = nullptr;      // per entry: operator slot
-    const int32_t* src = nullptr;       // kGroup per entry: each target's source box at the slot's offset, or -1
+    const int32_t* src = nullptr;       // tc_group per entry: each target's source box at the slot's offset, or -1
 };
+// Rows of the FP32 expansions per box: R rounded up to 16, 32 or a multiple of
+// 64.  Every kernel of the FP32 far field moves and multiplies all of them; with
+// 64 always, a 12-column apply of a 21,038-panel bus took 0.53 ms in the far
+// field, with 16 it takes 0.32 ms.
+inline int rhs_pad32(int R) { return R <= 16 ? 16 : R <= 32 ? 32 : (R + 63) / 64 * 64; }
 // L[t][r][m] = scale * sum K[m][l] E[s][r][l] for order-4 (node stride 64)
 // or order-5 (node stride 128) expansions; K32: 343 x ns x ns TF32-rounded
-// operators; R a multiple of 64.  err receives a nonzero code if a bounded
+// operators; R (rows per box) 16, 32 or a multiple of 64, lists built for
+// tc_group(R).  err receives a nonzero code if a bounded
 // wait on the tensor-core pipeline expired.  box_scale (per box, may be null):
 // each target box's own scale, for launches that cover several levels.
 void launch_m2l_tc(Ctx& c, const TcLevel& lv, int ns, const float* E, float* L, const float* K32, int R, float scale,

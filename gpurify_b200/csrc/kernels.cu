@@ -71,12 +71,15 @@ __global__ void k_diag_inv(DevPlan p, const double* __restrict__ P, double* __re
 // right-hand sides, Y[rows][.] = P_t[rows][0:S] X[src(0:S)][.] on FP64 matrix
 // instructions.  KC source panels per stage go through a three-stage cp.async
 // ring: the item's P rows (contiguous along the contraction) and the gathered
-// X rows (contiguous along the right-hand sides).  Four warps: NT / NTW of
-// them side by side over the columns, the others (WK in all) over the
-// contraction, their partial tiles added in a fixed order at the end.  Narrow
-// chunks thus split the contraction instead of leaving warps without columns.
-// Row tiles past the item's rows are skipped, so a 12-row leaf costs 16 rows.
-// Pitches of 4 more than a multiple of 8 doubles keep fragment reads free of
+// X rows (contiguous along the right-hand sides).  Four warps: WN = NT / NTW of
+// them side by side over the columns, WM over the 8-row tiles (tile i belongs
+// to warp i % WM), so narrow chunks do not leave warps without work.  Row tiles
+// past the item's rows are skipped: a 12-row leaf costs 16 rows.  One warp runs
+// the whole contraction of an output, in ascending order, and the instruction
+// itself is the ascending chain of fused multiply-adds, so every result has
+// the bits of a scalar loop: the mixed path's inner solves, whose TF32 far
+// field truncates, turn any other rounding of the residual into another
+// iterate.  Pitches of 4 more than a multiple of 8 doubles keep fragment reads free of
 // bank conflicts.  P rows are padded to a multiple of 4 entries and R is a
 // multiple of 4, so every 16-byte copy is aligned.
 // Bound: the FP64 rate from R = 32 up (2 R flop per 8-byte entry), below it
@@ -88,17 +91,17 @@ __global__ void k_diag_inv(DevPlan p, const double* __restrict__ P, double* __re
 template <int NT>
 struct NearMma {
     static constexpr int NTW = NT % 3 == 0 ? 3 : NT == 1 ? 1 : 2;  // column tiles per warp
-    static constexpr int WN = NT / NTW, WK = 4 / WN;
+    static constexpr int WN = NT / NTW, WM = 4 / WN;
     static constexpr int KC = NT <= 3 ? 32 : 16, S = NT == 8 ? 2 : 3;
-    static constexpr int kMinCtas = NT == 8 ? 4 : 2;
     static constexpr int PP = KC + 4, XP = 8 * NT + 4;
+    static constexpr int kMinCtas = NT == 8 ? 4 : 2;
 };
 template <int NT>
 __global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(DevPlan p, const double* __restrict__ P,
                                                         const double* __restrict__ X, double* __restrict__ Y, int R,
                                                         int tile_rows) {
     using C = NearMma<NT>;
-    constexpr int NTW = C::NTW, WK = C::WK, KC = C::KC, S = C::S, PP = C::PP, XP = C::XP;
+    constexpr int NTW = C::NTW, WM = C::WM, MT = 8 / WM, KC = C::KC, S = C::S, PP = C::PP, XP = C::XP;
     const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int rc = blockIdx.y * (8 * NT);
     const int64_t tb = p.leaf_begin[t] + r0;
@@ -140,10 +143,10 @@ __global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(D
         }
         cp_async_fence();
     };
-    const int wn = warp % C::WN, wk = warp / C::WN;
-    double acc[8][NTW][2];
+    const int wn = warp % C::WN, wm = warp / C::WN;
+    double acc[MT][NTW][2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int j = 0; j < NTW; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
@@ -152,54 +155,28 @@ __global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(D
         cp_async_wait_for<S - 2>();
         __syncthreads();
         issue(st + S - 1);
-        const double* ps = Ps + (st % S) * tile_rows * PP + g * PP + q;
+        const double* ps = Ps + (st % S) * tile_rows * PP + (8 * wm + g) * PP + q;
         const double* xs = Xs + (st % S) * KC * XP + q * XP + 8 * NTW * wn + g;
 #pragma unroll
-        for (int k = 4 * wk; k < KC; k += 4 * WK) {
+        for (int k = 0; k < KC; k += 4) {
             double b[NTW];
 #pragma unroll
             for (int j = 0; j < NTW; ++j) b[j] = xs[k * XP + 8 * j];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i < mt) {
+            for (int i = 0; i < MT; ++i)
+                if (wm + WM * i < mt) {
                     // rows m .. 8 mt - 1 of the last tile hold leftovers of
                     // other stages or items: their outputs are never stored
-                    const double a = ps[8 * i * PP + k];
+                    const double a = ps[8 * WM * i * PP + k];
 #pragma unroll
                     for (int j = 0; j < NTW; ++j) dmma(acc[i][j], a, b[j]);
                 }
         }
     }
     cp_async_wait_for<0>();
-    if constexpr (WK > 1) {
-        // partial tiles of the warps wk >= 1 through shared memory
-        __syncthreads();
-        double2* red = reinterpret_cast<double2*>(near_smem);  // [(WK - 1) WN][mt][NTW][32]
-        if (wk > 0)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i < mt)
-#pragma unroll
-                    for (int j = 0; j < NTW; ++j)
-                        red[((((wk - 1) * C::WN + wn) * mt + i) * NTW + j) * 32 + lane] =
-                            make_double2(acc[i][j][0], acc[i][j][1]);
-        __syncthreads();
-        if (wk > 0) return;
-#pragma unroll
-        for (int w = 0; w < WK - 1; ++w)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i < mt)
-#pragma unroll
-                    for (int j = 0; j < NTW; ++j) {
-                        const double2 v = red[(((w * C::WN + wn) * mt + i) * NTW + j) * 32 + lane];
-                        acc[i][j][0] += v.x;
-                        acc[i][j][1] += v.y;
-                    }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = 8 * i + g;
+    for (int i = 0; i < MT; ++i) {
+        const int row = 8 * (wm + WM * i) + g;
         if (row >= m) continue;
 #pragma unroll
         for (int j = 0; j < NTW; ++j) {

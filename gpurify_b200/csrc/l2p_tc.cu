@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
     const uint32_t tmem = *tslot;
     // copies of slice q into stage q % 2: A rows = the item's panels (rows
     // past cnt are not loaded: their D rows are never stored), B rows = the
-    // leaf's right-hand sides (all 64 rows valid: L has Rb rows per box)
+    // leaf's right-hand sides (L has Rb rows per box; the chunk's others are zero)
     auto issue = [&](int q) {
         const uint32_t a = base + (uint32_t)(q & 1) * kStage;
         for (int e = tid; e < 64 * 8; e += kThreads) {
@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
                 cp16(a + swz(row, c), Shi + off, true);
                 cp16(a + kATile + swz(row, c), Slo + off, true);
             }
-            cp16(a + 2 * kATile + swz(row, c), src + (int64_t)row * NS + 32 * q + 4 * c, true);
+            const bool have = rc + row < Rb;
+            cp16(a + 2 * kATile + swz(row, c), have ? src + (int64_t)row * NS + 32 * q + 4 * c : L, have);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
 void launch_l2p_tc(Ctx& c, const DevPlan& p, const float* L, const float* Shi, const float* Slo, double* Y, int R,
                    int Rb, double coef, int* err) {
     if (p.nitems == 0) return;
-    if (R % 4 != 0 || Rb % 64 != 0) throw Error(GPX_ERR_INTERNAL, "tensor-core L2P needs R % 4 == 0, Rb % 64 == 0");
+    if (R % 4 != 0 || Rb % 16 != 0) throw Error(GPX_ERR_INTERNAL, "tensor-core L2P needs R % 4 == 0, Rb % 16 == 0");
     const dim3 grid(p.nitems, (R + 63) / 64);
     if (p.ns == 128) {
         set_smem_once(k_l2p_tc<128>, (int)kSmemBytes);

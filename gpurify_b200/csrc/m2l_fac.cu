@@ -12,12 +12,13 @@
 // the plan's upload).
 //
 // FP64 runs on mma.sync (dmma.cuh) with column tiles that follow R, FP32 on
-// the CUDA cores.  One FP64 apply (both phases), against the 64-column
+// the CUDA cores with 16-, 32- or 64-column tiles (31,940 box pairs, R = 16:
+// 0.22 ms per FP32 apply, 0.54 with 64 columns).  One FP64 apply (both phases), against the 64-column
 // FMA tiles it replaced:
-//   order 5, R = 64, 62,802 box pairs:  1.04 ms (1.98 before; 0.8 at the FP64 rate)
-//   order 6, R = 24, 96,750 box pairs:  1.35 ms (6.23)
-//   order 5, R = 16, 31,940 box pairs:  0.21 ms (0.95)
-//   order 4, R = 4, 4,528 box pairs:    32 us (135)
+//   order 5, R = 64, 62,802 box pairs:  1.05 ms (1.98 before; 0.8 at the FP64 rate)
+//   order 6, R = 24, 96,750 box pairs:  1.38 ms (6.23)
+//   order 5, R = 16, 31,940 box pairs:  0.22 ms (0.95)
+//   order 4, R = 4, 4,528 box pairs:    34 us (135)
 #include "dmma.cuh"
 #include "farfield.cuh"
 
@@ -56,10 +57,9 @@ __device__ __forceinline__ void expand_target(const FacM2L<T>& f, int t, uint16_
 // right-hand sides).  The source expansion (8 NT rows of ns nodes) is staged
 // once in shared memory; each warp takes blocks of 8 MT columns and reads
 // their Vt rows, which no other warp of the item needs, straight into
-// registers, two 8-node steps ahead.  Both operands are contiguous along the
-// contraction: a lane reads nodes 2q, 2q + 1 (q = lane % 4) as one 16-byte
-// load, feeding two instructions (nodes 2q, then 2q + 1, of each 8).  The row
-// pitch ns + 8 spreads a quarter-warp's 16-byte reads over all banks.
+// registers, two 8-node steps ahead.  The row pitch ns + 4 puts the 4 nodes of
+// 4 rows in distinct banks.  Nodes are contracted in ascending order (see the
+// near apply in kernels.cu).
 // Bound: FP64 tensor rate at R = 64 (per column 2 n^3 R flop against 8 n^3
 // bytes of Vt from L2); L2 at R <= 16.
 template <int NT, int MT>
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(128) k_fac_v64(FacM2L<double> f, const FacItem
                                                  const double* __restrict__ E, int R, int ksteps) {
     const FacItem it = items[blockIdx.x];
     const int rc = blockIdx.y * (8 * NT);
-    const int rows = min(8 * NT, R - rc), ns = f.ns, pitch = ns + 8;
+    const int rows = min(8 * NT, R - rc), ns = f.ns, pitch = ns + 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* Es = reinterpret_cast<double*>(smem_raw);                       // [8 NT][pitch]
     int64_t* col_t = reinterpret_cast<int64_t*>(Es + 8 * NT * pitch);       // [kFacItemCols]
@@ -84,42 +84,47 @@ __global__ void __launch_bounds__(128) k_fac_v64(FacM2L<double> f, const FacItem
     cp_async_wait_for<0>();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = lane >> 2, q = lane & 3;
-    const double* eb = Es + row * pitch + 2 * q;
+    const double* eb = Es + row * pitch + q;
     for (int c0 = warp * 8 * MT; c0 < ncols; c0 += 4 * 8 * MT) {
         const double* a_ptr[MT];
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
             const int c = min(c0 + 8 * i + row, ncols - 1);  // rows past the end repeat the last column, never stored
-            a_ptr[i] = f.Vt + (int64_t)col_vt[c] * ns + 2 * q;
+            a_ptr[i] = f.Vt + (int64_t)col_vt[c] * ns + q;
         }
         double acc[MT][NT][2];
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
             for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-        double2 a[2][MT];  // the next two steps (ksteps >= 1; rows hold ns >= 32 nodes, so step 1 is readable)
+        double a[2][MT][2];  // the next two 8-node steps (rows hold ns >= 32 nodes, so step 1 is readable)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < MT; ++i) a[h][i] = __ldg(reinterpret_cast<const double2*>(a_ptr[i] + 8 * h));
+            for (int i = 0; i < MT; ++i) {
+                a[h][i][0] = __ldg(a_ptr[i] + 8 * h);
+                a[h][i][1] = __ldg(a_ptr[i] + 8 * h + 4);
+            }
 #pragma unroll 2
         for (int s = 0; s < ksteps; ++s) {
-            double2 cur[MT];
+            double cur[MT][2];
             const int nx = min(s + 2, ksteps - 1);
 #pragma unroll
-            for (int i = 0; i < MT; ++i) {
-                cur[i] = a[0][i];
-                a[0][i] = a[1][i];
-                a[1][i] = __ldg(reinterpret_cast<const double2*>(a_ptr[i] + 8 * nx));
-            }
+            for (int i = 0; i < MT; ++i)
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                const double2 b = *reinterpret_cast<const double2*>(eb + 8 * j * pitch + 8 * s);
+                for (int h = 0; h < 2; ++h) {
+                    cur[i][h] = a[0][i][h];
+                    a[0][i][h] = a[1][i][h];
+                    a[1][i][h] = __ldg(a_ptr[i] + 8 * nx + 4 * h);
+                }
 #pragma unroll
-                for (int i = 0; i < MT; ++i) dmma(acc[i][j], cur[i].x, b.x);
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int i = 0; i < MT; ++i) dmma(acc[i][j], cur[i].y, b.y);
-            }
+                for (int j = 0; j < NT; ++j) {
+                    const double b = eb[8 * j * pitch + 8 * s + 4 * h];
+#pragma unroll
+                    for (int i = 0; i < MT; ++i) dmma(acc[i][j], cur[i][h], b);
+                }
         }
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
@@ -229,21 +234,21 @@ __global__ void __launch_bounds__(NS, (FacU64<NT, NS>::kMinCtas))
     }
 }
 
-// Phase 1, FP32: a transposed GEMM per (source item, 64 right-hand sides),
+// Phase 1, FP32: a transposed GEMM per (source item, 8 RI right-hand sides),
 // C[c][r] = sum_l Vt_c[l] E_s[r][l].  E_s^T (B) is staged once per item; the
 // gathered Vt rows (A) of each CT-column sub-block stream through a cp.async
-// double buffer over the ns nodes.  CT threads, 8 x 8 outputs per thread
+// double buffer over the ns nodes.  CT threads, 8 x RI outputs per thread
 // (columns ty + (CT/8) i, rows tx + 8 j).
-template <int CT>
+template <int CT, int RI>
 __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* __restrict__ items,
                                                 const float* __restrict__ E, int R) {
     constexpr int V = 4, KC = 32, PP = KC + V;
-    constexpr int BP = 64 + 1;  // odd pitch: the transposed staging stores hit distinct banks
+    constexpr int BP = 8 * RI + 1;  // odd pitch: the transposed staging stores hit distinct banks
     constexpr int CS = CT / 8;  // column stride of a thread's tile
     const int ns = f.ns;
     const FacItem it = items[blockIdx.x];
-    const int rc = blockIdx.y * 64;
-    const int rows = min(64, R - rc);
+    const int rc = blockIdx.y * (8 * RI);
+    const int rows = min(8 * RI, R - rc);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float(*As)[CT][PP] = reinterpret_cast<float(*)[CT][PP]>(smem_raw);  // [2][CT][PP]: [c][l]
     int64_t* col_t = reinterpret_cast<int64_t*>(smem_raw + sizeof(float) * 2 * CT * PP);
@@ -270,18 +275,18 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
     };
     issue(0);
     const float* Es = E + ((int64_t)it.src * R + rc) * ns;
-    for (int e = tid; e < 64 * ns; e += CT) {
+    for (int e = tid; e < 8 * RI * ns; e += CT) {
         const int r = e / ns, l = e % ns;
         Bs[l][r] = r < rows ? Es[(int64_t)r * ns + l] : 0.f;
     }
-    float acc[8][8];
+    float acc[8][RI];
     for (int step = 0; step < nsteps; ++step) {
         const int sub = step / nch, ch = step % nch;
         if (ch == 0) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+                for (int j = 0; j < RI; ++j) acc[i][j] = 0.f;
         }
         __syncthreads();
         if (step + 1 < nsteps) {
@@ -294,15 +299,15 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
         const int buf = step & 1;
 #pragma unroll 4
         for (int kk = 0; kk < KC; ++kk) {
-            float a[8], b[8];
+            float a[8], b[RI];
 #pragma unroll
             for (int i = 0; i < 8; ++i) a[i] = As[buf][ty + CS * i][kk];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) b[j] = Bs[ch * KC + kk][tx + 8 * j];
+            for (int j = 0; j < RI; ++j) b[j] = Bs[ch * KC + kk][tx + 8 * j];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
+                for (int j = 0; j < RI; ++j) acc[i][j] += a[i] * b[j];
         }
         if (ch == nch - 1) {
             const int nc = min(CT, ncols - CT * sub);
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
                 if (c >= nc) continue;
                 float* dst = f.Tm + col_t[CT * sub + c] * R + rc;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < RI; ++j) {
                     const int r = tx + 8 * j;
                     if (r < rows) dst[r] = acc[i][j];
                 }
@@ -321,21 +326,21 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
     }
 }
 
-// Phase 2, FP32: CTA per (target box, 64 rows r, MW nodes m), MW threads, 8 x
+// Phase 2, FP32: CTA per (target box, 8 RI rows r, MW nodes m), MW threads, RI x
 // 8 outputs per thread (rows ty + 8 i, nodes tx + (MW/8) j); the contraction
 // over the target's concatenated ranks streams A = T rows and B = gathered Ut
 // rows through a cp.async double buffer.  L is written, not added to.
-template <int MW>
+template <int MW, int RI>
 __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* __restrict__ L, int R) {
-    constexpr int V = 4, KC = 32, XP = MW + V, AP = 64 + V, TXN = MW / 8;
+    constexpr int V = 4, KC = 32, XP = MW + V, RW = 8 * RI, AP = RW + V, TXN = MW / 8;
     const int ns = f.ns;
     const int t = b0 + blockIdx.x;
-    const int rc = blockIdx.y * 64;
+    const int rc = blockIdx.y * RW;
     const int m0 = blockIdx.z * MW;
     const int K = (int)(f.tgt_col_off[t + 1] - f.tgt_col_off[t]);
     const float sc = (float)f.box_scale[t];
     const float* A = f.Tm + f.tgt_base[t] * R + rc;  // column-major: A[c][r] at c * R + r
-    const int m = min(64, R - rc);
+    const int m = min(RW, R - rc);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float(*As)[KC][AP] = reinterpret_cast<float(*)[KC][AP]>(smem_raw);                             // [2][KC][AP]: [c][r]
     float(*Bs)[KC][XP] = reinterpret_cast<float(*)[KC][XP]>(smem_raw + sizeof(float) * 2 * KC * AP);  // [2][KC][XP]
@@ -344,8 +349,8 @@ __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* 
     const int nchunk = (K + KC - 1) / KC;
     auto issue = [&](int cch) {
         const int k0 = cch * KC, buf = cch & 1;
-        for (int id = tid; id < KC * (64 / V); id += MW) {
-            const int kk = id / (64 / V), rr = (id % (64 / V)) * V;
+        for (int id = tid; id < KC * (RW / V); id += MW) {
+            const int kk = id / (RW / V), rr = (id % (RW / V)) * V;
             const bool ok = k0 + kk < K && rr < m;
             cp_async_16(&As[buf][kk][rr], ok ? A + (int64_t)(k0 + kk) * R + rr : f.Tm, ok);
         }
@@ -356,9 +361,9 @@ __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* 
         }
         cp_async_fence();
     };
-    float acc[8][8];
+    float acc[RI][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     if (K > 0) {
@@ -378,19 +383,19 @@ __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* 
         const int buf = cch & 1;
 #pragma unroll 4
         for (int kk = 0; kk < KC; ++kk) {
-            float a[8], b[8];
+            float a[RI], b[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = As[buf][kk][ty + 8 * i];
+            for (int i = 0; i < RI; ++i) a[i] = As[buf][kk][ty + 8 * i];
 #pragma unroll
             for (int j = 0; j < 8; ++j) b[j] = Bs[buf][kk][tx + TXN * j];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < RI; ++i) {
         const int r = ty + 8 * i;
         if (r >= m) continue;
 #pragma unroll
@@ -414,7 +419,7 @@ template <int NT>
 void run_fac64(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, const double* E, int R, int n3) {
     constexpr int MT = NT >= 6 ? 2 : NT == 5 ? 3 : 4;  // at most 16 accumulator tiles a warp
     if (f.nitems > 0) {
-        const int smem = (int)(sizeof(double) * 8 * NT * (f.ns + 8) + 12 * kFacItemCols);
+        const int smem = (int)(sizeof(double) * 8 * NT * (f.ns + 4) + 12 * kFacItemCols);
         set_smem_once(k_fac_v64<NT, MT>, smem);
         k_fac_v64<NT, MT><<<dim3(f.nitems, cdiv(R, 8 * NT)), 128, smem, c.stream>>>(f, f.items, E, R, (n3 + 7) / 8);
         GPX_LAUNCH_CHECK();
@@ -426,6 +431,30 @@ void run_fac64(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, const
         default:
             if constexpr (NT <= 4) run_fac_u64<NT, 224>(c, f, b0, nb, L, R);
     }
+}
+
+template <int RI>
+void run_fac32(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const float* E, int R) {
+    constexpr int V = 4, KC = 32, CT = 128, RW = 8 * RI;
+    if (f.nitems > 0) {
+        const int smem = (int)(sizeof(float) * (2 * CT * (KC + V) + f.ns * (RW + 1)) + 12 * kFacItemCols);
+        set_smem_once(k_fac_v32<CT, RI>, smem);
+        k_fac_v32<CT, RI><<<dim3(f.nitems, cdiv(R, RW)), CT, smem, c.stream>>>(f, f.items, E, R);
+        GPX_LAUNCH_CHECK();
+    }
+    const int cols = 2 * ((f.max_cols + 7) & ~7);
+    if (f.ns >= 128) {
+        constexpr int MW = 128;
+        const int smem = (int)(sizeof(float) * 2 * KC * (RW + V + MW + V)) + cols;
+        set_smem_once(k_fac_u32<MW, RI>, smem);
+        k_fac_u32<MW, RI><<<dim3(nb, cdiv(R, RW), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
+    } else {
+        constexpr int MW = 64;
+        const int smem = (int)(sizeof(float) * 2 * KC * (RW + V + MW + V)) + cols;
+        set_smem_once(k_fac_u32<MW, RI>, smem);
+        k_fac_u32<MW, RI><<<dim3(nb, cdiv(R, RW), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
+    }
+    GPX_LAUNCH_CHECK();
 }
 
 }  // namespace
@@ -447,28 +476,15 @@ void launch_m2l_fac<double>(Ctx& c, const FacM2L<double>& f, int b0, int nb, dou
     c.launches += 1;  // the caller counts the other one
 }
 
+// R: rows per box, padded to 16, 32 or a multiple of 64 (rhs_pad32).
 template <>
 void launch_m2l_fac<float>(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const float* E, int R, int) {
-    constexpr int V = 4, KC = 32, CT = 128;
-    if (f.nitems > 0) {
-        const int smem = (int)(sizeof(float) * (2 * CT * (KC + V) + f.ns * (64 + 1)) + 12 * kFacItemCols);
-        set_smem_once(k_fac_v32<CT>, smem);
-        k_fac_v32<CT><<<dim3(f.nitems, cdiv(R, 64)), CT, smem, c.stream>>>(f, f.items, E, R);
-        GPX_LAUNCH_CHECK();
-    }
-    const int cols = 2 * ((f.max_cols + 7) & ~7);
-    if (f.ns >= 128) {
-        constexpr int MW = 128;
-        const int smem = (int)(sizeof(float) * 2 * KC * (64 + V + MW + V)) + cols;
-        set_smem_once(k_fac_u32<MW>, smem);
-        k_fac_u32<MW><<<dim3(nb, cdiv(R, 64), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
-    } else {
-        constexpr int MW = 64;
-        const int smem = (int)(sizeof(float) * 2 * KC * (64 + V + MW + V)) + cols;
-        set_smem_once(k_fac_u32<MW>, smem);
-        k_fac_u32<MW><<<dim3(nb, cdiv(R, 64), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
-    }
-    GPX_LAUNCH_CHECK();
+    if (R <= 16)
+        run_fac32<2>(c, f, b0, nb, L, E, R);
+    else if (R <= 32)
+        run_fac32<4>(c, f, b0, nb, L, E, R);
+    else
+        run_fac32<8>(c, f, b0, nb, L, E, R);
     c.launches += 1;  // the caller counts the other one
 }
 

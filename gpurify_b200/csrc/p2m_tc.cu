@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(kThreads) k_p2m_tc(DevPlan p, const int32_t* _
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (m < NS) {
 #pragma unroll
-                for (int k = 0; k < 16; ++k) out[(int64_t)(cb * 16 + k) * NS] = __uint_as_float(v[k]);
+                for (int k = 0; k < 16; ++k)
+                    if (rc + cb * 16 < Rb) out[(int64_t)(cb * 16 + k) * NS] = __uint_as_float(v[k]);
             }
         }
     }
@@ -230,8 +231,8 @@ void launch_split_weights(Ctx& c, const double* W, int ns, const double* area, b
 void launch_p2m_tc(Ctx& c, const DevPlan& p, const int32_t* slot, const float* Whi, const float* Wlo, const float* Xhi,
                    const float* Xlo, float* E, int R, int Rb, int* err) {
     if (p.nitems == 0) return;
-    if (R % 4 != 0 || Rb % 64 != 0) throw Error(GPX_ERR_INTERNAL, "tensor-core P2M needs R % 4 == 0, Rb % 64 == 0");
-    const dim3 grid(p.nitems, Rb / 64);
+    if (R % 4 != 0 || Rb % 16 != 0) throw Error(GPX_ERR_INTERNAL, "tensor-core P2M needs R % 4 == 0, Rb % 16 == 0");
+    const dim3 grid(p.nitems, (Rb + 63) / 64);
     if (p.ns == 128) {
         set_smem_once(k_p2m_tc<128>, (int)kSmemBytes);
         k_p2m_tc<128><<<grid, kThreads, kSmemBytes, c.stream>>>(p, slot, Whi, Wlo, Xhi, Xlo, E, R, Rb, err);

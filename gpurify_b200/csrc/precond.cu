@@ -87,17 +87,14 @@ __global__ void __launch_bounds__(256) k_block_invert(DevPlan p, const double* _
 
 // Z[rows] = Minv V[rows] on FP64 matrix instructions, one CTA per (block,
 // chunk of 8 NT columns).  The block's V rows are staged; each warp takes 16
-// rows of the inverse at a time, read once, straight into registers (a lane's
-// 16 bytes hold columns k + 2q and k + 2q + 1, q = lane % 4, for two
-// instructions).  The pitch 8 NT + 2 puts V rows k, k + 2, k + 4, k + 6 in
-// distinct banks.  Only the block's own rows and columns are read and
+// rows of the inverse at a time, read once, straight into registers.  Only the block's own rows and columns are read and
 // multiplied (a 12-panel leaf costs 16 x 16, not 96 x 96).
 template <int kB, int NT>
 __global__ void __launch_bounds__(128) k_block_apply(const double* __restrict__ Minv,
                                                      const int64_t* __restrict__ blk_start,
                                                      const int32_t* __restrict__ blk_size, const double* __restrict__ V,
                                                      DevIndex di, double* __restrict__ Z, int R, int add) {
-    constexpr int VP = 8 * NT + 2;
+    constexpr int VP = 8 * NT + 4;
     V = dev_offset(V, di);
     const int bi = blockIdx.x;
     const int rc = blockIdx.y * (8 * NT), cols = min(8 * NT, R - rc);
@@ -112,7 +109,7 @@ __global__ void __launch_bounds__(128) k_block_apply(const double* __restrict__ 
     }
     cp_async_fence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
-    const double* M = Minv + (int64_t)bi * kB * kB + 2 * q;
+    const double* M = Minv + (int64_t)bi * kB * kB + q;
     cp_async_wait_for<0>();
     __syncthreads();
     for (int i0 = 16 * warp; i0 < b; i0 += 64) {
@@ -122,24 +119,28 @@ __global__ void __launch_bounds__(128) k_block_apply(const double* __restrict__ 
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-        double2 nx[2];
+        double nx[2][2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) nx[i] = __ldg(reinterpret_cast<const double2*>(m0 + 8 * i * kB));
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) nx[i][h] = __ldg(m0 + 8 * i * kB + 4 * h);
         for (int k = 0; k < b8; k += 8) {
-            double2 a[2];
+            double a[2][2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                a[i] = nx[i];
-                nx[i] = __ldg(reinterpret_cast<const double2*>(m0 + 8 * i * kB + min(k + 8, kB - 8)));
-            }
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                const double v0 = Vs[(k + 2 * q) * VP + 8 * j + g], v1 = Vs[(k + 2 * q + 1) * VP + 8 * j + g];
+                for (int h = 0; h < 2; ++h) {
+                    a[i][h] = nx[i][h];
+                    nx[i][h] = __ldg(m0 + 8 * i * kB + min(k + 8, kB - 8) + 4 * h);
+                }
 #pragma unroll
-                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].x, v0);
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i].y, v1);
-            }
+                for (int j = 0; j < NT; ++j) {
+                    const double v = Vs[(k + 4 * h + q) * VP + 8 * j + g];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) dmma(acc[i][j], a[i][h], v);
+                }
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -319,7 +320,7 @@ void BlockJacobi::check(Ctx& c) const {
 
 template <int kB, int NT>
 static void block_apply(Ctx& c, const BlockJacobi& bj, const double* V, double* Z, int R, bool add, const DevIndex& di) {
-    const int smem = (int)sizeof(double) * kB * (8 * NT + 2);
+    const int smem = (int)sizeof(double) * kB * (8 * NT + 4);
     set_smem_once(k_block_apply<kB, NT>, smem);
     k_block_apply<kB, NT><<<dim3(bj.nblk, (R + 8 * NT - 1) / (8 * NT)), 128, smem, c.stream>>>(
         bj.Minv.p, bj.d_start.p, bj.d_size.p, V, di, Z, R, add ? 1 : 0);

@@ -347,7 +347,7 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
     d.far.m2l_off = p.m2l_off.data();
 }
 
-// Tensor-core M2L work lists of every level (groups of kGroup target boxes of
+// Tensor-core M2L work lists of every level (groups of tc_group target boxes of
 // the same octant class in Morton order sharing one offset loop).
 struct TcLists {
     std::vector<TcLevel> level;  // per level (empty below 2)
@@ -355,7 +355,7 @@ struct TcLists {
     DBuf<int32_t> item_t, item_off, slot, src;
 };
 
-void build_tc_lists(Ctx& ctx, const Plan& pl, TcLists& out) {
+void build_tc_lists(Ctx& ctx, const Plan& pl, int group, TcLists& out) {
     std::vector<int32_t> it, ioff, sl, src;
     struct LevelRange {
         size_t it0, off0;
@@ -363,7 +363,7 @@ void build_tc_lists(Ctx& ctx, const Plan& pl, TcLists& out) {
     };
     std::vector<LevelRange> ranges(pl.L + 1, {0, 0, 0});
     for (int l = 2; l <= pl.L; ++l) {
-        ranges[l].it0 = it.size() / kGroup;
+        ranges[l].it0 = it.size() / group;
         ranges[l].off0 = ioff.size();
         std::vector<int32_t> cls[8];
         for (int32_t b = pl.lvl_off[l]; b < pl.lvl_off[l + 1]; ++b) {
@@ -372,24 +372,24 @@ void build_tc_lists(Ctx& ctx, const Plan& pl, TcLists& out) {
             cls[(c[0] & 1) | ((c[1] & 1) << 1) | ((c[2] & 1) << 2)].push_back(b);
         }
         int n = 0;
-        std::vector<int32_t> per((size_t)kGroup * 343);
+        std::vector<int32_t> per((size_t)group * 343);
         for (auto& v : cls)
-            for (size_t k = 0; k < v.size(); k += kGroup) {
-                std::fill(per.begin(), per.end(), -1);  // per[slot * kGroup + i]
-                for (int i = 0; i < kGroup; ++i) {
+            for (size_t k = 0; k < v.size(); k += group) {
+                std::fill(per.begin(), per.end(), -1);  // per[slot * group + i]
+                for (int i = 0; i < group; ++i) {
                     const int32_t t = k + i < v.size() ? v[k + i] : -1;
                     it.push_back(t);
                     if (t < 0) continue;
                     for (int64_t e = pl.m2l_off[t]; e < pl.m2l_off[t + 1]; ++e)
-                        per[(size_t)pl.m2l_slot[e] * kGroup + i] = pl.m2l_src[e];
+                        per[(size_t)pl.m2l_slot[e] * group + i] = pl.m2l_src[e];
                 }
                 ioff.push_back((int32_t)sl.size());
                 for (int q = 0; q < 343; ++q) {
                     bool any = false;
-                    for (int i = 0; i < kGroup; ++i) any = any || per[(size_t)q * kGroup + i] >= 0;
+                    for (int i = 0; i < group; ++i) any = any || per[(size_t)q * group + i] >= 0;
                     if (!any) continue;
                     sl.push_back(q);
-                    for (int i = 0; i < kGroup; ++i) src.push_back(per[(size_t)q * kGroup + i]);
+                    for (int i = 0; i < group; ++i) src.push_back(per[(size_t)q * group + i]);
                 }
                 ++n;
             }
@@ -405,7 +405,7 @@ void build_tc_lists(Ctx& ctx, const Plan& pl, TcLists& out) {
     for (int l = 2; l <= pl.L; ++l) {
         TcLevel& v = out.level[l];
         v.nitems = ranges[l].n;
-        v.item_t = out.item_t.p + (size_t)kGroup * ranges[l].it0;
+        v.item_t = out.item_t.p + (size_t)group * ranges[l].it0;
         v.item_off = out.item_off.p + ranges[l].off0;
         v.slot = out.slot.p;
         v.src = out.src.p;
@@ -645,7 +645,7 @@ struct Operator {
             tc_err.zero();
             if (has_far()) {
                 const int ns = node_stride(pl.n);
-                Rb32 = (R + 63) / 64 * 64;
+                Rb32 = rhs_pad32(R);
                 E32.alloc((size_t)(pl.nbox() + d.far.npart) * ns * Rb32, s);
                 L32.alloc((size_t)pl.nbox() * ns * Rb32, s);
                 W32.alloc((size_t)pl.N * node_stride(pl.n), s);
@@ -674,7 +674,7 @@ struct Operator {
                         launch_split_weights(ctx, d.wsrc.p, ns, d.area.p, true, Shi32.p, Slo32.p, pl.N);
                     }
                 }
-                if (tc32 || shared) build_tc_lists(ctx, pl, tc);
+                if (tc32 || shared) build_tc_lists(ctx, pl, tc_group(Rb32), tc);
                 if (shared) {
                     ensure_shared(ctx, *const_cast<DevM2L*>(m2l));
                     Eh32.alloc((size_t)pl.nbox() * Rb32 * kShared, s);
@@ -762,7 +762,7 @@ struct Operator {
         fac64.Ut = m2l->Ut64.p;
         fac64.Vt = m2l->Vt64.p;
         if (mixed) {  // also with the tensor-core M2L: the stall guard may switch to this form
-            Rb32 = (R + 63) / 64 * 64;
+            Rb32 = rhs_pad32(R);
             T32.alloc((size_t)acc * Rb32, s);
             fac32.Tm = T32.p;
             fac32.Ut = m2l->Ut32.p;

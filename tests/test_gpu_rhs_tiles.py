@@ -29,3 +29,23 @@ def test_apply_at_column_tile_edges(ctx, orc, order, nrhs):
     for j in sorted({0, nrhs // 2, 7, 8, 63, 64, nrhs - 1} & set(range(nrhs))):
         yo, _ = orc.fmm_cap_apply(p["verts"], sig[:, j], order, 4)
         assert np.linalg.norm(y[:, j] - yo) / np.linalg.norm(yo) < 1e-11
+
+
+@pytest.mark.parametrize("order,m2l,far_tc,cols", [(4, 2, 0, 3), (4, 0, 1, 16), (5, 3, 0, 5), (5, 3, 1, 17), (5, 2, 1, 32),
+                                                   (5, 0, 0, 33), (6, 3, 0, 12), (6, 0, 0, 64)])
+def test_mixed_apply_at_row_padding_edges(ctx, order, m2l, far_tc, cols):
+    """The FP32 far field pads the right-hand sides to 16, 32 or a multiple of
+    64 rows per box and groups 8, 4 or 2 boxes per tensor-core item: a column's
+    result does not depend on how many columns are applied with it (the kernels
+    sum every output in the same order), so the columns of a 130-column apply
+    (three chunks of 64) agree bit for bit."""
+    lay = layouts.two_wires(length_nm=6000)
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, mesh_max_edge_m=0.3e-6,
+                             max_panels=-1)
+    sig = np.random.default_rng(order + cols).standard_normal((len(p["verts"]), 130))
+    kw = dict(order=order, max_level=4, dense_below=-1, precision=_lib.PREC_MIXED, mixed_m2l=m2l, mixed_far_tc=far_tc,
+              far_quad=1)
+    wide, rep = ctx.operator_apply(p["verts"], sig, **kw)
+    assert rep["m2l_pairs"] > 0 and rep["dense"] == 0
+    few, _ = ctx.operator_apply(p["verts"], sig[:, :cols], **kw)
+    assert np.isfinite(few).all() and np.array_equal(few, wide[:, :cols])
