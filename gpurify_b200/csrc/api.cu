@@ -100,6 +100,40 @@ void solve_panelized(Ctx& ctx, const PanelizeResult& pr, const Opts& o, std::vec
     }
 }
 
+// A context of its own (parent null), or a worker of `parent`'s batched solve
+// with a stream of its own, the parent's M2L tables and one of its pinned slots.
+gpx_status make_ctx(gpx_ctx** out, int device, const Ctx* parent, int slot) {
+    gpx_ctx* c = new (std::nothrow) gpx_ctx();
+    if (!c) return GPX_ERR_OUT_OF_MEMORY;
+    gpx_status s = guarded(nullptr, [&] {
+        c->impl.device = device;
+        GPX_CUDA(cudaSetDevice(device));
+        GPX_CUDA(cudaStreamCreateWithFlags(&c->impl.stream, cudaStreamNonBlocking));
+        GPX_CUDA(cudaDeviceGetAttribute(&c->impl.sm_count, cudaDevAttrMultiProcessorCount, device));
+        if (parent) {
+            c->impl.m2l = parent->m2l;
+            c->impl.host_words = parent->pinned + slot * kHostWords;
+        } else {
+            c->impl.m2l = std::make_shared<M2LCache>();
+            c->impl.m2l->stream = c->impl.stream;
+            GPX_CUDA(cudaMallocHost((void**)&c->impl.pinned, kHostSlots * kHostWords * sizeof(int32_t)));
+            c->impl.host_words = c->impl.pinned;
+        }
+        cudaMemPool_t pool;
+        GPX_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
+        uint64_t thresh = UINT64_MAX;  // keep freed blocks cached between solves
+        GPX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh));
+    });
+    if (s != GPX_OK) {
+        if (c->impl.pinned) cudaFreeHost(c->impl.pinned);
+        if (c->impl.stream) cudaStreamDestroy(c->impl.stream);
+        delete c;
+        return s;
+    }
+    *out = c;
+    return GPX_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -115,31 +149,17 @@ gpx_status gpx_ctx_create(gpx_ctx** out, int device) {
         g_noctx_error = "no CUDA device " + std::to_string(device);
         return GPX_ERR_NO_DEVICE;
     }
-    gpx_ctx* c = new (std::nothrow) gpx_ctx();
-    if (!c) return GPX_ERR_OUT_OF_MEMORY;
-    gpx_status s = guarded(nullptr, [&] {
-        c->impl.device = device;
-        GPX_CUDA(cudaSetDevice(device));
-        GPX_CUDA(cudaStreamCreateWithFlags(&c->impl.stream, cudaStreamNonBlocking));
-        GPX_CUDA(cudaDeviceGetAttribute(&c->impl.sm_count, cudaDevAttrMultiProcessorCount, device));
-        cudaMemPool_t pool;
-        GPX_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
-        uint64_t thresh = UINT64_MAX;  // keep freed blocks cached between solves
-        GPX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh));
-    });
-    if (s != GPX_OK) {
-        if (c->impl.stream) cudaStreamDestroy(c->impl.stream);
-        delete c;
-        return s;
-    }
-    *out = c;
-    return GPX_OK;
+    return make_ctx(out, device, nullptr, 0);
 }
 
 void gpx_ctx_destroy(gpx_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->impl.device);
-    ctx->impl.m2l_cache.clear();
+    ctx->impl.m2l.reset();
+    if (ctx->impl.pinned) {
+        cudaStreamSynchronize(ctx->impl.stream);
+        cudaFreeHost(ctx->impl.pinned);
+    }
     if (ctx->impl.stream) {
         cudaStreamSynchronize(ctx->impl.stream);
         cudaStreamDestroy(ctx->impl.stream);
@@ -208,9 +228,9 @@ gpx_status gpx_cap_solve_batched(gpx_ctx* ctx, const gpx_panel_problem* pbs, int
         std::vector<gpx_status> st(n, GPX_OK);
         std::vector<std::string> msg(n);
         const int device = ctx->impl.device;
-        auto work = [&] {
+        auto work = [&](int w) {
             gpx_ctx* sub = nullptr;
-            if (gpx_ctx_create(&sub, device) != GPX_OK) {
+            if (make_ctx(&sub, device, &ctx->impl, 1 + w) != GPX_OK) {
                 for (int32_t k; (k = next.fetch_add(1)) < n;) {
                     st[order[k]] = GPX_ERR_CUDA;
                     msg[order[k]] = "could not create a worker stream";
@@ -231,7 +251,7 @@ gpx_status gpx_cap_solve_batched(gpx_ctx* ctx, const gpx_panel_problem* pbs, int
             gpx_ctx_destroy(sub);
         };
         std::vector<std::thread> pool;
-        for (int w = 0; w < workers; ++w) pool.emplace_back(work);
+        for (int w = 0; w < workers; ++w) pool.emplace_back(work, w);
         for (auto& t : pool) t.join();
         ctx->impl.launches += launches.load();
         GPX_CUDA(cudaSetDevice(device));

@@ -102,6 +102,24 @@ struct DBuf {
 
 struct DevM2L;  // device M2L operator table, cached per (order, mode)
 
+// The device M2L tables of one context, shared with the worker contexts of its
+// batched solves (each used to build its own, about 200 MB of uploads per
+// worker and call).  Tables are built under the lock, on the owner's stream,
+// which has finished before another context sees them; they are read-only
+// afterwards and go with the owner.
+struct M2LCache {
+    std::mutex mu;
+    cudaStream_t stream = nullptr;  // the owner's
+    std::vector<std::shared_ptr<DevM2L>> tables;
+};
+
+// Pinned host words a solve reads device counters through (one slot per
+// context).  A context's slots are allocated with it and lent to the workers of
+// its batched solves: pinning and unpinning a page per GMRES call took 2.8 ms
+// in the median and up to 1 s where the host is shared.
+constexpr int kHostWords = 16;  // int32 per slot
+constexpr int kHostSlots = 33;  // the context and at most 32 batch workers
+
 // An iteration index held in device memory, for kernels replayed by a
 // device-side loop: the kernel reads k = *k at run time and offsets a vector
 // pointer by (k + add) * stride.  k == nullptr: no offset (host-known index).
@@ -144,7 +162,9 @@ struct Ctx {
     std::string last_error;
     int64_t launches = 0;  // kernel launches issued by this context
     int sm_count = 148;
-    std::vector<std::shared_ptr<DevM2L>> m2l_cache;
+    std::shared_ptr<M2LCache> m2l;   // own, or the calling context's (batch workers)
+    int32_t* host_words = nullptr;   // this context's slot
+    int32_t* pinned = nullptr;       // all slots, owned (null in batch workers)
     // per-kernel timing (enabled by gpx_ctx_set_profiling)
     bool profile = false;
     // true while a device-side GMRES loop is being captured: operator applies

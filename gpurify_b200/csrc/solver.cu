@@ -95,7 +95,9 @@ float tf32_rna(double x) {
 
 // Device tables of the shared-basis M2L for a cached operator table.
 void ensure_shared(Ctx& ctx, DevM2L& d) {
+    std::lock_guard<std::mutex> lk(ctx.m2l->mu);
     if (d.shared_ok) return;
+    cudaStream_t stream = ctx.m2l->stream;
     if (d.n < 5 || d.n > 6) throw Error(GPX_ERR_INVALID_ARG, "the shared-basis M2L runs orders 5 and 6");
     auto b = host_shared(d.n, d.mode);
     const int n3 = d.n * d.n * d.n, ns = node_stride(d.n), r = kShared, ldb = (ns + 63) / 64 * 64;
@@ -110,30 +112,32 @@ void ensure_shared(Ctx& ctx, DevM2L& d) {
             ul[(size_t)l * r + k] = tf32_rna(u - (double)uh[(size_t)l * r + k]);
         }
     for (size_t i = 0; i < c.size(); ++i) c[i] = tf32_rna(b->C[i]);
-    d.Vt_hi.upload(vh, ctx.stream);
-    d.Vt_lo.upload(vl, ctx.stream);
-    d.U_hi.upload(uh, ctx.stream);
-    d.U_lo.upload(ul, ctx.stream);
-    d.C32.upload(c, ctx.stream);
-    GPX_CUDA(cudaStreamSynchronize(ctx.stream));
+    d.Vt_hi.upload(vh, stream);
+    d.Vt_lo.upload(vl, stream);
+    d.U_hi.upload(uh, stream);
+    d.U_lo.upload(ul, stream);
+    d.C32.upload(c, stream);
+    GPX_CUDA(cudaStreamSynchronize(stream));
     d.shared_err = b->rel_err;
     d.shared_ok = true;
 }
 
 std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
-    for (auto& t : ctx.m2l_cache)
+    std::lock_guard<std::mutex> lk(ctx.m2l->mu);
+    cudaStream_t stream = ctx.m2l->stream;
+    for (auto& t : ctx.m2l->tables)
         if (t->n == n && t->mode == mode) return t;
     const M2LTable& host = *host_m2l(n, mode);
     auto d = std::make_shared<DevM2L>();
     d->n = n;
     d->mode = mode;
     d->rank = host.rank;
-    d->K.upload(host.K, ctx.stream);
+    d->K.upload(host.K, stream);
     if (mode == GPX_M2L_COMPRESSED) {
-        d->U.upload(host.U, ctx.stream);
-        d->Vt.upload(host.Vt, ctx.stream);
+        d->U.upload(host.U, stream);
+        d->Vt.upload(host.Vt, stream);
     }
-    d->d_rank.upload(host.rank, ctx.stream);
+    d->d_rank.upload(host.rank, stream);
     for (int32_t r : host.rank) d->max_rank = std::max(d->max_rank, (int)r);
     if (mode == GPX_M2L_COMPRESSED && d->max_rank <= kFacMaxRank) {
         // factored tables: Vt rows and transposed U rows, kFacMaxRank rows of
@@ -151,11 +155,11 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
                     ut32[o] = (float)ut[o];
                     vt32[o] = (float)vt[o];
                 }
-        d->Ut64.upload(ut, ctx.stream);
-        d->Vt64.upload(vt, ctx.stream);
+        d->Ut64.upload(ut, stream);
+        d->Vt64.upload(vt, stream);
         if (n >= 4) {  // the mixed path runs orders 4 to 6
-            d->Ut32.upload(ut32, ctx.stream);
-            d->Vt32.upload(vt32, ctx.stream);
+            d->Ut32.upload(ut32, stream);
+            d->Vt32.upload(vt32, stream);
         }
         d->factored_ok = true;
     }
@@ -174,10 +178,10 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
                     std::memcpy(&f, &u, 4);
                     k32[((size_t)sl * ns + m) * ns + l] = f;
                 }
-        d->K32.upload(k32, ctx.stream);
+        d->K32.upload(k32, stream);
     }
-    GPX_CUDA(cudaStreamSynchronize(ctx.stream));
-    ctx.m2l_cache.push_back(d);
+    GPX_CUDA(cudaStreamSynchronize(stream));
+    ctx.m2l->tables.push_back(d);
     return d;
 }
 
@@ -1010,12 +1014,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
                 act.p, done.p, kused.p};
     // pinned host words: [0] active-column count, [1] loop step counter read
     // back, [2] loop step counter to start from
-    int32_t* hcount = nullptr;
-    GPX_CUDA(cudaMallocHost((void**)&hcount, 4 * sizeof(int32_t)));
-    struct HostFree {
-        int32_t* p;
-        ~HostFree() { cudaFreeHost(p); }
-    } hf{hcount};
+    int32_t* const hcount = ctx.host_words;
     auto read_count = [&](const int32_t* flags, bool count_zero) -> int {
         launch_count_active(ctx, flags, R, cnt.p);
         GPX_CUDA(cudaMemcpyAsync(hcount, cnt.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
