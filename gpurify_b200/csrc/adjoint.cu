@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kDThreads) k_near_assemble_dual(DevPlan p, con
     if (threadIdx.x < 32) near_ranges_warp(p, t, threadIdx.x, s_beg, s_pre);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kDThreads / 32;
-    for (int base = 0; base < S; base += kDTile) {
+    for (int base = kDTile * blockIdx.y; base < S; base += kDTile * gridDim.y) {
         const int cnt = min(kDTile, S - base);
         if (threadIdx.x < cnt) {
             int s = base + threadIdx.x, e = 0;
@@ -294,7 +294,7 @@ void launch_panel_dprops(Ctx& c, const DevPlan& p, const double* V, double* dcen
 void launch_near_assemble_dual(Ctx& c, const DevPlan& p, int64_t nnz, const double* V, const double* dcent,
                                double* dP, double coef) {
     KTimer t(c, K_NEAR_ASSEMBLE, 8.0 * nnz, 0.0);
-    k_near_assemble_dual<<<p.nitems, kDThreads, 0, c.stream>>>(p, V, dcent, dP, coef);
+    k_near_assemble_dual<<<dim3(p.nitems, assembly_split(p.nitems)), kDThreads, 0, c.stream>>>(p, V, dcent, dP, coef);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }

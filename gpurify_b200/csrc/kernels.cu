@@ -21,8 +21,11 @@ namespace {
 constexpr int kAsmThreads = 256;
 constexpr int kAsmTile = 64;
 
-// One CTA per work item (target leaf, <= 64 rows): rows of the leaf's
-// P block m_t x S_t, row-major.
+// One CTA per work item (target leaf, <= 64 rows) and every gridDim.y-th tile
+// of 64 sources: rows of the leaf's P block m_t x S_t, row-major.  Bound: the
+// FP64 pipe (about 1,900 multiply-add slots per entry: 4 edges of 2 square
+// roots, log1p, 2 arc tangents and their divisions), so few items are split
+// over the sources until the chip is full (assembly_split).
 __global__ void __launch_bounds__(kAsmThreads, 2) k_near_assemble(DevPlan p, double* __restrict__ P, double coef) {
     const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int64_t tb = p.leaf_begin[t];
@@ -36,7 +39,7 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_near_assemble(DevPlan p, dou
     if (threadIdx.x < 32) near_ranges_warp(p, t, threadIdx.x, s_beg, s_pre);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kAsmThreads / 32;
-    for (int base = 0; base < S; base += kAsmTile) {
+    for (int base = kAsmTile * blockIdx.y; base < S; base += kAsmTile * gridDim.y) {
         const int cnt = min(kAsmTile, S - base);
         if (threadIdx.x < cnt) {
             int s = base + threadIdx.x, e = 0;
@@ -383,7 +386,7 @@ __global__ void k_potential_matrix(const double* __restrict__ sv, int64_t ns, co
 void launch_near_assemble(Ctx& c, const DevPlan& p, int64_t nnz, double* P, double coef) {
     if (p.nleaf == 0) return;
     KTimer t(c, K_NEAR_ASSEMBLE, 8.0 * nnz, (double)nnz);
-    k_near_assemble<<<p.nitems, kAsmThreads, 0, c.stream>>>(p, P, coef);
+    k_near_assemble<<<dim3(p.nitems, assembly_split(p.nitems)), kAsmThreads, 0, c.stream>>>(p, P, coef);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }

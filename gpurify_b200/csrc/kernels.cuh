@@ -69,7 +69,12 @@ __device__ __forceinline__ void near_ranges_warp(const DevPlan& p, int t, int la
     if (lane == ne - 1) s_pre[ne] = inc;
 }
 
-// Wilton near-field block assembly: P (nnz doubles), one CTA per target leaf.
+// Blocks over the sources of each near item of the assembly and its derivative:
+// enough for about eight CTAs an SM in all (two are resident), at most 16.
+// 470 panels (8 items): assembly 0.69 ms with one block per item, 0.11 with 16;
+// 466 items 1.04 ms with one, 0.59 with two; above 592 items one block each.
+inline int assembly_split(int nitems) { return nitems > 592 ? 1 : nitems < 74 ? 16 : 1184 / nitems; }
+// Wilton near-field block assembly: P (nnz doubles).
 void launch_near_assemble(Ctx& c, const DevPlan& p, int64_t nnz, double* P, double coef);
 // inv_diag[i] = 1 / P_ii (|P_ii| > 1e-30 else 1), the reference's DiagJacobi.
 void launch_diag_inv(Ctx& c, const DevPlan& p, const double* P, double* inv_diag);

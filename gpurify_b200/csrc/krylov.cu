@@ -13,23 +13,46 @@ namespace {
 
 constexpr int kRedThreads = 256;
 
+// Sum of one output's block partials: lane l adds blocks l, l + 32, ... and the
+// lanes combine in a fixed shuffle tree.
+__device__ __forceinline__ double sum_blocks(const double* __restrict__ partial, int nblk, int64_t stride, int o,
+                                             int lane) {
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += __ldcg(partial + b * stride + o);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    return s;
+}
+
 // partial[b][i][r] = sum over rows of block b of A_i[n][r] * B[n][r].
 // Eight vectors A_i per pass over the block's rows: B is read once per eight,
-// and each thread keeps eight independent loads in flight per row.  Each
-// partial sums the same rows in the same order as a one-vector pass.
+// and each thread keeps eight independent loads in flight per row.  Blocks
+// (., y) take every gridDim.y-th group of eight vectors: few rows (few blocks
+// x) spread the vectors over the SMs instead of running the groups one after
+// another.  Each partial sums the same rows in the same order as a one-vector
+// pass, whatever the grid.
+// With `ctr` (one zeroed counter per y) the last block of a y also adds its
+// vectors' partials into out[i][r] (the square root of the sum with `root`)
+// and leaves the counter at zero; without it k_reduce_blocks does.
+// Bound: the stream of the basis from HBM at large N * R; at a few thousand
+// values, latency: 470 panels, 4 columns, 1 to 58 vectors 28 us a launch with
+// its reduction before, 12 us now (both with event timing).
 template <class TA>
 __global__ void __launch_bounds__(kRedThreads) k_multidot(const TA* __restrict__ A, int64_t strideA, int ni,
                                                           const int32_t* __restrict__ kdev,
                                                           const double* __restrict__ B, int64_t N, int R,
-                                                          double* __restrict__ partial) {
+                                                          double* __restrict__ partial, int32_t* __restrict__ ctr,
+                                                          double* __restrict__ out, int root) {
     constexpr int kV = 8;
     if (kdev) ni = *kdev + 1;
+    const int y0 = kV * blockIdx.y, ystep = kV * gridDim.y;
+    if (y0 >= ni) return;
     const int nsub = kRedThreads / R;
     const int r = threadIdx.x % R, sub = threadIdx.x / R;
     const int64_t per = (N + gridDim.x - 1) / gridDim.x;
     const int64_t n0 = (int64_t)blockIdx.x * per, n1 = min(N, n0 + per);
     __shared__ double red[kV][kRedThreads];
-    for (int i0 = 0; i0 < ni; i0 += kV) {
+    for (int i0 = y0; i0 < ni; i0 += ystep) {
         const int nv = min(kV, ni - i0);
         const TA* A0 = A + i0 * strideA;
         double acc[kV];
@@ -62,32 +85,50 @@ __global__ void __launch_bounds__(kRedThreads) k_multidot(const TA* __restrict__
 #pragma unroll
         for (int q = 0; q < kV; ++q) red[q][threadIdx.x] = acc[q];
         __syncthreads();
-        if (sub == 0)
-            for (int q = 0; q < nv; ++q) {
-                double s = red[q][r];
-                for (int k = 1; k < nsub; ++k) s += red[q][k * R + r];
-                partial[((int64_t)blockIdx.x * ni + i0 + q) * R + r] = s;
-            }
+        for (int o = threadIdx.x; o < nv * R; o += kRedThreads) {
+            const int q = o / R, c = o - q * R;
+            double s = red[q][c];
+#pragma unroll 8
+            for (int k = 1; k < nsub; ++k) s += red[q][k * R + c];
+            __stcg(partial + ((int64_t)blockIdx.x * ni + i0 + q) * R + c, s);
+        }
         __syncthreads();
     }
+    if (!ctr) return;
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ctr + blockIdx.y, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int lane = threadIdx.x & 31;
+    for (int i0 = y0; i0 < ni; i0 += ystep) {
+        const int nv = min(kV, ni - i0);
+        for (int o = threadIdx.x >> 5; o < nv * R; o += kRedThreads / 32) {
+            const double s = sum_blocks(partial, gridDim.x, (int64_t)ni * R, i0 * R + o, lane);
+            if (lane == 0) out[i0 * R + o] = root ? sqrt(s) : s;
+        }
+    }
+    if (threadIdx.x == 0) ctr[blockIdx.y] = 0;
 }
 
-// out[i][r] (+)= sum_b partial[b][i][r]; one warp per (i, r): lane l sums
-// blocks l, l + 32, ... and the lanes combine in a fixed shuffle tree.
+// out[i][r] = sum_b partial[b][i][r] (its square root with `root`); one warp
+// per (i, r).
 __global__ void k_reduce_blocks(const double* __restrict__ partial, int nblk, int ni, const int32_t* __restrict__ kdev,
-                                int R, double* __restrict__ out, int accumulate) {
+                                int R, double* __restrict__ out, int root) {
     if (kdev) ni = *kdev + 1;
     const int o = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (o >= ni * R) return;
-    const int64_t stride = (int64_t)ni * R;
-    double s = 0.0;
-    for (int b = lane; b < nblk; b += 32) s += partial[b * stride + o];
-#pragma unroll
-    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-    if (lane == 0) out[o] = accumulate ? out[o] + s : s;
+    const double s = sum_blocks(partial, nblk, (int64_t)ni * R, o, lane);
+    if (lane == 0) out[o] = root ? sqrt(s) : s;
 }
 
 // W[n][r] -= sum_{i<ni} h[i][r] * V_i[n][r]
+// Bound: the stream of the basis; 64 columns of 73,011 rows run at 6.1 TB/s
+// (93 % of the measured copy).  The compiler's unrolling by four is the best
+// found: by eight the kernel took 1.3x the time, with the last group's loads
+// predicated 3x.
 template <class TV>
 __global__ void k_multi_axpy(const TV* __restrict__ V, int64_t strideV, int ni, const int32_t* __restrict__ kdev,
                              const double* __restrict__ h, double* __restrict__ W, int64_t N, int R) {
@@ -114,11 +155,6 @@ __global__ void k_scale_cols(const double* __restrict__ src, const double* __res
     const double v = d > thresh ? src[o] / d : src[o];
     dst[o] = (TD)v;
     if (cur) cur[o] = v;
-}
-
-__global__ void k_sqrt(double* v, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = sqrt(v[i]);
 }
 
 // Z[n][r] (+)= inv_diag[n] * V[n][r]
@@ -168,12 +204,9 @@ __global__ void k_zero_cols(double* __restrict__ V, const int32_t* __restrict__ 
     if (o < N * R && mask[o % R]) V[o] = 0.0;
 }
 
-// Per-column Hessenberg column k update, Givens rotation (krylov.rs:118-142,
+// Column r's Hessenberg column k update, Givens rotation (krylov.rs:118-142,
 // :195-207), residual estimate and freeze of converged columns.
-__global__ void k_givens(GmresDev g, int k, const int32_t* __restrict__ kdev) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= g.R) return;
-    if (kdev) k = *kdev;
+__device__ __forceinline__ void givens_column(const GmresDev& g, int k, int r) {
     const int m = g.m, R = g.R;
     if (!g.act[r]) return;
     double* H = g.H;  // H[(i*m + k)*R + r]
@@ -182,7 +215,7 @@ __global__ void k_givens(GmresDev g, int k, const int32_t* __restrict__ kdev) {
     // is carried from one rotation to the next (in a register); the loads of
     // each step do not depend on the previous one, so they overlap.
     double cur = g.h1[r] + g.h2[r];
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < k; ++i) {
         const double cs = g.cs[i * R + r], sn = g.sn[i * R + r];
         const double nx = g.h1[(i + 1) * R + r] + g.h2[(i + 1) * R + r];
@@ -214,6 +247,34 @@ __global__ void k_givens(GmresDev g, int k, const int32_t* __restrict__ kdev) {
     const double est = fabs(g.g[(k + 1) * R + r]) / g.bnorm[r];
     g.est[r] = est;
     if (est <= g.tol) g.act[r] = 0;
+}
+
+// Givens step k of every column and the number of columns still active (one CTA).
+__global__ void k_givens(GmresDev g, int k, int32_t* __restrict__ active) {
+    int n = 0;
+    for (int r0 = 0; r0 < g.R; r0 += blockDim.x) {
+        const int r = r0 + threadIdx.x;
+        if (r < g.R) givens_column(g, k, r);
+        n += __syncthreads_count(r < g.R && g.act[r]);
+    }
+    if (threadIdx.x == 0) *active = n;
+}
+
+// The same as the last kernel of the device-side Arnoldi loop's body: one more
+// iteration has completed (*kdev += 1); the loop goes on while a column is
+// still active and fewer than m iterations ran.
+__global__ void k_givens_loop(GmresDev g, cudaGraphConditionalHandle h, int32_t* __restrict__ kdev) {
+    const int k = *kdev;
+    int active = 0;
+    for (int r = threadIdx.x; r < g.R; r += blockDim.x) {
+        givens_column(g, k, r);
+        active |= g.act[r];
+    }
+    active = __syncthreads_or(active);
+    if (threadIdx.x == 0) {
+        *kdev = k + 1;
+        cudaGraphSetConditional(h, (active && k + 1 < g.m) ? 1u : 0u);
+    }
 }
 
 // Back substitution H y = g per column (krylov.rs:144-152); y[i][r].
@@ -271,25 +332,14 @@ __global__ void k_count_active(const int32_t* act, int R, int32_t* out) {
     if (threadIdx.x == 0) *out = red[0];
 }
 
-// Control of the device-side Arnoldi loop (one CTA of 256 threads): with
-// `advance`, one more iteration has completed (*kdev += 1); the loop goes on
-// while a column is still active and fewer than m iterations ran.
-__global__ void k_loop_ctl(cudaGraphConditionalHandle h, const int32_t* __restrict__ act, int R,
-                           int32_t* __restrict__ kdev, int m, int advance) {
-    int c = 0;
-    for (int r = threadIdx.x; r < R; r += blockDim.x) c += act[r] != 0;
-    __shared__ int red[256];
-    red[threadIdx.x] = c;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const int k = *kdev + (advance ? 1 : 0);
-        *kdev = k;
-        cudaGraphSetConditional(h, (red[0] > 0 && k < m) ? 1u : 0u);
-    }
+// Entry of the device-side Arnoldi loop (one CTA): run it if a column is
+// active and fewer than m iterations ran.
+__global__ void k_loop_enter(cudaGraphConditionalHandle h, const int32_t* __restrict__ act, int R,
+                             const int32_t* __restrict__ kdev, int m) {
+    int active = 0;
+    for (int r = threadIdx.x; r < R; r += blockDim.x) active |= act[r];
+    active = __syncthreads_or(active);
+    if (threadIdx.x == 0) cudaGraphSetConditional(h, (active && *kdev < m) ? 1u : 0u);
 }
 
 __global__ void k_zero_words(float4* __restrict__ p, int64_t n) {
@@ -303,40 +353,57 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 
 int reduce_blocks_for(int64_t N) { return (int)std::min<int64_t>(592, std::max<int64_t>(1, N / 64)); }
 
+void DotScratch::alloc(int64_t N, int max_vectors, int R, cudaStream_t s) {
+    nblk = reduce_blocks_for(N);
+    partial.alloc((size_t)nblk * max_vectors * R, s);
+    ctr.alloc(kMaxY, s);
+    ctr.zero();
+}
+
+// Blocks y of a dot of ni vectors: as many as bring the grid to four blocks an
+// SM, at most one per eight vectors.
+static int dot_grid_y(int nblk, int ni) {
+    return std::max(1, std::min({(ni + 7) / 8, 592 / nblk, DotScratch::kMaxY}));
+}
+
+// Up to 32 row blocks (about 2,000 rows) the last block of a y adds the
+// partials itself: one or two per lane, where a launch of its own costs more.
+// Above that the sums are too many for one block (64 columns, 75 vectors, 592
+// partials each) and k_reduce_blocks spreads them over the chip.
+constexpr int kFuseBlocks = 32;
+
 template <class TA>
-void multidot_t(Ctx& c, const TA* A, int64_t strideA, int ni, const double* B, int64_t N, int R, double* partial,
-                int nblk, double* out, int accumulate, int tag, const int32_t* kdev) {
+void multidot_t(Ctx& c, const TA* A, int64_t strideA, int ni, const double* B, int64_t N, int R, const DotScratch& d,
+                double* out, int tag, const int32_t* kdev, bool root) {
     // with kdev the vector count is *kdev + 1 <= ni, read on the device
+    const bool fuse = d.nblk <= kFuseBlocks;
     {
         KTimer t(c, tag, ((double)sizeof(TA) * ni + 8.0) * (double)N * R, 2.0 * ni * (double)N * R);
-        k_multidot<<<nblk, kRedThreads, 0, c.stream>>>(A, strideA, ni, kdev, B, N, R, partial);
+        k_multidot<<<dim3(d.nblk, dot_grid_y(d.nblk, ni)), kRedThreads, 0, c.stream>>>(
+            A, strideA, ni, kdev, B, N, R, d.partial.p, fuse ? d.ctr.p : nullptr, out, root ? 1 : 0);
         GPX_LAUNCH_CHECK();
     }
-    {
-        KTimer t(c, K_SMALL);
-        k_reduce_blocks<<<blocks_for((int64_t)ni * R, 8), 256, 0, c.stream>>>(partial, nblk, ni, kdev, R, out,
-                                                                              accumulate);
-        GPX_LAUNCH_CHECK();
-    }
-    c.launches += 2;
+    c.launches += 1;
+    if (fuse) return;
+    KTimer t(c, K_SMALL);
+    k_reduce_blocks<<<blocks_for((int64_t)ni * R, 8), 256, 0, c.stream>>>(d.partial.p, d.nblk, ni, kdev, R, out,
+                                                                          root ? 1 : 0);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
 }
 
 void launch_multidot(Ctx& c, const double* A, int64_t strideA, int ni, const double* B, int64_t N, int R,
-                     double* partial, int nblk, double* out, int accumulate, int tag, const int32_t* kdev) {
-    multidot_t(c, A, strideA, ni, B, N, R, partial, nblk, out, accumulate, tag, kdev);
+                     const DotScratch& d, double* out, const int32_t* kdev) {
+    multidot_t(c, A, strideA, ni, B, N, R, d, out, K_GS_DOT, kdev, false);
 }
 
 void launch_multidot(Ctx& c, const float* A, int64_t strideA, int ni, const double* B, int64_t N, int R,
-                     double* partial, int nblk, double* out, int accumulate, int tag, const int32_t* kdev) {
-    multidot_t(c, A, strideA, ni, B, N, R, partial, nblk, out, accumulate, tag, kdev);
+                     const DotScratch& d, double* out, const int32_t* kdev) {
+    multidot_t(c, A, strideA, ni, B, N, R, d, out, K_GS_DOT, kdev, false);
 }
 
-void launch_colnorm(Ctx& c, const double* A, int64_t N, int R, double* partial, int nblk, double* out) {
-    launch_multidot(c, A, 0, 1, A, N, R, partial, nblk, out, 0, K_VEC);
-    KTimer t(c, K_SMALL);
-    k_sqrt<<<blocks_for(R, 128), 128, 0, c.stream>>>(out, R);
-    GPX_LAUNCH_CHECK();
-    c.launches += 1;
+void launch_colnorm(Ctx& c, const double* A, int64_t N, int R, const DotScratch& d, double* out) {
+    multidot_t(c, A, 0, 1, A, N, R, d, out, K_VEC, nullptr, true);
 }
 
 template <class TV>
@@ -428,9 +495,15 @@ void launch_zero_cols(Ctx& c, double* V, const int32_t* mask, int64_t N, int R) 
     c.launches += 1;
 }
 
-void launch_givens(Ctx& c, const GmresDev& g, int k, const int32_t* kdev) {
+void launch_givens(Ctx& c, const GmresDev& g, int k, int32_t* active) {
     KTimer t(c, K_SMALL);
-    k_givens<<<blocks_for(g.R, 64), 64, 0, c.stream>>>(g, k, kdev);
+    k_givens<<<1, 128, 0, c.stream>>>(g, k, active);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+}
+
+void launch_givens_loop(Ctx& c, const GmresDev& g, cudaGraphConditionalHandle h, int32_t* kdev) {
+    k_givens_loop<<<1, 128, 0, c.stream>>>(g, h, kdev);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }
@@ -456,10 +529,8 @@ void launch_cycle_end(Ctx& c, const GmresDev& g, const double* rnorm) {
     c.launches += 1;
 }
 
-void launch_loop_ctl(Ctx& c, cudaGraphConditionalHandle h, const int32_t* act, int R, int32_t* kdev, int m,
-                     bool advance) {
-    KTimer t(c, K_SMALL);
-    k_loop_ctl<<<1, 256, 0, c.stream>>>(h, act, R, kdev, m, advance ? 1 : 0);
+void launch_loop_enter(Ctx& c, cudaGraphConditionalHandle h, const int32_t* act, int R, const int32_t* kdev, int m) {
+    k_loop_enter<<<1, 128, 0, c.stream>>>(h, act, R, kdev, m);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }

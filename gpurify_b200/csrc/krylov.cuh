@@ -35,13 +35,22 @@ int reduce_blocks_for(int64_t N);
 // arguments then give the launch sizes for the largest k).
 // The basis vectors (A, V) are FP64, or FP32 for the inner solves of the
 // mixed path (products and sums stay FP64).
+// Scratch of the column reductions over N rows: block partials of up to
+// max_vectors vectors, and the zeroed counters of the blocks that add them.
+struct DotScratch {
+    static constexpr int kMaxY = 32;
+    int nblk = 1;
+    DBuf<double> partial;
+    DBuf<int32_t> ctr;
+    void alloc(int64_t N, int max_vectors, int R, cudaStream_t s);
+};
+// out[i][r] = sum_n A_i[n][r] B[n][r], i < ni (kdev: i <= *kdev).
 void launch_multidot(Ctx& c, const double* A, int64_t strideA, int ni, const double* B, int64_t N, int R,
-                     double* partial, int nblk, double* out, int accumulate, int tag = K_GS_DOT,
-                     const int32_t* kdev = nullptr);
+                     const DotScratch& d, double* out, const int32_t* kdev = nullptr);
 void launch_multidot(Ctx& c, const float* A, int64_t strideA, int ni, const double* B, int64_t N, int R,
-                     double* partial, int nblk, double* out, int accumulate, int tag = K_GS_DOT,
-                     const int32_t* kdev = nullptr);
-void launch_colnorm(Ctx& c, const double* A, int64_t N, int R, double* partial, int nblk, double* out);
+                     const DotScratch& d, double* out, const int32_t* kdev = nullptr);
+// out[r] = ||A[.][r]||
+void launch_colnorm(Ctx& c, const double* A, int64_t N, int R, const DotScratch& d, double* out);
 void launch_multi_axpy(Ctx& c, const double* V, int64_t strideV, int ni, const double* h, double* W, int64_t N, int R,
                        const int32_t* kdev = nullptr);
 void launch_multi_axpy(Ctx& c, const float* V, int64_t strideV, int ni, const double* h, double* W, int64_t N, int R,
@@ -61,11 +70,13 @@ void launch_residual(Ctx& c, const int32_t* cond, const int32_t* rhs_cond, const
 void launch_sub(Ctx& c, const double* B, const double* AX, double* Res, int64_t n);
 void launch_add(Ctx& c, double* X, const double* D, int64_t n);
 void launch_zero_cols(Ctx& c, double* V, const int32_t* mask, int64_t N, int R);
-void launch_givens(Ctx& c, const GmresDev& g, int k, const int32_t* kdev = nullptr);
-// Device-side loop control: counts the active columns, advances *kdev when
-// `advance`, and sets the loop's condition (active columns left and *kdev < m).
-void launch_loop_ctl(Ctx& c, cudaGraphConditionalHandle h, const int32_t* act, int R, int32_t* kdev, int m,
-                     bool advance);
+// Givens step k; *active = columns still active.
+void launch_givens(Ctx& c, const GmresDev& g, int k, int32_t* active);
+// The device-side loop's last kernel: Givens step *kdev, then *kdev += 1 and
+// the loop's condition (active columns left and *kdev < m).
+void launch_givens_loop(Ctx& c, const GmresDev& g, cudaGraphConditionalHandle h, int32_t* kdev);
+// Sets the condition on entry.
+void launch_loop_enter(Ctx& c, cudaGraphConditionalHandle h, const int32_t* act, int R, const int32_t* kdev, int m);
 // Zero `bytes` (a multiple of 16, 16-byte aligned) with a kernel.
 void launch_zero(Ctx& c, void* p, size_t bytes);
 void launch_trisolve(Ctx& c, const GmresDev& g);

@@ -932,8 +932,8 @@ using PrecondFn = std::function<void(const double*, double*, bool, const DevInde
 
 // The device-side Arnoldi loop of one gmres_multi call: a CUDA graph whose
 // first node evaluates the loop condition and whose conditional WHILE node
-// runs one Arnoldi step per pass (operator apply, Gram-Schmidt, Givens) and
-// then advances the step counter on the device.  The loop ends when every
+// runs one Arnoldi step per pass (operator apply, Gram-Schmidt, Givens), the
+// last kernel of which advances the step counter on the device.  The loop ends when every
 // column has converged or the restart length is reached, so a cycle needs no
 // host round trip per step.
 struct ArnoldiGraph {
@@ -983,7 +983,8 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
     if (m < m_asked) max_restarts = (int)std::min<int64_t>(1000, (int64_t)max_restarts * ((m_asked + m - 1) / m));
     DBuf<TB> V;
     DBuf<double> Vcur;  // FP32 basis: the newest basis vector in FP64
-    DBuf<double> W, Z, Res, H, cs, sn, g, y, h1, h2, hnorm, bnorm, bcur, est, resid, beta, partial;
+    DBuf<double> W, Z, Res, H, cs, sn, g, y, h1, h2, hnorm, bnorm, bcur, est, resid, beta;
+    DotScratch dots;
     DBuf<int32_t> act, done, kused, cnt, kdev;
     V.alloc((size_t)(m + 1) * NR, s);
     if (f32) Vcur.alloc(NR, s);
@@ -1004,8 +1005,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
     kused.alloc(R, s);
     cnt.alloc(1, s);
     kdev.alloc(1, s);
-    const int nblk = reduce_blocks_for(N);
-    partial.alloc((size_t)nblk * (m + 1) * R, s);
+    dots.alloc(N, m + 1, R, s);
     X.alloc(NR, s);
     X.zero();
     done.zero();
@@ -1015,11 +1015,15 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
     // pinned host words: [0] active-column count, [1] loop step counter read
     // back, [2] loop step counter to start from
     int32_t* const hcount = ctx.host_words;
-    auto read_count = [&](const int32_t* flags, bool count_zero) -> int {
-        launch_count_active(ctx, flags, R, cnt.p);
+    auto read_cnt = [&]() -> int {
         GPX_CUDA(cudaMemcpyAsync(hcount, cnt.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         GPX_CUDA(cudaStreamSynchronize(s));
-        return count_zero ? R - *hcount : *hcount;
+        return *hcount;
+    };
+    auto read_count = [&](const int32_t* flags, bool count_zero) -> int {
+        launch_count_active(ctx, flags, R, cnt.p);
+        const int n = read_cnt();
+        return count_zero ? R - n : n;
     };
     // One Arnoldi step: k from the host, or (kd) from device memory.
     auto step = [&](int k, const int32_t* kd) {
@@ -1030,18 +1034,18 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
             Minv(kd ? V.p : V.p + (int64_t)k * NR, Z.p, false, dk);
         A(Z.p, W.p);
         const int ni = kd ? m : k + 1;  // launch sizes cover the largest k
-        launch_multidot(ctx, V.p, NR, ni, W.p, N, R, partial.p, nblk, h1.p, 0, K_GS_DOT, kd);
+        launch_multidot(ctx, V.p, NR, ni, W.p, N, R, dots, h1.p, kd);
         launch_multi_axpy(ctx, V.p, NR, ni, h1.p, W.p, N, R, kd);
         if (reorth) {
-            launch_multidot(ctx, V.p, NR, ni, W.p, N, R, partial.p, nblk, h2.p, 0, K_GS_DOT, kd);
+            launch_multidot(ctx, V.p, NR, ni, W.p, N, R, dots, h2.p, kd);
             launch_multi_axpy(ctx, V.p, NR, ni, h2.p, W.p, N, R, kd);
         }
-        launch_colnorm(ctx, W.p, N, R, partial.p, nblk, hnorm.p);
+        launch_colnorm(ctx, W.p, N, R, dots, hnorm.p);
         if constexpr (f32)
             launch_scale_cols(ctx, W.p, hnorm.p, 1e-14, kd ? V.p : V.p + (int64_t)(k + 1) * NR, Vcur.p, N, R, dk1);
         else
             launch_scale_cols(ctx, W.p, hnorm.p, 1e-14, kd ? V.p : V.p + (int64_t)(k + 1) * NR, N, R, dk1);
-        launch_givens(ctx, gd, k, kd);
+        if (!kd) launch_givens(ctx, gd, k, cnt.p);  // the loop's own Givens kernel also advances it
     };
     ArnoldiGraph loop;
     int64_t step_launches = 0;  // kernels of one pass of the loop body
@@ -1058,7 +1062,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
         GPX_CUDA(cudaGraphConditionalHandleCreate(&h, gr, 0, cudaGraphCondAssignDefault));
         GPX_CUDA(cudaStreamBeginCaptureToGraph(s, gr, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         try {
-            launch_loop_ctl(ctx, h, act.p, R, kdev.p, m, false);
+            launch_loop_enter(ctx, h, act.p, R, kdev.p, m);
         } catch (...) {
             cudaGraph_t dummy;
             cudaStreamEndCapture(s, &dummy);
@@ -1082,7 +1086,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
         GPX_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         try {
             step(0, kdev.p);
-            launch_loop_ctl(ctx, h, act.p, R, kdev.p, m, true);
+            launch_givens_loop(ctx, gd, h, kdev.p);
         } catch (...) {
             ctx.capturing = false;
             cudaGraph_t dummy;
@@ -1102,7 +1106,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
         GPX_CUDA(cudaMemcpyAsync(Res.p, B, (size_t)NR * sizeof(double), cudaMemcpyDeviceToDevice, s));
     else
         launch_residual(ctx, d_cond, d_rhs_cond, nullptr, Res.p, N, R);
-    launch_colnorm(ctx, Res.p, N, R, partial.p, nblk, bnorm.p);
+    launch_colnorm(ctx, Res.p, N, R, dots, bnorm.p);
     {
         KTimer kt(ctx, K_SMALL);
         k_clamp_min<<<(R + 63) / 64, 64, 0, s>>>(bnorm.p, R, 2.2250738585072014e-308);
@@ -1113,7 +1117,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
     st.m_used = m;
     for (int cycle = 0; cycle < max_restarts; ++cycle) {
         st.cycles = cycle + 1;
-        launch_colnorm(ctx, Res.p, N, R, partial.p, nblk, beta.p);
+        launch_colnorm(ctx, Res.p, N, R, dots, beta.p);
         launch_cycle_start(ctx, gd, beta.p);
         if constexpr (f32)
             launch_scale_cols(ctx, Res.p, beta.p, 0.0, V.p, Vcur.p, N, R);
@@ -1126,7 +1130,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
             step(0, nullptr);
             st.iterations += 1;
             kmax = 1;
-            if (m > 1 && read_count(act.p, false) > 0) build_loop();
+            if (m > 1 && read_cnt() > 0) build_loop();
         }
         if (device_loop && loop.exec && kmax < m) {
             hcount[2] = kmax;
@@ -1143,7 +1147,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
                 step(k, nullptr);
                 st.iterations += 1;
                 kmax = k + 1;
-                if (read_count(act.p, false) == 0) break;
+                if (read_cnt() == 0) break;
             }
         }
         launch_trisolve(ctx, gd);
@@ -1154,7 +1158,7 @@ void gmres_multi_t(Ctx& ctx, const ApplyFn& A, const PrecondFn& Minv, const int3
             launch_sub(ctx, B, W.p, Res.p, NR);
         else
             launch_residual(ctx, d_cond, d_rhs_cond, W.p, Res.p, N, R);
-        launch_colnorm(ctx, Res.p, N, R, partial.p, nblk, beta.p);
+        launch_colnorm(ctx, Res.p, N, R, dots, beta.p);
         launch_cycle_end(ctx, gd, beta.p);
         if (read_count(done.p, true) == 0) break;
     }
@@ -1323,14 +1327,14 @@ void mixed_solve(Ctx& ctx, Operator& op, const int32_t* d_cond, const int32_t* d
     cudaStream_t s = ctx.stream;
     const int64_t NR = N * R;
     const double floor_tol = std::pow(10.0, -o.inner_tol_exp);
-    DBuf<double> Res, W, D, partial, bn, rn;
+    DBuf<double> Res, W, D, bn, rn;
+    DotScratch dots;
     DBuf<int32_t> mask;
     Res.alloc(NR, s);
     W.alloc(NR, s);
     X.alloc(NR, s);
     X.zero();
-    const int nblk = reduce_blocks_for(N);
-    partial.alloc((size_t)nblk * R, s);
+    dots.alloc(N, 1, R, s);
     bn.alloc(R, s);
     rn.alloc(R, s);
     mask.alloc(R, s);
@@ -1338,7 +1342,7 @@ void mixed_solve(Ctx& ctx, Operator& op, const int32_t* d_cond, const int32_t* d
         GPX_CUDA(cudaMemcpyAsync(Res.p, B, (size_t)NR * sizeof(double), cudaMemcpyDeviceToDevice, s));
     else
         launch_residual(ctx, d_cond, d_rhs, nullptr, Res.p, N, R);
-    launch_colnorm(ctx, Res.p, N, R, partial.p, nblk, bn.p);
+    launch_colnorm(ctx, Res.p, N, R, dots, bn.p);
     std::vector<double> hb(R), hr(R);
     std::vector<int32_t> hm(R);
     bn.download(hb.data(), R);
@@ -1349,7 +1353,7 @@ void mixed_solve(Ctx& ctx, Operator& op, const int32_t* d_cond, const int32_t* d
     const ApplyFn a32 = [&](const double* x, double* y) { op.apply32(x, y); };
     double prev_resid = INFINITY;
     for (int it = 0; it <= 12; ++it) {
-        launch_colnorm(ctx, Res.p, N, R, partial.p, nblk, rn.p);
+        launch_colnorm(ctx, Res.p, N, R, dots, rn.p);
         rn.download(hr.data(), R);
         GPX_CUDA(cudaStreamSynchronize(s));
         bool all = true;

@@ -49,3 +49,20 @@ def test_mixed_apply_at_row_padding_edges(ctx, order, m2l, far_tc, cols):
     assert rep["m2l_pairs"] > 0 and rep["dense"] == 0
     few, _ = ctx.operator_apply(p["verts"], sig[:, :cols], **kw)
     assert np.isfinite(few).all() and np.array_equal(few, wide[:, :cols])
+
+
+@pytest.mark.parametrize("nets", [1, 2, 5])
+@pytest.mark.parametrize("panels_um", [1.2, 0.3])
+def test_device_loop_matches_host_loop_at_reduction_sizes(ctx, nets, panels_um):
+    """Column reductions below and above the size where the last block adds the
+    partials itself, and Givens steps with their loop control: the device-side
+    loop and the host-driven one run the same sums (bit-identical matrices, same
+    iterations), for column counts whose rows do not divide the block."""
+    lay = layouts.routing_window(nets, 8.0, seed=5, len_um=(0.5, 4.0))
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly,
+                             mesh_max_edge_m=panels_um * 1e-6, max_panels=-1)
+    nc = len(p["nets"]) + 1
+    kw = dict(order=4, max_level=3, dense_below=300, precond=1)
+    a, ra = ctx.cap_solve(p["verts"], p["cond"], nc, **kw)
+    b, rb = ctx.cap_solve(p["verts"], p["cond"], nc, no_graphs=1, **kw)
+    assert np.array_equal(a, b) and ra["iterations"] == rb["iterations"] > 1
