@@ -26,21 +26,6 @@ namespace gpx {
 
 namespace {
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool valid) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-
-// One 4- or 8-byte element copied global -> shared asynchronously: a CTA
-// puts all its copies in flight before one wait instead of a load round trip
-// per loop pass.
-template <class T>
-__device__ __forceinline__ void cp_elem(T* dst, const T* src) {
-    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async.ca copies 4, 8 or 16 bytes");
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"((int)sizeof(T)) : "memory");
-}
-
 // Panels per near-field work item (the plan's kRowsPerItem).
 constexpr int kItemPanels = 64;
 
@@ -477,108 +462,111 @@ constexpr int tree_rc() {
 }
 template <class T, int N>
 constexpr size_t tree_smem() {
-    return sizeof(T) * (size_t)(8 + 4 + 2) * tree_rc<T, N>() * Ord<N>::n3;
-}
-// Resident M2M / L2L blocks per SM asked of the register allocator: three
-// for FP32 order 5 (56 KB of shared memory each), where the default
-// allocation (80-92 registers) leaves two.
-template <class T, int N>
-constexpr int tree_min_blocks() {
-    return (sizeof(T) == 4 && N == 5) ? 3 : 1;
+    return sizeof(T) * (size_t)(4 + 2) * tree_rc<T, N>() * Ord<N>::n3;
 }
 
-// 1-D operators of the three axes as T: M1[axis][bit][m][k] (m parent node,
-// k child node), from the plan's per-octant table mat[(o*3+axis)*n*n + m*n + k].
+// 1-D operators of the three axes: m[axis][bit][m * n + k] (m parent node, k
+// child node).  A kernel argument, so that every multiply-add takes its
+// coefficient from the constant bank: held in registers (50 values at order 5)
+// they left one FP64 CTA per SM, read from shared memory they cost a load each.
 template <class T, int N>
-__device__ __forceinline__ void load_m1(const double* m2m1d, T (*M1)[2][N * N]) {
-    for (int e = threadIdx.x; e < 3 * 2 * N * N; e += blockDim.x) {
-        const int axis = e / (2 * N * N), bit = (e / (N * N)) & 1, mk = e % (N * N);
-        const int oct = bit << axis;  // any octant with this bit on this axis
-        M1[axis][bit][mk] = (T)m2m1d[(oct * 3 + axis) * N * N + mk];
-    }
+struct TreeOps {
+    T m[3][2][N * N];
+};
+// From the plan's per-octant table mat[(o*3+axis)*n*n + m*n + k].
+template <class T, int N>
+TreeOps<T, N> tree_ops(const double* mat) {
+    TreeOps<T, N> o;
+    for (int axis = 0; axis < 3; ++axis)
+        for (int bit = 0; bit < 2; ++bit)
+            for (int mk = 0; mk < N * N; ++mk)  // any octant with this bit on this axis
+                o.m[axis][bit][mk] = (T)mat[((bit << axis) * 3 + axis) * N * N + mk];
+    return o;
 }
 
 // M2M, one CTA per (parent box, chunk of RC rows r); children are contiguous
-// (Morton order).  A[oct] holds the child of octant oct (zero if absent);
+// (Morton order).  With A[oct] the child of octant oct (zero if absent),
 // B[q] = sum_oz Z_oz A[q | oz<<2] (q = ox | oy<<1); C[ox] = sum_oy Y_oy B;
 // E_par = sum_ox X_ox C[ox].  The parent row is overwritten (the parent has
 // no other contribution), padding nodes written as zero.
+// Each stage runs one 1-D line per thread (the n values along the contracted
+// axis).  The first stage reads the children's lines straight from global
+// memory: along z a line is n consecutive values, so a warp reads a contiguous
+// stretch, and shared memory holds only B and C (24 KB in FP32 at order 5, eight
+// CTAs an SM; staging the children took 56 KB, three CTAs, a clearing pass and
+// an element-wise copy).  Bound: L2 latency and the lines' shared-memory reads.
 template <class T, int N>
-__global__ void __launch_bounds__(256, tree_min_blocks<T, N>()) k_m2m_tree(DevPlan p, int pb0, const int32_t* __restrict__ child_first,
+__global__ void __launch_bounds__(256) k_m2m_tree(const __grid_constant__ TreeOps<T, N> ops,
+                                                  const int32_t* __restrict__ octant, int pb0,
+                                                  const int32_t* __restrict__ child_first,
                                                   const int32_t* __restrict__ child_count, T* __restrict__ E, int Rb) {
     constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, RC = tree_rc<T, N>(), NN = N * N;
     const int pb = pb0 + blockIdx.x;
     const int r0 = blockIdx.y * RC;
     const int rc = min(RC, Rb - r0);
     extern __shared__ __align__(16) unsigned char tree_smem_raw[];
-    T* A = reinterpret_cast<T*>(tree_smem_raw);  // [8][RC][N3]
-    T* B = A + 8 * RC * N3;                      // [4][RC][N3]
-    T* C = B + 4 * RC * N3;                      // [2][RC][N3]
-    __shared__ T M1[3][2][NN];
-    __shared__ int oct_s[8];
-    load_m1<T, N>(p.m2m1d, M1);
+    T* B = reinterpret_cast<T*>(tree_smem_raw);  // [RC][4][N3]
+    T* C = B + 4 * RC * N3;                      // [RC][2][N3]
+    __shared__ int child[8];  // by octant, -1 if absent
+    if (threadIdx.x < 8) child[threadIdx.x] = -1;
+    __syncthreads();
     const int cf = child_first[pb], cc = child_count[pb];  // cc <= 8 (octree)
-    if (threadIdx.x < cc) oct_s[threadIdx.x] = p.box_octant[cf + threadIdx.x];
-    for (int e = threadIdx.x; e < 8 * RC * N3; e += blockDim.x) A[e] = (T)0;
+    if (threadIdx.x < cc) child[octant[cf + threadIdx.x]] = cf + threadIdx.x;
     __syncthreads();
-    // every child row of the chunk in flight at once, then one wait
-    const int per = rc * N3;
-    for (int e = threadIdx.x; e < cc * per; e += blockDim.x) {
-        const int k = e / per, rm = e - k * per, r = rm / N3, m = rm - r * N3;
-        cp_elem(A + (oct_s[k] * RC + r) * N3 + m, E + ((int64_t)(cf + k) * Rb + r0 + r) * NS + m);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    // Each stage runs one 1-D line per thread (the n values along the
-    // contracted axis), so the index arithmetic is per line, not per value.
-    // z: B[q][r][(a,b,c')] = sum_oz sum_c Z_oz[c'][c] A[q|oz<<2][r][(a,b,c)]
-    for (int e = threadIdx.x; e < 4 * RC * NN; e += blockDim.x) {
-        const int q = e / (RC * NN), r = (e / NN) % RC, ab = e % NN;
-        const T* a0 = A + (q * RC + r) * N3 + ab * N;
-        const T* a1 = A + ((q | 4) * RC + r) * N3 + ab * N;
+    // z: B[r][q][(a,b,c')] = sum_oz sum_c Z_oz[c'][c] A[q|oz<<2][r][(a,b,c)]
+    for (int e = threadIdx.x; e < rc * 4 * NN; e += 256) {
+        const int r = e / (4 * NN), q = (e / NN) & 3, ab = e % NN;
+        const int c0 = child[q], c1 = child[q | 4];
         T x0[N], x1[N];
 #pragma unroll
-        for (int c = 0; c < N; ++c) {
-            x0[c] = a0[c];
-            x1[c] = a1[c];
+        for (int c = 0; c < N; ++c) x0[c] = x1[c] = (T)0;
+        if (c0 >= 0) {
+            const T* a = E + ((int64_t)c0 * Rb + r0 + r) * NS + ab * N;
+#pragma unroll
+            for (int c = 0; c < N; ++c) x0[c] = a[c];
         }
-        T* out = B + (q * RC + r) * N3 + ab * N;
+        if (c1 >= 0) {
+            const T* a = E + ((int64_t)c1 * Rb + r0 + r) * NS + ab * N;
+#pragma unroll
+            for (int c = 0; c < N; ++c) x1[c] = a[c];
+        }
+        T* out = B + (r * 4 + q) * N3 + ab * N;
 #pragma unroll
         for (int cp = 0; cp < N; ++cp) {
             T s = (T)0;
 #pragma unroll
-            for (int c = 0; c < N; ++c) s += M1[2][0][cp * N + c] * x0[c] + M1[2][1][cp * N + c] * x1[c];
+            for (int c = 0; c < N; ++c) s += ops.m[2][0][cp * N + c] * x0[c] + ops.m[2][1][cp * N + c] * x1[c];
             out[cp] = s;
         }
     }
     __syncthreads();
-    // y: C[ox][r][(a,b',c)] = sum_oy sum_b Y_oy[b'][b] B[ox|oy<<1][r][(a,b,c)]
-    for (int e = threadIdx.x; e < 2 * RC * NN; e += blockDim.x) {
-        const int ox = e / (RC * NN), r = (e / NN) % RC, ac = e % NN, a = ac / N, c = ac % N;
-        const T* b0 = B + (ox * RC + r) * N3 + a * NN + c;
-        const T* b1 = B + ((ox | 2) * RC + r) * N3 + a * NN + c;
+    // y: C[r][ox][(a,b',c)] = sum_oy sum_b Y_oy[b'][b] B[r][ox|oy<<1][(a,b,c)]
+    for (int e = threadIdx.x; e < rc * 2 * NN; e += 256) {
+        const int r = e / (2 * NN), ox = (e / NN) & 1, ac = e % NN, a = ac / N, c = ac % N;
+        const T* b0 = B + (r * 4 + ox) * N3 + a * NN + c;
+        const T* b1 = B + (r * 4 + (ox | 2)) * N3 + a * NN + c;
         T x0[N], x1[N];
 #pragma unroll
         for (int b = 0; b < N; ++b) {
             x0[b] = b0[b * N];
             x1[b] = b1[b * N];
         }
-        T* out = C + (ox * RC + r) * N3 + a * NN + c;
+        T* out = C + (r * 2 + ox) * N3 + a * NN + c;
 #pragma unroll
         for (int bp = 0; bp < N; ++bp) {
             T s = (T)0;
 #pragma unroll
-            for (int b = 0; b < N; ++b) s += M1[1][0][bp * N + b] * x0[b] + M1[1][1][bp * N + b] * x1[b];
+            for (int b = 0; b < N; ++b) s += ops.m[1][0][bp * N + b] * x0[b] + ops.m[1][1][bp * N + b] * x1[b];
             out[bp * N] = s;
         }
     }
     __syncthreads();
-    // x: E_par[r][(a',b,c)] = sum_ox sum_a X_ox[a'][a] C[ox][r][(a,b,c)]; padding nodes zero
+    // x: E_par[r][(a',b,c)] = sum_ox sum_a X_ox[a'][a] C[r][ox][(a,b,c)]; padding nodes zero
     T* dst = E + ((int64_t)pb * Rb + r0) * NS;
-    for (int e = threadIdx.x; e < rc * NN; e += blockDim.x) {
+    for (int e = threadIdx.x; e < rc * NN; e += 256) {
         const int r = e / NN, bc = e % NN;
-        const T* c0 = C + r * N3 + bc;
-        const T* c1 = C + (RC + r) * N3 + bc;
+        const T* c0 = C + r * 2 * N3 + bc;
+        const T* c1 = c0 + N3;
         T x0[N], x1[N];
 #pragma unroll
         for (int a = 0; a < N; ++a) {
@@ -589,12 +577,12 @@ __global__ void __launch_bounds__(256, tree_min_blocks<T, N>()) k_m2m_tree(DevPl
         for (int ap = 0; ap < N; ++ap) {
             T s = (T)0;
 #pragma unroll
-            for (int a = 0; a < N; ++a) s += M1[0][0][ap * N + a] * x0[a] + M1[0][1][ap * N + a] * x1[a];
+            for (int a = 0; a < N; ++a) s += ops.m[0][0][ap * N + a] * x0[a] + ops.m[0][1][ap * N + a] * x1[a];
             dst[(int64_t)r * NS + ap * NN + bc] = s;
         }
     }
     if constexpr (NS > N3)
-        for (int e = threadIdx.x; e < rc * (NS - N3); e += blockDim.x) {
+        for (int e = threadIdx.x; e < rc * (NS - N3); e += 256) {
             const int r = e / (NS - N3), m = N3 + e % (NS - N3);
             dst[(int64_t)r * NS + m] = (T)0;
         }
@@ -602,185 +590,91 @@ __global__ void __launch_bounds__(256, tree_min_blocks<T, N>()) k_m2m_tree(DevPl
 
 // L2L, one CTA per (parent box, chunk of RC rows r): the transposed tree.
 // C[ox] = X_ox^T L_par; B[ox|oy<<1] = Y_oy^T C[ox]; child of octant oct:
-// L_child += Z_oz^T B[oct & 3].
+// L_child += Z_oz^T B[oct & 3].  As in M2M the first stage reads the parent's
+// lines and the last one updates the children's in global memory, contiguous
+// over a warp; shared memory holds C and B.
 template <class T, int N>
-__global__ void __launch_bounds__(256, tree_min_blocks<T, N>()) k_l2l_tree(DevPlan p, int pb0, const int32_t* __restrict__ child_first,
+__global__ void __launch_bounds__(256) k_l2l_tree(const __grid_constant__ TreeOps<T, N> ops,
+                                                  const int32_t* __restrict__ octant, int pb0,
+                                                  const int32_t* __restrict__ child_first,
                                                   const int32_t* __restrict__ child_count, T* __restrict__ L, int Rb) {
     constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, RC = tree_rc<T, N>(), NN = N * N;
     const int pb = pb0 + blockIdx.x;
-    const int r0 = blockIdx.y * RC;
-    const int rc = min(RC, Rb - r0);
-    extern __shared__ __align__(16) unsigned char tree_smem_raw[];
-    T* Ch = reinterpret_cast<T*>(tree_smem_raw);  // [8][RC][N3]: the children's rows of the chunk
-    T* B = Ch + 8 * RC * N3;                      // [4][RC][N3]
-    T* C = B + 4 * RC * N3;                       // [2][RC][N3]
-    T* P = B;                                     // [RC][N3]: the parent, dead once C is formed
-    __shared__ T M1[3][2][NN];
-    __shared__ int oct_s[8];
-    load_m1<T, N>(p.m2m1d, M1);
     const int cf = child_first[pb], cc = child_count[pb];  // cc <= 8 (octree)
-    if (threadIdx.x < cc) oct_s[threadIdx.x] = p.box_octant[cf + threadIdx.x];
-    const T* src = L + ((int64_t)pb * Rb + r0) * NS;
-    for (int e = threadIdx.x; e < RC * N3; e += blockDim.x) {
-        const int r = e / N3, m = e % N3;
-        if (r < rc)
-            cp_elem(P + e, src + (int64_t)r * NS + m);
-        else
-            P[e] = (T)0;
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // The children's current rows, needed only by the last stage: their
-    // copies stay in flight through the x and y stages.
-    const int per = rc * N3;
-    for (int e = threadIdx.x; e < cc * per; e += blockDim.x) {
-        const int k = e / per, rm = e - k * per, r = rm / N3, m = rm - r * N3;
-        cp_elem(Ch + (k * RC + r) * N3 + m, L + ((int64_t)(cf + k) * Rb + r0 + r) * NS + m);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-    // x: C[ox][r][(a,b,c)] = sum_a' X_ox[a'][a] P[r][(a',b,c)]  (one line per thread)
-    for (int e = threadIdx.x; e < RC * NN; e += blockDim.x) {
-        const int r = e / NN, bc = e % NN;
-        const T* pr = P + r * N3 + bc;
-        T x[N];
-#pragma unroll
-        for (int ap = 0; ap < N; ++ap) x[ap] = pr[ap * NN];
-#pragma unroll
-        for (int ox = 0; ox < 2; ++ox) {
-            T* out = C + (ox * RC + r) * N3 + bc;
-#pragma unroll
-            for (int a = 0; a < N; ++a) {
-                T s = (T)0;
-#pragma unroll
-                for (int ap = 0; ap < N; ++ap) s += M1[0][ox][ap * N + a] * x[ap];
-                out[a * NN] = s;
-            }
-        }
-    }
-    __syncthreads();
-    // y: B[q][r][(a,b,c)] = sum_b' Y_oy[b'][b] C[ox][r][(a,b',c)],  q = ox | oy<<1
-    for (int e = threadIdx.x; e < 2 * RC * NN; e += blockDim.x) {
-        const int ox = e / (RC * NN), r = (e / NN) % RC, ac = e % NN, a = ac / N, c = ac % N;
-        const T* cr = C + (ox * RC + r) * N3 + a * NN + c;
-        T x[N];
-#pragma unroll
-        for (int bp = 0; bp < N; ++bp) x[bp] = cr[bp * N];
-#pragma unroll
-        for (int oy = 0; oy < 2; ++oy) {
-            T* out = B + ((ox | (oy << 1)) * RC + r) * N3 + a * NN + c;
-#pragma unroll
-            for (int b = 0; b < N; ++b) {
-                T s = (T)0;
-#pragma unroll
-                for (int bp = 0; bp < N; ++bp) s += M1[1][oy][bp * N + b] * x[bp];
-                out[b * N] = s;
-            }
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    // z, straight into each existing child: L_child[r][(a,b,c)] += sum_c' Z_oz[c'][c] B[oct&3][r][(a,b,c')]
-    for (int e = threadIdx.x; e < cc * rc * NN; e += blockDim.x) {
-        const int k = e / (rc * NN), r = (e / NN) % rc, ab = e % NN;
-        const int ch = cf + k;
-        const int oc = oct_s[k], q = oc & 3, oz = oc >> 2;
-        const T* br = B + (q * RC + r) * N3 + ab * N;
-        const T* old = Ch + (k * RC + r) * N3 + ab * N;
-        T x[N];
-#pragma unroll
-        for (int cp = 0; cp < N; ++cp) x[cp] = br[cp];
-        T* dst = L + ((int64_t)ch * Rb + r0 + r) * NS + ab * N;
-#pragma unroll
-        for (int c = 0; c < N; ++c) {
-            T s = (T)0;
-#pragma unroll
-            for (int cp = 0; cp < N; ++cp) s += M1[2][oz][cp * N + c] * x[cp];
-            dst[c] = old[c] + s;
-        }
-    }
-}
-
-// L2L as above, with the children's rows read and written in place by the
-// last stage instead of prefetched: faster for FP32, whose prefetch takes
-// 4-byte copies.
-template <class T, int N>
-__global__ void __launch_bounds__(256, tree_min_blocks<T, N>()) k_l2l_tree_inplace(DevPlan p, int pb0, const int32_t* __restrict__ child_first,
-                                                  const int32_t* __restrict__ child_count, T* __restrict__ L, int Rb) {
-    constexpr int N3 = Ord<N>::n3, NS = Ord<N>::ns, RC = tree_rc<T, N>(), NN = N * N;
-    const int pb = pb0 + blockIdx.x;
+    if (cc == 0) return;
     const int r0 = blockIdx.y * RC;
     const int rc = min(RC, Rb - r0);
     extern __shared__ __align__(16) unsigned char tree_smem_raw[];
-    T* P = reinterpret_cast<T*>(tree_smem_raw);  // [RC][N3]
-    T* B = P + 8 * RC * N3;                      // [4][RC][N3]
-    T* C = B + 4 * RC * N3;                      // [2][RC][N3]
-    __shared__ T M1[3][2][NN];
-    load_m1<T, N>(p.m2m1d, M1);
+    T* B = reinterpret_cast<T*>(tree_smem_raw);  // [RC][4][N3]
+    T* C = B + 4 * RC * N3;                      // [RC][2][N3]
+    __shared__ int oct_s[8];
+    if (threadIdx.x < cc) oct_s[threadIdx.x] = octant[cf + threadIdx.x];
+    // x: C[r][ox][(a,b,c)] = sum_a' X_ox[a'][a] P[r][(a',b,c)]  (one line per thread)
     const T* src = L + ((int64_t)pb * Rb + r0) * NS;
-    for (int e = threadIdx.x; e < RC * N3; e += blockDim.x) {
-        const int r = e / N3, m = e % N3;
-        P[e] = r < rc ? src[(int64_t)r * NS + m] : (T)0;
-    }
-    __syncthreads();
-    // x: C[ox][r][(a,b,c)] = sum_a' X_ox[a'][a] P[r][(a',b,c)]  (one line per thread)
-    for (int e = threadIdx.x; e < RC * NN; e += blockDim.x) {
+    for (int e = threadIdx.x; e < rc * NN; e += 256) {
         const int r = e / NN, bc = e % NN;
-        const T* pr = P + r * N3 + bc;
         T x[N];
 #pragma unroll
-        for (int ap = 0; ap < N; ++ap) x[ap] = pr[ap * NN];
+        for (int ap = 0; ap < N; ++ap) x[ap] = src[(int64_t)r * NS + ap * NN + bc];
 #pragma unroll
         for (int ox = 0; ox < 2; ++ox) {
-            T* out = C + (ox * RC + r) * N3 + bc;
+            T* out = C + (r * 2 + ox) * N3 + bc;
 #pragma unroll
             for (int a = 0; a < N; ++a) {
                 T s = (T)0;
 #pragma unroll
-                for (int ap = 0; ap < N; ++ap) s += M1[0][ox][ap * N + a] * x[ap];
+                for (int ap = 0; ap < N; ++ap) s += ops.m[0][ox][ap * N + a] * x[ap];
                 out[a * NN] = s;
             }
         }
     }
     __syncthreads();
-    // y: B[q][r][(a,b,c)] = sum_b' Y_oy[b'][b] C[ox][r][(a,b',c)],  q = ox | oy<<1
-    for (int e = threadIdx.x; e < 2 * RC * NN; e += blockDim.x) {
-        const int ox = e / (RC * NN), r = (e / NN) % RC, ac = e % NN, a = ac / N, c = ac % N;
-        const T* cr = C + (ox * RC + r) * N3 + a * NN + c;
+    // y: B[r][q][(a,b,c)] = sum_b' Y_oy[b'][b] C[r][ox][(a,b',c)],  q = ox | oy<<1
+    for (int e = threadIdx.x; e < rc * 2 * NN; e += 256) {
+        const int r = e / (2 * NN), ox = (e / NN) & 1, ac = e % NN, a = ac / N, c = ac % N;
+        const T* cr = C + (r * 2 + ox) * N3 + a * NN + c;
         T x[N];
 #pragma unroll
         for (int bp = 0; bp < N; ++bp) x[bp] = cr[bp * N];
 #pragma unroll
         for (int oy = 0; oy < 2; ++oy) {
-            T* out = B + ((ox | (oy << 1)) * RC + r) * N3 + a * NN + c;
+            T* out = B + (r * 4 + (ox | (oy << 1))) * N3 + a * NN + c;
 #pragma unroll
             for (int b = 0; b < N; ++b) {
                 T s = (T)0;
 #pragma unroll
-                for (int bp = 0; bp < N; ++bp) s += M1[1][oy][bp * N + b] * x[bp];
+                for (int bp = 0; bp < N; ++bp) s += ops.m[1][oy][bp * N + b] * x[bp];
                 out[b * N] = s;
             }
         }
     }
     __syncthreads();
-    // z, straight into each existing child: L_child[r][(a,b,c)] += sum_c' Z_oz[c'][c] B[oct&3][r][(a,b,c')]
-    const int cf = child_first[pb], cc = child_count[pb];
-    for (int e = threadIdx.x; e < cc * rc * NN; e += blockDim.x) {
-        const int k = e / (rc * NN), r = (e / NN) % rc, ab = e % NN;
-        const int ch = cf + k;
-        const int oc = p.box_octant[ch], q = oc & 3, oz = oc >> 2;
-        const T* br = B + (q * RC + r) * N3 + ab * N;
+    // z, straight into each existing child: L_child[r][(a,b,c)] += sum_c' Z_oz[c'][c] B[r][oct&3][(a,b,c')]
+    for (int e = threadIdx.x; e < cc * RC * NN; e += 256) {
+        const int k = e / (RC * NN), r = (e / NN) % RC, ab = e % NN;
+        if (r >= rc) continue;
+        const int oc = oct_s[k], q = oc & 3, oz = oc >> 2;
+        T* dst = L + ((int64_t)(cf + k) * Rb + r0 + r) * NS + ab * N;
+        T old[N];
+#pragma unroll
+        for (int c = 0; c < N; ++c) old[c] = dst[c];
+        const T* br = B + (r * 4 + q) * N3 + ab * N;
         T x[N];
 #pragma unroll
         for (int cp = 0; cp < N; ++cp) x[cp] = br[cp];
-        T* dst = L + ((int64_t)ch * Rb + r0 + r) * NS + ab * N;
+        auto line = [&](const T* m) {
 #pragma unroll
-        for (int c = 0; c < N; ++c) {
-            T s = (T)0;
+            for (int c = 0; c < N; ++c) {
+                T s = (T)0;
 #pragma unroll
-            for (int cp = 0; cp < N; ++cp) s += M1[2][oz][cp * N + c] * x[cp];
-            dst[c] += s;
-        }
+                for (int cp = 0; cp < N; ++cp) s += m[cp * N + c] * x[cp];
+                dst[c] = old[c] + s;
+            }
+        };
+        if (oz)  // a branch, so that the coefficients' addresses are constants
+            line(ops.m[2][1]);
+        else
+            line(ops.m[2][0]);
     }
 }
 
@@ -872,16 +766,17 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
             c.launches += 1;
         }
     }
-    if (smem > 48 * 1024) {
+    const TreeOps<T, N> ops = tree_ops<T, N>(f.m2m1d);
+    if (smem > 40 * 1024) {  // with the static part above the 48 KB default
         set_smem_once(k_m2m_tree<T, N>, (int)smem);
         set_smem_once(k_l2l_tree<T, N>, (int)smem);
-        set_smem_once(k_l2l_tree_inplace<T, N>, (int)smem);
     }
     for (int l = Lv; l >= 3; --l) {
         const int pb0 = f.lvl_off[l - 1], npb = f.lvl_off[l] - pb0, nch = f.lvl_off[l + 1] - f.lvl_off[l];
         if (npb == 0) continue;
         KTimer t(c, prec_tag<T>(K_M2M), (double)(npb + nch) * box_bytes, 2.0 * 14.0 * N * N3 * R * (double)npb);
-        k_m2m_tree<T, N><<<dim3(npb, rchunks_tree), 256, smem, s>>>(p, pb0, f.child_first, f.child_count, E, Rb);
+        k_m2m_tree<T, N><<<dim3(npb, rchunks_tree), 256, smem, s>>>(ops, p.box_octant, pb0, f.child_first,
+                                                                    f.child_count, E, Rb);
         GPX_LAUNCH_CHECK();
         c.launches += 1;
     }
@@ -908,11 +803,8 @@ void far_field_n(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, const
         const int pb0 = f.lvl_off[l], npb = f.lvl_off[l + 1] - pb0, ncb = f.lvl_off[l + 2] - f.lvl_off[l + 1];
         if (ncb == 0) continue;
         KTimer t(c, prec_tag<T>(K_L2L), (double)(npb + 2 * ncb) * box_bytes, 2.0 * 14.0 * N * N3 * R * (double)npb);
-        if constexpr (sizeof(T) == 4)
-            k_l2l_tree_inplace<T, N><<<dim3(npb, rchunks_tree), 256, smem, s>>>(p, pb0, f.child_first, f.child_count,
-                                                                               L, Rb);
-        else
-            k_l2l_tree<T, N><<<dim3(npb, rchunks_tree), 256, smem, s>>>(p, pb0, f.child_first, f.child_count, L, Rb);
+        k_l2l_tree<T, N><<<dim3(npb, rchunks_tree), 256, smem, s>>>(ops, p.box_octant, pb0, f.child_first,
+                                                                    f.child_count, L, Rb);
         GPX_LAUNCH_CHECK();
         c.launches += 1;
     }

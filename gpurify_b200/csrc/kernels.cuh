@@ -34,7 +34,6 @@ struct DevPlan {
     const int64_t* m2l_off;
     const int32_t* m2l_src;
     const int32_t* m2l_slot;
-    const double* m2m1d;      // 24 n x n
     const double* m2l_K;      // 343 n3 x n3 (FP64 table)
     const double* leaf_ctr;   // 3 per leaf: box centre
     const int32_t* leaf_of;   // per panel: its leaf
@@ -89,6 +88,7 @@ inline int node_stride(int n) { return (n * n * n + 31) & ~31; }
 struct FarLaunch {
     const int32_t* lvl_off;      // host, L+2 entries
     const double* lvl_half;      // host, L+1 entries
+    const double* m2m1d;         // host, 24 n x n
     const int32_t* child_first;  // device, per box
     const int32_t* child_count;  // device, per box
     const int32_t* leaf_of;      // device, per sorted panel

@@ -186,7 +186,7 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
 }
 
 struct DevPlanBufs {
-    DBuf<double> verts, cent, area, w1d, m2m1d;
+    DBuf<double> verts, cent, area, w1d;
     DBuf<int32_t> cond, near_off, near_src, near_S, box_parent, box_octant, m2l_src, m2l_slot, child_first,
         child_count, leaf_of, item_leaf, item_row0, item_order, item128_leaf, item128_row0, near_rev, near_pre, p2m_slot,
         fix_leaf, fix_first, fix_cnt;
@@ -203,7 +203,6 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
     d.cent.upload(p.cent, s);
     d.area.upload(p.area, s);
     d.w1d.upload(p.w1d, s);
-    d.m2m1d.upload(p.m2m1d, s);
     d.cond.upload(p.cond, s);
     d.near_off.upload(p.near_off, s);
     d.near_src.upload(p.near_src, s);
@@ -341,10 +340,10 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
     v.m2l_off = d.m2l_off.p;
     v.m2l_src = d.m2l_src.p;
     v.m2l_slot = d.m2l_slot.p;
-    v.m2m1d = d.m2m1d.p;
     v.m2l_K = m2l ? m2l->K.p : nullptr;
     d.far.lvl_off = p.lvl_off.data();
     d.far.lvl_half = p.lvl_half.data();
+    d.far.m2m1d = p.m2m1d.data();
     d.far.child_first = d.child_first.p;
     d.far.child_count = d.child_count.p;
     d.far.leaf_of = d.leaf_of.p;
