@@ -29,9 +29,10 @@ __host__ __device__ inline Dual operator+(Dual a, Dual b) { return {a.v + b.v, a
 __host__ __device__ inline Dual operator-(Dual a, Dual b) { return {a.v - b.v, a.d - b.d}; }
 __host__ __device__ inline Dual operator-(Dual a) { return {-a.v, -a.d}; }
 __host__ __device__ inline Dual operator*(Dual a, Dual b) { return {a.v * b.v, a.d * b.v + a.v * b.d}; }
+// One division for the value and the derivative.
 __host__ __device__ inline Dual operator/(Dual a, Dual b) {
-    const double q = a.v / b.v;
-    return {q, (a.d - q * b.d) / b.v};
+    const double inv = 1.0 / b.v, q = a.v * inv;
+    return {q, (a.d - q * b.d) * inv};
 }
 __host__ __device__ inline Dual operator+(Dual a, double b) { return {a.v + b, a.d}; }
 __host__ __device__ inline Dual operator+(double a, Dual b) { return {a + b.v, b.d}; }

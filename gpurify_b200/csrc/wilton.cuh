@@ -72,9 +72,20 @@ __device__ __forceinline__ void prep_source_t(const S* g, SrcPanelT<S>& s) {
 // form rounds num or den to <= 0 it falls back to the asinh difference; the
 // stable form needs no fallback, and a point on the edge line (r0 = 0)
 // contributes 0 exactly as the reference's fallback does.
-template <class S>
-__device__ __forceinline__ S wilton_t(const SrcPanelT<S>& s, S px, S py, S pz) {
-    using ::atan;
+//
+// The arc-tangent term of one edge, ad (atan(tp) - atan(tm)).
+__device__ __forceinline__ double edge_angle(double ad, double tp, double tm) { return ad * (::atan(tp) - ::atan(tm)); }
+// On dual numbers the derivative alone (wilton_t<Dual> is used for nothing
+// else): the angle itself counts only where the height over the panel changes.
+__device__ __forceinline__ Dual edge_angle(Dual ad, Dual tp, Dual tm) {
+    const double angle = ad.d != 0.0 ? ::atan(tp.v) - ::atan(tm.v) : 0.0;
+    const double pp = 1.0 + tp.v * tp.v, mm = 1.0 + tm.v * tm.v;
+    return {0.0, ad.d * angle + ad.v * ((tp.d * mm - tm.d * pp) / (pp * mm))};
+}
+
+// P: scalar of the panel, S: scalar of the point (and of the result).
+template <class S, class P = S>
+__device__ __forceinline__ S wilton_t(const SrcPanelT<P>& s, S px, S py, S pz) {
     using ::fabs;
     using ::log1p;
     using ::sqrt;
@@ -85,8 +96,8 @@ __device__ __forceinline__ S wilton_t(const SrcPanelT<S>& s, S px, S py, S pz) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (s.el[i] == 0.0) continue;
-        const S* a = s.v[i];
-        const S* b = s.v[(i + 1) & 3];
+        const P* a = s.v[i];
+        const P* b = s.v[(i + 1) & 3];
         const S am[3] = {a[0] - p0[0], a[1] - p0[1], a[2] - p0[2]};
         const S bm[3] = {b[0] - p0[0], b[1] - p0[1], b[2] - p0[2]};
         const S pp = am[0] * s.uh[i][0] + am[1] * s.uh[i][1] + am[2] * s.uh[i][2];
@@ -103,7 +114,7 @@ __device__ __forceinline__ S wilton_t(const SrcPanelT<S>& s, S px, S py, S pz) {
         if (ad > 0.0 && pp != 0.0) {
             const S tp = (pp * sp) / (r0sq + ad * rp);
             const S tm = (pp * sm) / (r0sq + ad * rm);
-            at = ad * (atan(tp) - atan(tm));
+            at = edge_angle(ad, tp, tm);
         }
         total += lt - at;
     }
