@@ -106,13 +106,15 @@ void launch_m2l_fac<float>(Ctx& c, const FacM2L<float>& f, int b0, int nb, float
 
 // Tensor-core (tcgen05, TF32 inputs, FP32 accumulation) M2L work list of one
 // level: groups of target boxes sharing one offset loop.
-// An item holds 128 operand rows: 128 / Rb target boxes of one octant class
-// (so that their interaction lists use the same offsets) with Rb right-hand
-// sides each, Rb = 16, 32 or 64 (two boxes for a multiple of 64).  Four boxes
-// of 64 with two accumulators sharing each operator tile measured slower on
-// the bench window (0.385 against 0.309 ms per launch: half the CTAs per SM by
-// shared memory, and more zero-filled rows in the union of four boxes' offsets).
-inline int tc_group(int Rb) { return Rb >= 64 ? 2 : 128 / Rb; }
+// An item holds tc_group(Rb) target boxes of one octant class (so that their
+// interaction lists use the same offsets): two of 64 right-hand sides, four of
+// 16 or 32.  More boxes share each operator tile but add zero-filled rows in
+// the union of their offsets and leave fewer, longer items: at 16 columns an
+// apply of a 21,195-panel bus (depth 5) takes 66 us with two or four boxes and
+// 158 us with eight, the 64-net window 71, 48 and 64 us; at 32 columns the
+// window takes 75 us with two and 66 us with four.  Four boxes of 64 with two
+// accumulators measured slower on the window (0.385 against 0.309 ms).
+constexpr int tc_group(int Rb) { return Rb >= 64 ? 2 : 4; }
 struct TcLevel {
     int nitems = 0;
     const int32_t* item_t = nullptr;    // tc_group per item: target boxes (trailing ones may be -1)
@@ -131,8 +133,8 @@ inline int rhs_pad32(int R) { return R <= 16 ? 16 : R <= 32 ? 32 : (R + 63) / 64
 // tc_group(R).  err receives a nonzero code if a bounded
 // wait on the tensor-core pipeline expired.  box_scale (per box, may be null):
 // each target box's own scale, for launches that cover several levels.
-void launch_m2l_tc(Ctx& c, const TcLevel& lv, int ns, const float* E, float* L, const float* K32, int R, float scale,
-                   const double* box_scale, int* err);
+void launch_m2l_tc(Ctx& c, const TcLevel& lv, int ns, const float* E, int64_t nbox, float* L, const float* K32, int R,
+                   float scale, const double* box_scale, int* err);
 
 // Shared-basis M2L (SharedBasis in plan.h), rank kShared: expansion rows
 // (box, right-hand side) [row0, row0 + nrows) compressed, E^ = V^T E, and

@@ -4,37 +4,41 @@
 //
 // For one offset o every target box t with a source s = t + o needs
 //     L_t^T (R x NS) += E_s^T (R x NS) * K_o^T (NS x NS).
-// A CTA owns G = 128 / RB target boxes of one octant class (so their
-// interaction lists use the same offsets) with RB = 16, 32 or 64 right-hand
-// sides each (a 64-wide chunk of them for more): one accumulator D (128 x NS,
-// FP32, in TMEM), row RB g + r = right-hand side r of box g, D = the stacked
-// E_s(g)^T (A operand) times K_o^T (NS x NS, B operand), accumulated over the
-// union of the boxes' offsets.  Few right-hand sides thus fill the rows with
-// boxes instead of padding.  Expansions are stored E[box][r][node] and the
-// operator table K[o][m][l] (target node m, source node l), both with node
-// stride NS, so every A row (one right-hand side) and every B row (one target
-// node) is a contiguous K-major row: the contraction over source nodes runs in
-// chunks of 32 TF32 (one 128-byte swizzle atom per row), and each chunk is one
-// pipeline stage: A (128 rows x 128 B) and B (NS rows x 128 B).
-// Warp-specialised: four producer warps copy each stage with cp.async
-// straight into the 128-byte-swizzled layout the MMA descriptors name and
-// signal the stage's `full` mbarrier with cp.async.mbarrier.arrive (128
-// arrivals); one thread of the fifth warp waits on `full`, issues the
-// 4 K=8 MMAs of the chunk and commits them to the stage's `empty` mbarrier,
-// which the producers wait on before refilling the stage.  kStages stages
-// are in flight, with no block-wide barrier in the main loop.
+// A CTA owns G target boxes of one octant class (so their interaction lists
+// use the same offsets) with RB right-hand sides each: four boxes of 16 or 32,
+// two of 64 (a 64-wide chunk of them for more).  It owns one accumulator D
+// (128 x NS, FP32, in TMEM) whose rows are the boxes' right-hand sides, D =
+// the stacked E_s(g)^T (A operand) times K_o^T (NS x NS, B operand),
+// accumulated over the union of the boxes' offsets.  Expansions are stored
+// E[box][r][node] and the operator table K[o][m][l] (target node m, source
+// node l), both with node stride NS, so every A row (one right-hand side) and
+// every B row (one target node) is a contiguous K-major row: the contraction
+// over source nodes runs in atoms of 32 TF32 (one 128-byte swizzle atom per
+// row), one or two of them per pipeline stage.
+// One thread copies each stage with TMA (a tile per box and one of the
+// operator; a box without a source at the offset reads rows past the end of E,
+// which are zero) and one thread of another warp waits for the stage's bytes,
+// issues its MMAs and commits them to the stage's `empty` mbarrier, on which
+// the copies of the next pass wait.  No block-wide barrier in the main loop.
+// The work is a stream of tiles from L2 (0.3 to 0.8 GB per apply), so what
+// counts is bytes in flight and copies issued: cp.async by 128 threads, each
+// arriving on the stage's barrier, took 0.4 us per 24 KB stage whatever was in
+// flight, and TMA takes 0.06 us per tile, hence both atoms in one tile where
+// they fit.  At 16 columns (21,195-panel bus, depth 5) cp.async over eight
+// boxes and two stages took 150 us an apply, this takes 66; at 64 columns (64-
+// net window) 134 us and 95.
 // The tensor cores read FP32 operands as TF32 (the operator table is stored
 // rounded to TF32, the expansions are truncated by the hardware).
 // Every mbarrier wait is bounded; on expiry the kernel records an error code,
 // drains (bounded) its own MMAs and copies, frees its TMEM and returns.
 #include "farfield.cuh"
+#include "tma.cuh"
 
 namespace gpx {
 
 namespace {
 
-constexpr int kProducers = 128;            // four producer warps
-constexpr int kThreads = kProducers + 32;  // + the MMA warp
+constexpr int kThreads = 128;  // warp 0 copies, warp 1 multiplies, all four store the accumulator
 constexpr int kWaitLimit = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -50,15 +54,6 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
     d |= (uint64_t)1 << 46;             // descriptor version (sm_100)
     d |= (uint64_t)2 << 61;             // SWIZZLE_128B
     return d;
-}
-
-// Byte offset of 16-byte chunk `chunk` (0..7) of row `row` in a 128B-swizzled tile.
-__device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t chunk) {
-    return (row >> 3) * 1024u + (row & 7u) * 128u + ((chunk ^ (row & 7u)) << 4);
-}
-
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
@@ -82,31 +77,46 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "r"(taddr));
 }
 
-template <int NS>
+template <int NS, int RB>
 struct TcCfg {
-    static constexpr int kStages = 2;
-    static constexpr uint32_t kATile = 128 * 128;              // 128 rows x 128 B
-    static constexpr uint32_t kBTile = NS * 128;               // NS rows x 128 B
-    static constexpr uint32_t kStage = kATile + kBTile;  // multiple of 1024
-    static constexpr uint32_t kSmem = kStages * kStage + 1024 + 256;  // + alignment slack + barriers
+    static constexpr int kMaxStages = 8;
+    static constexpr int kGroup = tc_group(RB);  // boxes
+    // Column atoms (32 source nodes) per stage: two where the accumulator's 128
+    // rows hold both atoms' rows of every box, so that one copy brings both.
+    static constexpr int kAtoms = 2 * kGroup * RB <= 128 ? 2 : 1;
+    static constexpr uint32_t kBox = kAtoms * RB * 128;           // one box's operand rows, atom-major
+    static constexpr uint32_t kATile = kGroup * kBox;
+    static constexpr uint32_t kBTile = kAtoms * NS * 128;
+    static constexpr uint32_t kStage = kATile + kBTile;           // multiple of 1024
+    // The MMA reads 128 A rows from an atom's start: those that are not its
+    // boxes' are the other atom's, other stage memory and past the last stage
+    // this pad.  They only reach accumulator rows that are never read.
+    static constexpr uint32_t kRead = (kAtoms - 1) * RB * 128 + 128 * 128;
+    static constexpr uint32_t kPad = kStage < kRead ? kRead - kStage : 0;
+    static constexpr uint32_t smem(int stages) {
+        return stages * kStage + kPad + 1024 + 256;  // + alignment slack + barriers
+    }
     static constexpr uint32_t kTmemCols = NS;                  // FP32 columns
-    static constexpr int kChunks = NS / 32;                    // contraction chunks per entry
+    static constexpr int kChunks = NS / (32 * kAtoms);         // contraction chunks (stages) per entry
     // Instruction descriptor: D F32, A/B TF32, both K-major, N = NS, M = 128.
     static constexpr uint32_t kIdesc =
         (1u << 4) | (2u << 7) | (2u << 10) | (((uint32_t)NS >> 3) << 17) | ((128u >> 4) << 24);
 };
 
 template <int NS, int RB>
-__global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __restrict__ E, float* __restrict__ L,
-                                                     const float* __restrict__ K32, int R, float scale,
-                                                     const double* __restrict__ box_scale, int* __restrict__ err) {
-    using C = TcCfg<NS>;
-    constexpr int S = C::kStages, G = 128 / RB;
+__global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const __grid_constant__ CUtensorMap E,
+                                                     const __grid_constant__ CUtensorMap K32, float* __restrict__ L,
+                                                     int R, int erows, float scale,
+                                                     const double* __restrict__ box_scale, int* __restrict__ err,
+                                                     int S) {
+    using C = TcCfg<NS, RB>;
+    constexpr int G = C::kGroup;
+    static_assert(C::kAtoms * G * RB <= 128, "one accumulator of 128 rows");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* sbase = smem_raw + (base - raw);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sbase + S * C::kStage);  // full[S], empty[S]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sbase + S * C::kStage + C::kPad);  // full[S], empty[S]
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2 * S);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int item = blockIdx.x;
@@ -119,13 +129,13 @@ __global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __
     __shared__ int s_bad;
     if (tid == 0) {
         for (int k = 0; k < S; ++k) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[k])), "r"(kProducers));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[k])), "r"(1));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[k])));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_bad = 0;
     }
-    if (warp == 4) {
+    if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(C::kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -135,63 +145,66 @@ __global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
 
-    // Copies of chunk q (entry q / kChunks, source nodes 32 (q % kChunks) ..)
-    // into stage q % S: A rows RB g .. RB g + RB - 1 from target g's source
-    // (zero-filled where a target has no source at this offset); B rows = the
-    // operator's target nodes.  Every producer thread copies 8 pieces of 16
-    // bytes of A and NS/16 of B; 8 consecutive threads read one 128-byte row
-    // segment, and the 16 rows of one pass lie within one box.
-    auto issue = [&](int q) {
-        const int e = e0 + q / C::kChunks, kc = q % C::kChunks;
-        const uint32_t a = base + (uint32_t)(q % S) * C::kStage;
-        const uint32_t b = a + C::kATile;
-        int srcs[G];
+    int issued = 0;  // chunks copied (copy thread), chunks whose MMAs were committed (MMA thread)
+    if (tid == 0) {
+        // Chunk (entry e, source nodes 32 kc ..) into stage st: A rows RB g ..
+        // RB g + RB - 1 from target g's source (rows past the end of E, which
+        // read as zero, where a target has no source at this offset); B rows =
+        // the operator's target nodes.  The indices of entry e + 1 are read
+        // while entry e is copied.
+        int cur[G], slot = 0, st = 0, round = 0;  // stage and pass of the ring
+        auto fetch = [&](int e, int (&srcs)[G], int& sl) {
 #pragma unroll
-        for (int g = 0; g < G; ++g) srcs[g] = lv.src[(int64_t)e * G + g];
+            for (int g = 0; g < G; ++g) srcs[g] = lv.src[(int64_t)e * G + g];
+            sl = lv.slot[e];
+        };
+        if (e0 < e1) fetch(e0, cur, slot);
+        bool stop = false;
+        for (int e = e0; e < e1 && !stop; ++e) {
+            int next[G], nslot;
+            fetch(min(e + 1, e1 - 1), next, nslot);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int row = (tid >> 3) + 16 * i, pc = tid & 7;
-            const int src = srcs[16 * i / RB];
-            const float* g = src >= 0 ? E + ((int64_t)src * R + r0 + row % RB) * NS + kc * 32 + pc * 4 : E;
-            cp16(a + swz(row, pc), g, src >= 0);
+            for (int kc = 0; kc < C::kChunks; ++kc) {
+                if ((round > 0 && !mbar_wait(smem_u32(&empty[st]), (uint32_t)((round - 1) & 1))) ||
+                    *(volatile int*)&s_bad) {
+                    atomicExch(&s_bad, 1);
+                    stop = true;
+                    break;
+                }
+                const uint32_t a = base + (uint32_t)st * C::kStage, bar = smem_u32(&full[st]);
+                mbar_expect(bar, C::kStage);
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    tma_load_atoms(a + g * C::kBox, &E, kc * C::kAtoms, cur[g] >= 0 ? cur[g] * R + r0 : erows, bar);
+                tma_load_atoms(a + C::kATile, &K32, kc * C::kAtoms, slot * NS, bar);
+                ++issued;
+                if (++st == S) {
+                    st = 0;
+                    ++round;
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) cur[g] = next[g];
+            slot = nslot;
         }
-        const float* Ko = K32 + (int64_t)lv.slot[e] * NS * NS + kc * 32;
-#pragma unroll
-        for (int i = 0; i < NS / 16; ++i) {
-            const int id = tid + kProducers * i, row = id >> 3, pc = id & 7;
-            cp16(b + swz(row, pc), Ko + (int64_t)row * NS + pc * 4, true);
-        }
-    };
-
-    int issued = 0;  // chunks whose MMAs were committed (MMA thread)
-    if (tid < kProducers) {
+        // no copy may be in flight when the block ends
+        for (int q = issued > S ? issued - S : 0; q < issued; ++q)
+            if (!mbar_wait(smem_u32(&full[q % S]), (uint32_t)((q / S) & 1))) atomicExch(&s_bad, 1);
+    } else if (tid == 32) {
+        int st = 0, round = 0;
         for (int q = 0; q < total; ++q) {
-            const int st = q % S;
-            if (q >= S && !mbar_wait(smem_u32(&empty[st]), (uint32_t)(((q / S) - 1) & 1))) {
+            if (!mbar_wait(smem_u32(&full[st]), (uint32_t)(round & 1))) {
                 atomicExch(&s_bad, 1);
                 break;
             }
-            if (*(volatile int*)&s_bad) break;
-            issue(q);
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[st]))
-                         : "memory");
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (tid == kProducers) {
-        for (int q = 0; q < total; ++q) {
-            const int st = q % S;
-            if (!mbar_wait(smem_u32(&full[st]), (uint32_t)((q / S) & 1))) {
-                atomicExch(&s_bad, 1);
-                break;
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t abase = base + (uint32_t)st * C::kStage, bbase = abase + C::kATile;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint64_t bd = desc_sw128(bbase + (uint32_t)k * 32u);
-                const uint32_t acc = (q > 0 || k > 0) ? 1u : 0u;
-                const uint64_t ad = desc_sw128(abase + (uint32_t)k * 32u);
+            for (int i = 0; i < 4 * C::kAtoms; ++i) {
+                const uint32_t at = i / 4, k = i % 4;
+                const uint64_t bd = desc_sw128(bbase + at * (NS * 128) + k * 32u);
+                const uint32_t acc = (q > 0 || i > 0) ? 1u : 0u;
+                const uint64_t ad = desc_sw128(abase + at * (RB * 128) + k * 32u);
                 asm volatile(
                     "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
@@ -201,6 +214,10 @@ __global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __
                              smem_u32(&empty[st]))
                          : "memory");
             issued = q + 1;
+            if (++st == S) {
+                st = 0;
+                ++round;
+            }
         }
         // Drain: the last commit covers every MMA issued before it (after an
         // expired wait too, so the TMEM is idle before it is freed).
@@ -213,11 +230,12 @@ __global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (s_bad) {
         if (tid == 0) atomicExch(err, 1);
-    } else if (tid < kProducers && total > 0) {
+    } else if (total > 0) {
         // Epilogue: warp w (0..3) reads TMEM lanes 32w..32w+31 = rows of D.
         const int row = warp * 32 + lane;
-        const int t = lv.item_t[(int64_t)item * G + row / RB];
-        float* dst = (t >= 0) ? L + ((int64_t)t * R + r0 + row % RB) * NS : nullptr;
+        const int g = row / (C::kAtoms * RB), rr = row % (C::kAtoms * RB);
+        const int t = g < G && rr < RB ? lv.item_t[(int64_t)item * G + g] : -1;
+        float* dst = (t >= 0) ? L + ((int64_t)t * R + r0 + rr) * NS : nullptr;
         const float sc = (t >= 0 && box_scale) ? (float)box_scale[t] : scale;
 #pragma unroll
         for (int cb = 0; cb < NS / 16; ++cb) {
@@ -236,42 +254,52 @@ __global__ void __launch_bounds__(kThreads) k_m2l_tc(TcLevel lv, const float* __
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 4)
+    if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::kTmemCols));
 }
 
+// Stages: what the CTAs that share an SM leave each other of its shared memory
+// (227 KB, 1 KB of it reserved per CTA), four CTAs at most, since the grids of
+// many items fill the copy path with four CTAs of two stages.
 template <int NS, int RB>
-void launch_rb(Ctx& c, const TcLevel& lv, const float* E, float* L, const float* K32, int R, float scale,
-               const double* box_scale, int* err) {
-    using Cf = TcCfg<NS>;
-    set_smem_once(k_m2l_tc<NS, RB>, (int)Cf::kSmem);
-    k_m2l_tc<NS, RB><<<dim3(lv.nitems, R / RB), kThreads, Cf::kSmem, c.stream>>>(lv, E, L, K32, R, scale, box_scale,
-                                                                                 err);
+void launch_rb(Ctx& c, const TcLevel& lv, const float* E, int64_t nbox, float* L, const float* K32, int R,
+              float scale, const double* box_scale, int* err) {
+    using Cf = TcCfg<NS, RB>;
+    const int64_t ctas = (int64_t)lv.nitems * (R / RB);
+    const int per_sm = (int)std::min<int64_t>(4, (ctas + 147) / 148);
+    const int room = 227 * 1024 / per_sm - 1024;
+    int S = Cf::kMaxStages;
+    while (S > 2 && (int)Cf::smem(S) > room) --S;
+    set_smem_once(k_m2l_tc<NS, RB>, (int)Cf::smem(S));
+    k_m2l_tc<NS, RB><<<dim3(lv.nitems, R / RB), kThreads, Cf::smem(S), c.stream>>>(
+        lv, tma_map_f32(E, nbox * R, NS, RB, Cf::kAtoms), tma_map_f32(K32, (int64_t)343 * NS, NS, NS, Cf::kAtoms), L, R, (int)(nbox * R),
+        scale, box_scale, err, S);
     GPX_LAUNCH_CHECK();
 }
 
 template <int NS>
-void launch_ns(Ctx& c, const TcLevel& lv, const float* E, float* L, const float* K32, int R, float scale,
-               const double* box_scale, int* err) {
+void launch_ns(Ctx& c, const TcLevel& lv, const float* E, int64_t nbox, float* L, const float* K32, int R,
+               float scale, const double* box_scale, int* err) {
     if (R == 16)
-        launch_rb<NS, 16>(c, lv, E, L, K32, R, scale, box_scale, err);
+        launch_rb<NS, 16>(c, lv, E, nbox, L, K32, R, scale, box_scale, err);
     else if (R == 32)
-        launch_rb<NS, 32>(c, lv, E, L, K32, R, scale, box_scale, err);
+        launch_rb<NS, 32>(c, lv, E, nbox, L, K32, R, scale, box_scale, err);
     else
-        launch_rb<NS, 64>(c, lv, E, L, K32, R, scale, box_scale, err);
+        launch_rb<NS, 64>(c, lv, E, nbox, L, K32, R, scale, box_scale, err);
 }
 
 }  // namespace
 
-void launch_m2l_tc(Ctx& c, const TcLevel& lv, int ns, const float* E, float* L, const float* K32, int R, float scale,
-                   const double* box_scale, int* err) {
+void launch_m2l_tc(Ctx& c, const TcLevel& lv, int ns, const float* E, int64_t nbox, float* L, const float* K32, int R,
+                   float scale, const double* box_scale, int* err) {
     if (lv.nitems == 0) return;
     if (R != 16 && R != 32 && R % 64 != 0)
         throw Error(GPX_ERR_INTERNAL, "tensor-core M2L needs 16, 32 or a multiple of 64 rows per box");
+    if (nbox * R > INT32_MAX - 128) throw Error(GPX_ERR_INTERNAL, "expansion rows past 32-bit tile coordinates");
     if (ns == 64)
-        launch_ns<64>(c, lv, E, L, K32, R, scale, box_scale, err);
+        launch_ns<64>(c, lv, E, nbox, L, K32, R, scale, box_scale, err);
     else if (ns == 128)
-        launch_ns<128>(c, lv, E, L, K32, R, scale, box_scale, err);
+        launch_ns<128>(c, lv, E, nbox, L, K32, R, scale, box_scale, err);
     else
         throw Error(GPX_ERR_INTERNAL, "tensor-core M2L runs node strides 64 and 128 (orders 4 and 5)");
 }

@@ -351,7 +351,9 @@ void upload_plan(Ctx& ctx, const Plan& p, const DevM2L* m2l, DevPlanBufs& d) {
 }
 
 // Tensor-core M2L work lists of every level (groups of tc_group target boxes of
-// the same octant class in Morton order sharing one offset loop).
+// the same octant class, consecutive in Morton order, sharing one offset loop;
+// the items of a level with the longest lists first, so that no SM starts one
+// of them last).
 struct TcLists {
     std::vector<TcLevel> level;  // per level (empty below 2)
     TcLevel all;                 // levels 2..L in one list
@@ -376,26 +378,41 @@ void build_tc_lists(Ctx& ctx, const Plan& pl, int group, TcLists& out) {
         }
         int n = 0;
         std::vector<int32_t> per((size_t)group * 343);
-        for (auto& v : cls)
-            for (size_t k = 0; k < v.size(); k += group) {
-                std::fill(per.begin(), per.end(), -1);  // per[slot * group + i]
-                for (int i = 0; i < group; ++i) {
-                    const int32_t t = k + i < v.size() ? v[k + i] : -1;
-                    it.push_back(t);
-                    if (t < 0) continue;
-                    for (int64_t e = pl.m2l_off[t]; e < pl.m2l_off[t + 1]; ++e)
-                        per[(size_t)pl.m2l_slot[e] * group + i] = pl.m2l_src[e];
-                }
-                ioff.push_back((int32_t)sl.size());
-                for (int q = 0; q < 343; ++q) {
-                    bool any = false;
-                    for (int i = 0; i < group; ++i) any = any || per[(size_t)q * group + i] >= 0;
-                    if (!any) continue;
-                    sl.push_back(q);
-                    for (int i = 0; i < group; ++i) src.push_back(per[(size_t)q * group + i]);
-                }
-                ++n;
+        struct Item {
+            int cls;
+            size_t k;
+            int64_t len;
+        };
+        std::vector<Item> order;
+        for (int q = 0; q < 8; ++q)
+            for (size_t k = 0; k < cls[q].size(); k += group) {
+                int64_t len = 0;
+                for (size_t i = k; i < std::min(k + group, cls[q].size()); ++i)
+                    len = std::max(len, pl.m2l_off[cls[q][i] + 1] - pl.m2l_off[cls[q][i]]);
+                order.push_back({q, k, len});
             }
+        std::stable_sort(order.begin(), order.end(), [](const Item& a, const Item& b) { return a.len > b.len; });
+        for (const Item& o : order) {
+            const auto& v = cls[o.cls];
+            const size_t k = o.k;
+            std::fill(per.begin(), per.end(), -1);  // per[slot * group + i]
+            for (int i = 0; i < group; ++i) {
+                const int32_t t = k + i < v.size() ? v[k + i] : -1;
+                it.push_back(t);
+                if (t < 0) continue;
+                for (int64_t e = pl.m2l_off[t]; e < pl.m2l_off[t + 1]; ++e)
+                    per[(size_t)pl.m2l_slot[e] * group + i] = pl.m2l_src[e];
+            }
+            ioff.push_back((int32_t)sl.size());
+            for (int q = 0; q < 343; ++q) {
+                bool any = false;
+                for (int i = 0; i < group; ++i) any = any || per[(size_t)q * group + i] >= 0;
+                if (!any) continue;
+                sl.push_back(q);
+                for (int i = 0; i < group; ++i) src.push_back(per[(size_t)q * group + i]);
+            }
+            ++n;
+        }
         ranges[l].n = n;
     }
     ioff.push_back((int32_t)sl.size());
@@ -836,11 +853,11 @@ struct Operator {
                     // L^ rows of boxes with M2L work are overwritten; the others stay
                     // at the zero they were allocated with
                     launch_m2l_compress(ctx, E32.p, ns, m2l->Vt_hi.p, m2l->Vt_lo.p, Eh32.p, row0, nrows, tc_err.p);
-                    launch_m2l_tc(ctx, level < 0 ? tc.all : tc.level[level], kShared, Eh32.p, Lh32.p, m2l->C32.p,
-                                  Rb32, (float)scale, level < 0 ? box_scale.p : nullptr, tc_err.p);
+                    launch_m2l_tc(ctx, level < 0 ? tc.all : tc.level[level], kShared, Eh32.p, pl.nbox(), Lh32.p,
+                                  m2l->C32.p, Rb32, (float)scale, level < 0 ? box_scale.p : nullptr, tc_err.p);
                     launch_m2l_decompress(ctx, Lh32.p, m2l->U_hi.p, m2l->U_lo.p, ns, L32.p, row0, nrows, tc_err.p);
                 } else if (tc32)
-                    launch_m2l_tc(ctx, level < 0 ? tc.all : tc.level[level], node_stride(pl.n), E32.p, L32.p,
+                    launch_m2l_tc(ctx, level < 0 ? tc.all : tc.level[level], node_stride(pl.n), E32.p, pl.nbox(), L32.p,
                                   m2l->K32.p, Rb32, (float)scale, level < 0 ? box_scale.p : nullptr, tc_err.p);
                 else
                     launch_m2l_fac<float>(ctx, fac32, b0, nb, L32.p, E32.p, Rb32, pl.n3);

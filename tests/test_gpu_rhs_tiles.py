@@ -35,7 +35,7 @@ def test_apply_at_column_tile_edges(ctx, orc, order, nrhs):
                                                    (5, 0, 0, 33), (6, 3, 0, 12), (6, 0, 0, 64)])
 def test_mixed_apply_at_row_padding_edges(ctx, order, m2l, far_tc, cols):
     """The FP32 far field pads the right-hand sides to 16, 32 or a multiple of
-    64 rows per box and groups 8, 4 or 2 boxes per tensor-core item: a column's
+    64 rows per box and groups 4 or 2 boxes per tensor-core item: a column's
     result does not depend on how many columns are applied with it (the kernels
     sum every output in the same order), so the columns of a 130-column apply
     (three chunks of 64) agree bit for bit."""
