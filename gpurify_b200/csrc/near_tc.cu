@@ -6,18 +6,27 @@
 // CUDA cores it is compute bound; on the tensor cores it is bound by streaming
 // the near blocks from HBM.
 //
-// One CTA per (work item = target leaf and <= 128 of its rows, 64-wide chunk
-// of right-hand sides), D = 128 x 64 FP32 in TMEM.  The contraction runs over
+// One CTA per (work item = target leaf and <= 128 of its rows, NT-wide chunk
+// of right-hand sides, NT = 16, 32 or 64), D = 128 x NT FP32 in TMEM (16
+// columns run as 32, the others never read).  The contraction runs over
 // the leaf's S near-source panels in slices of 32; each slice is one stage of
 // a kStages ring in shared memory:
 //   A (128 x 32, K-major, 128-byte swizzle) = the item's P rows, streamed from
 //     HBM;
-//   B_hi, B_lo (32 x 64 each, MN-major, 128-byte swizzle on a 32-byte base) = the 32 source
+//   B_hi, B_lo (32 x NT each, MN-major, 128-byte swizzle on a 32-byte base) = the 32 source
 //     panels' rows of X_hi = tf32(x) and X_lo = tf32(x - x_hi), gathered from
 //     the L2-resident split copies written by k_split_tf32.  A source row of
 //     X is 64 contiguous FP32 values, which is exactly one K row of an
 //     MN-major tile, so the gather is a plain copy: no transpose and no
 //     per-slice register work.
+// What bounds it: with 28 rows per leaf (bus) or 55 (window) the gather of X (8 NT bytes
+// a source panel against 4 per row of P) is most of what a CTA reads, from L2
+// at 55 to 60 bytes a clock and SM.  So the copies follow NT (a 12-column apply
+// of a 21,195-panel bus: 97 us with 64 columns copied, 68 with 16, and four
+// stages), and four neighbouring threads read 64 contiguous bytes, whole
+// sectors (64-net window, 64 columns: 228 -> 202 us).  One arrival per warp
+// after a lagging wait for its copies, in place of one per thread when they
+// land, was slower (300 and 104 us).
 // D += A B_hi + A B_lo represents X to about 2^-21, so the operator stays
 // linear in X (the GMRES inner solves converge as for any fixed matrix); the
 // one approximation left is P rounded once to TF32 (round to nearest, stored
@@ -41,29 +50,32 @@ namespace {
 constexpr int kProducers = 128;            // four producer warps, also the epilogue
 constexpr int kThreads = kProducers + 32;  // + the MMA warp
 constexpr uint32_t kATile = 128 * 128;      // 128 rows x 128 B
-constexpr uint32_t kBTile = 32 * 256;       // 32 K rows x 64 FP32
 // Operand modes: 0 = P (TF32) and the split X_hi, X_lo gathered from global
 // memory; 1 = P kept in FP32 and split into hi and lo on chip (three
 // products); 2 = X gathered once as FP32 and split into hi and lo on chip
 // (half the gather traffic of mode 0, the same products).
 // Stage layout: A, [A_lo in mode 1], B_hi, B_lo.  Modes 0 and 2 stage 32 KB
-// and three stages fit twice per SM; mode 1 stages 48 KB, two stages.
-template <int MODE>
+// at NT = 64 and 24 KB below, of which three and four stages fit twice per SM;
+// mode 1 stages 48 or 40 KB, two stages.
+template <int MODE, int NT>
 struct NearCfg {
     static constexpr bool SP = MODE == 1;
-    static constexpr int kStages = SP ? 2 : 3;
+    static constexpr int kN = NT < 32 ? 32 : NT;                      // columns of the MMA: whole 32-wide blocks
+    static constexpr int kBlocks = kN / 32;                           // of B
+    static constexpr uint32_t kBTile = 32 * 128 * kBlocks;            // 32 K rows
+    static constexpr int kStages = SP ? 2 : NT <= 32 ? 4 : 3;
     static constexpr uint32_t kALo = kATile;                          // offset of A_lo (SP)
     static constexpr uint32_t kBOff = SP ? 2 * kATile : kATile;       // offset of B_hi
     static constexpr uint32_t kStage = kBOff + 2 * kBTile;            // multiple of 1024
     // + alignment slack, barriers and TMEM slot, and 4 KB past the last
     // stage so that no MMA operand read can leave the allocation
     static constexpr uint32_t kSmemBytes = kStages * kStage + 1024 + 256 + 4096;
+    static constexpr uint32_t kTmemCols = kN;
+    // Instruction descriptor: D F32, A/B TF32, A K-major, B MN-major, N = kN, M = 128.
+    static constexpr uint32_t kIdesc =
+        (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | (((uint32_t)kN >> 3) << 17) | ((128u >> 4) << 24);
 };
-constexpr uint32_t kTmemCols = 64;
 constexpr int kWaitLimit = 1 << 22;
-// Instruction descriptor: D F32, A/B TF32, A K-major, B MN-major, N = 64, M = 128.
-constexpr uint32_t kIdesc =
-    (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -102,13 +114,14 @@ __device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t chunk) {
     return (row >> 3) * 1024u + (row & 7u) * 128u + ((chunk ^ (row & 7u)) << 4);
 }
 
-// Byte offset of 16-byte chunk q (0..15: FP32 columns 4q..4q+3) of K row k
-// (0..31) in the MN-major B tile: atom (4-row K group k/4, MN block q/8) at
-// (2 (k/4) + q/8) x 512 B, row k%4 of the atom, 32-byte granule (q%8)/2
-// swizzled by the row.
+// Byte offset of 16-byte chunk q (FP32 columns 4q..4q+3) of K row k (0..31) in
+// the MN-major B tile of NB 32-wide blocks: atom (4-row K group k/4, MN block
+// q/8) at (NB (k/4) + q/8) x 512 B, row k%4 of the atom, 32-byte granule
+// (q%8)/2 swizzled by the row.
+template <int NB>
 __device__ __forceinline__ uint32_t swz_mn(uint32_t k, uint32_t q) {
     const uint32_t r = k & 3u;
-    return ((k >> 2) * 2u + (q >> 3)) * 512u + r * 128u + ((((q & 7u) >> 1) ^ r) << 5) + ((q & 1u) << 4);
+    return ((k >> 2) * NB + (q >> 3)) * 512u + r * 128u + ((((q & 7u) >> 1) ^ r) << 5) + ((q & 1u) << 4);
 }
 
 __device__ __forceinline__ float to_tf32(float x) {
@@ -151,15 +164,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // a stage after its own copies of that stage completed and were split (one
 // stage of copies stays in flight per producer); in mode 0 the copies
 // signal the stage themselves.
-template <int MODE>
+template <int MODE, int NT>
 __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int32_t* __restrict__ it_leaf,
                                                             const int32_t* __restrict__ it_row0,
                                                             const float* __restrict__ P,
                                                             const float* __restrict__ Xhi,
                                                             const float* __restrict__ Xlo, double* __restrict__ Y,
                                                             int R, int* __restrict__ err) {
-    using Cfg = NearCfg<MODE>;
+    using Cfg = NearCfg<MODE, NT>;
     constexpr bool SP = Cfg::SP;
+    constexpr int NB = Cfg::kBlocks;
+    constexpr uint32_t kBTile = Cfg::kBTile;
     constexpr bool SB = MODE == 2;
     constexpr int kStages = Cfg::kStages;
     constexpr uint32_t kStage = Cfg::kStage;
@@ -176,7 +191,7 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t = it_leaf[blockIdx.x];
     const int r0 = it_row0[blockIdx.x];
-    const int rc = blockIdx.y * 64;
+    const int rc = blockIdx.y * NT;
     const int64_t tb = p.leaf_begin[t] + r0;
     const int m = min((int)(p.leaf_begin[t + 1] - p.leaf_begin[t]) - r0, 128);
     const int S = p.near_S[t];
@@ -195,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
     }
     if (warp == 4) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(kTmemCols));
+                     "r"(Cfg::kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -205,8 +220,9 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
 
     if (tid < kProducers) {
         // B: this thread copies K row kb = tid / 4 of every slice, chunks
-        // 4 (tid % 4) .. 4 (tid % 4) + 3 of X_hi and X_lo.
-        const int kb = tid >> 2, q0 = (tid & 3) * 4;
+        // 4 i + tid % 4 of X_hi and X_lo, so that four neighbouring threads
+        // read 64 contiguous bytes.
+        const int kb = tid >> 2, q0 = tid & 3;
         int e = 0;
         // SP: split the A chunks this thread copied into stage `jj` (after
         // its copies landed), then signal the stage.
@@ -229,13 +245,13 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[sst])) : "memory");
         };
         // SB: split the B chunks this thread copied into stage `jj` (K row kb,
-        // chunks q0 .. q0 + 3: FP32 x into hi in place and lo beside it).
+        // chunks q0 + 4 i: FP32 x into hi in place and lo beside it).
         auto split_b_and_signal = [&](int jj) {
             const int sst = jj % kStages;
             uint8_t* bt = sbase + (size_t)sst * kStage + Cfg::kBOff;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t d = swz_mn((uint32_t)kb, (uint32_t)(q0 + i));
+            for (int i = 0; i < NT / 16; ++i) {
+                const uint32_t d = swz_mn<NB>((uint32_t)kb, (uint32_t)(q0 + 4 * i));
                 float4* hp = reinterpret_cast<float4*>(bt + d);
                 float4* lp = reinterpret_cast<float4*>(bt + kBTile + d);
                 const float4 v = *hp;
@@ -249,11 +265,12 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
         int signalled = 0;  // modes 1 and 2: stages split and signalled
         for (int j = 0; j < nsl; ++j) {
             const int st = j % kStages;
+            bool stop = *(volatile int*)&s_bad;
             if (j >= kStages && !mbar_wait(smem_u32(&empty[st]), (uint32_t)(((j / kStages) - 1) & 1))) {
                 atomicExch(&s_bad, 1);
-                break;
+                stop = true;
             }
-            if (*(volatile int*)&s_bad) break;
+            if (__any_sync(0xffffffffu, stop)) break;
             const uint32_t a = base + (uint32_t)st * kStage;
             const uint32_t bh = a + Cfg::kBOff, bl = bh + kBTile;
             const int k0 = j * 32;
@@ -273,11 +290,11 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
                 gid = s_beg[e] + (k - s_pre[e]);
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int q = q0 + i, col = rc + 4 * q;
+            for (int i = 0; i < NT / 16; ++i) {
+                const int q = q0 + 4 * i, col = rc + 4 * q;
                 const bool ok = gid >= 0 && col < R;
                 const int64_t off = ok ? gid * R + col : 0;
-                const uint32_t d = swz_mn((uint32_t)kb, (uint32_t)q);
+                const uint32_t d = swz_mn<NB>((uint32_t)kb, (uint32_t)q);
                 cp16(bh + d, Xhi + off, ok);
                 if constexpr (!SB) cp16(bl + d, Xlo + off, ok);
             }
@@ -324,19 +341,19 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const uint64_t ad = desc_k_sw128(a + (uint32_t)kk * 32u);
-                const uint64_t bdh = desc_mn_sw128b32(bh + (uint32_t)kk * 2048u, 512u, 1024u);
-                const uint64_t bdl = desc_mn_sw128b32(bl + (uint32_t)kk * 2048u, 512u, 1024u);
+                const uint64_t bdh = desc_mn_sw128b32(bh + (uint32_t)kk * (NB * 1024u), 512u, NB * 512u);
+                const uint64_t bdl = desc_mn_sw128b32(bl + (uint32_t)kk * (NB * 1024u), 512u, NB * 512u);
                 const uint32_t accf = (j > 0 || kk > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bdh), "r"(kIdesc), "r"(accf));
+                    "l"(ad), "l"(bdh), "r"(Cfg::kIdesc), "r"(accf));
                 asm volatile("tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(ad), "l"(bdl),
-                             "r"(kIdesc));
+                             "r"(Cfg::kIdesc));
                 if constexpr (SP) {
                     const uint64_t adl = desc_k_sw128(a + Cfg::kALo + (uint32_t)kk * 32u);
                     asm volatile("tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(adl),
-                                 "l"(bdh), "r"(kIdesc));
+                                 "l"(bdh), "r"(Cfg::kIdesc));
                 }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -360,7 +377,7 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
         const int row = warp * 32 + lane;
         double* dst = row < m ? Y + (tb + row) * R + rc : nullptr;
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
+        for (int cb = 0; cb < NT / 16; ++cb) {
             uint32_t v[16];
             tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16), v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -377,7 +394,7 @@ __global__ void __launch_bounds__(kThreads) k_near_apply_tc(DevPlan p, const int
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+    if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::kTmemCols));
 }
 
 // X32 = (float) x for the FP32 far field, and the split X_hi = tf32(x),
@@ -408,14 +425,26 @@ void launch_to_tf32(Ctx& c, const double* a, float* b, int64_t n) {
     c.launches += 1;
 }
 
+template <int MODE, int NT>
+void near_tc_tile(Ctx& c, const DevPlan& p, int nitems, const int32_t* it_leaf, const int32_t* it_row0,
+                    const float* P, const float* Xa, const float* Xb, double* Y, int R, int* err) {
+    using Cfg = NearCfg<MODE, NT>;
+    const dim3 grid(nitems, (R + NT - 1) / NT);
+    set_smem_once(k_near_apply_tc<MODE, NT>, (int)Cfg::kSmemBytes);
+    k_near_apply_tc<MODE, NT>
+        <<<grid, kThreads, Cfg::kSmemBytes, c.stream>>>(p, it_leaf, it_row0, P, Xa, Xb, Y, R, err);
+    GPX_LAUNCH_CHECK();
+}
+
 template <int MODE>
 void near_tc_launch(Ctx& c, const DevPlan& p, int nitems, const int32_t* it_leaf, const int32_t* it_row0,
                     const float* P, const float* Xa, const float* Xb, double* Y, int R, int* err) {
-    const dim3 grid(nitems, (R + 63) / 64);
-    set_smem_once(k_near_apply_tc<MODE>, (int)NearCfg<MODE>::kSmemBytes);
-    k_near_apply_tc<MODE><<<grid, kThreads, NearCfg<MODE>::kSmemBytes, c.stream>>>(p, it_leaf, it_row0, P, Xa, Xb, Y,
-                                                                                  R, err);
-    GPX_LAUNCH_CHECK();
+    if (R <= 16)
+        near_tc_tile<MODE, 16>(c, p, nitems, it_leaf, it_row0, P, Xa, Xb, Y, R, err);
+    else if (R <= 32)
+        near_tc_tile<MODE, 32>(c, p, nitems, it_leaf, it_row0, P, Xa, Xb, Y, R, err);
+    else
+        near_tc_tile<MODE, 64>(c, p, nitems, it_leaf, it_row0, P, Xa, Xb, Y, R, err);
 }
 
 void launch_near_apply_tc(Ctx& c, const DevPlan& p, int64_t nnz, int nitems, const int32_t* it_leaf,

@@ -66,3 +66,19 @@ def test_device_loop_matches_host_loop_at_reduction_sizes(ctx, nets, panels_um):
     a, ra = ctx.cap_solve(p["verts"], p["cond"], nc, **kw)
     b, rb = ctx.cap_solve(p["verts"], p["cond"], nc, no_graphs=1, **kw)
     assert np.array_equal(a, b) and ra["iterations"] == rb["iterations"] > 1
+
+
+@pytest.mark.parametrize("near", [0, 2, 3])
+@pytest.mark.parametrize("cols", [4, 16, 20, 32, 36, 64])
+def test_mixed_near_apply_at_column_tile_edges(ctx, near, cols):
+    """The tensor-core near apply copies 16, 32 or 64 columns of X per item: a
+    column's sums do not depend on the tile it is in, so the columns of a
+    132-column apply (tiles of 64 and a remainder) agree bit for bit."""
+    lay = layouts.two_wires(length_nm=6000)
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, mesh_max_edge_m=0.3e-6,
+                             max_panels=-1)
+    sig = np.random.default_rng(10 * near + cols).standard_normal((len(p["verts"]), 132))
+    kw = dict(order=4, max_level=3, dense_below=-1, precision=_lib.PREC_MIXED, mixed_m2l=2, far_quad=1, mixed_near=near)
+    wide, _ = ctx.operator_apply(p["verts"], sig, **kw)
+    few, _ = ctx.operator_apply(p["verts"], np.ascontiguousarray(sig[:, :cols]), **kw)
+    assert np.isfinite(few).all() and np.array_equal(few, wide[:, :cols])
