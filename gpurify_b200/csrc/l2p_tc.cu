@@ -9,13 +9,19 @@
 //   A = S (panels x nodes): K-major, one row per panel (split into TF32 hi and
 //       lo parts once per solve, rows of 128 nodes);
 //   B = L[leaf] (right-hand sides x nodes): K-major, one row per right-hand
-//       side, split into TF32 hi and lo parts in shared memory once staged.
+//       side, split into TF32 hi and lo parts on the way to shared memory.
 // D = S_hi L_hi + S_hi L_lo + S_lo L_hi is accurate to about 2^-21.  The
 // contraction over the nodes runs in slices of 32 through a 2-stage ring:
-// all threads copy a slice with cp.async, split its L tile, and one thread
-// issues the slice's MMAs and commits them to the stage's mbarrier, which
-// the copies of the slice two ahead wait on (bounded).  The epilogue adds
-// coef D to the panels' FP64 rows of Y.
+// all threads copy the slice's S rows with cp.async and its L rows through
+// registers, read a slice ahead, and one thread issues the slice's MMAs and
+// commits them to the stage's mbarrier, which the copies of the slice two
+// ahead wait on (bounded).  The epilogue adds coef D to the panels' FP64 rows
+// of Y, staged through shared memory so that a warp updates a row at a time.
+// What bounds it: a CTA has four short slices and then its rows of Y, a chain
+// of latencies, so what counts is CTAs per SM and requests in flight.  With 64
+// staged S rows a stage takes 32 KB and three CTAs share an SM; on the 64-net
+// window (2,091 items, 64 columns) 72 us against 129 with 128 rows staged (two
+// CTAs), L split in place between two barriers, and a thread per row of Y.
 #include "farfield.cuh"
 
 namespace gpx {
@@ -24,10 +30,13 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWS = 128;                      // row stride of the split weight arrays
-constexpr uint32_t kATile = 128 * 128;        // 128 rows x 32 FP32 (128 B)
+// An item has at most 64 panels; the MMA reads 128 A rows from a tile's start,
+// the other 64 from the tile behind it, into accumulator rows nobody reads.
+constexpr uint32_t kATile = 64 * 128;         // 64 rows x 32 FP32 (128 B)
 constexpr uint32_t kBTile = 64 * 128;         // 64 rows x 32 FP32
-constexpr uint32_t kStage = 2 * kATile + 2 * kBTile;  // A_hi, A_lo, B_hi, B_lo: 48 KB
-constexpr uint32_t kSmemBytes = 2 * kStage + 1024 + 64 + 4096;
+constexpr uint32_t kStage = 2 * kATile + 2 * kBTile;  // A_hi, A_lo, B_hi, B_lo: 32 KB
+constexpr uint32_t kSmemBytes = 2 * kStage + 1024 + 64;
+constexpr int kPitch = 68;                    // floats per row of the staged result (64 rows in a stage's 32 KB)
 constexpr uint32_t kTmemCols = 64;
 constexpr int kWaitLimit = 1 << 22;
 // Instruction descriptor: D F32, A/B TF32, both K-major, N = 64, M = 128.
@@ -117,56 +126,63 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
-    // copies of slice q into stage q % 2: A rows = the item's panels (rows
-    // past cnt are not loaded: their D rows are never stored), B rows = the
-    // leaf's right-hand sides (L has Rb rows per box; the chunk's others are zero)
+    // S rows of slice q into stage q % 2 (rows past cnt are not loaded: their D
+    // rows are never read)
     auto issue = [&](int q) {
         const uint32_t a = base + (uint32_t)(q & 1) * kStage;
-        for (int e = tid; e < 64 * 8; e += kThreads) {
+        for (int e = tid; e < cnt * 8; e += kThreads) {
             const int row = e >> 3, c = e & 7;
-            if (row < cnt) {
-                const int64_t off = (jb + row) * kWS + 32 * q + 4 * c;
-                cp16(a + swz(row, c), Shi + off, true);
-                cp16(a + kATile + swz(row, c), Slo + off, true);
-            }
-            const bool have = rc + row < Rb;
-            cp16(a + 2 * kATile + swz(row, c), have ? src + (int64_t)row * NS + 32 * q + 4 * c : L, have);
+            const int64_t off = (jb + row) * kWS + 32 * q + 4 * c;
+            cp16(a + swz(row, c), Shi + off, true);
+            cp16(a + kATile + swz(row, c), Slo + off, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the leaf's right-hand sides of slice q (L has Rb rows per box; the
+    // chunk's others are zero), into registers while slice q - 1 is multiplied
+    float4 lr[4];
+    auto fetch = [&](int q) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 3) + 16 * i;
+            lr[i] = rc + row < Rb ? *reinterpret_cast<const float4*>(src + (int64_t)row * NS + 32 * q + 4 * (tid & 7))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     };
     bool bad = false;
     int committed = 0;  // slices whose MMAs thread 0 committed (uniform across the CTA)
     issue(0);
+    fetch(0);
     for (int q = 0; q < nsl; ++q) {
         const int st = q & 1;
+        // L_hi and L_lo of this slice; the stage's last MMAs were waited for before its S rows were requested
+        {
+            uint8_t* b = sbase + (size_t)st * kStage + 2 * kATile;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t o = swz((uint32_t)((tid >> 3) + 16 * i), (uint32_t)(tid & 7));
+                const float4 v = lr[i];
+                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+                *reinterpret_cast<float4*>(b + kBTile + o) =
+                    make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z), to_tf32(v.w - h.w));
+                *reinterpret_cast<float4*>(b + o) = h;
+            }
+        }
         if (q + 1 < nsl) {
             // stage (q+1)&1 last held slice q-1: its MMAs must be done
             if (q >= 1 && !mbar_wait(smem_u32(&bars[(q + 1) & 1]), (uint32_t)(((q - 1) >> 1) & 1))) bad = true;
-            if (__syncthreads_or(bad)) {
-                bad = true;
-                break;
-            }
-            issue(q + 1);
+            if (!bad) issue(q + 1);
+            fetch(q + 1);
+        }
+        if (q + 1 < nsl && !bad)
             asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
+        else
             asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        // split the L tile of this slice: B_hi in place, B_lo beside it
-        {
-            uint8_t* b = sbase + (size_t)st * kStage + 2 * kATile;
-            for (int e = tid; e < 64 * 8; e += kThreads) {
-                const uint32_t o = swz((uint32_t)(e >> 3), (uint32_t)(e & 7));
-                float4* hp = reinterpret_cast<float4*>(b + o);
-                float4* lp = reinterpret_cast<float4*>(b + kBTile + o);
-                const float4 v = *hp;
-                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-                *lp = make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z), to_tf32(v.w - h.w));
-                *hp = h;
-            }
-        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
+        if (__syncthreads_or(bad)) {
+            bad = true;
+            break;
+        }
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t ah = base + (uint32_t)st * kStage, al = ah + kATile;
@@ -205,26 +221,35 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
     }
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!bad) {
-        const int row = warp * 32 + lane;
-        double* y = row < cnt ? Y + (jb + row) * R + rc : nullptr;
+        // D through shared memory (the stages are idle), so that every warp
+        // updates whole rows of Y
+        float* d = reinterpret_cast<float*>(sbase);
+        if (warp * 32 < cnt) {
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (y) {
+            for (int cb = 0; cb < 4; ++cb) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float4* o = reinterpret_cast<float4*>(d + (warp * 32 + lane) * kPitch + cb * 16);
 #pragma unroll
-                for (int k = 0; k < 16; k += 2) {
-                    const int col = cb * 16 + k;
-                    if (rc + col + 1 < R) {
-                        double2 o = *reinterpret_cast<double2*>(y + col);
-                        o.x += coef * (double)__uint_as_float(v[k]);
-                        o.y += coef * (double)__uint_as_float(v[k + 1]);
-                        *reinterpret_cast<double2*>(y + col) = o;
-                    } else if (rc + col < R) {
-                        y[col] += coef * (double)__uint_as_float(v[k]);
-                    }
-                }
+                for (int k = 0; k < 4; ++k)
+                    o[k] = make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
+                                       __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3]));
+            }
+        }
+        __syncthreads();
+        // R is a multiple of 4
+        const int col = 2 * lane;
+        if (rc + col < R) {
+            double* y = Y + jb * R + rc + col;
+#pragma unroll 8
+            for (int row = warp; row < cnt; row += 4) {
+                const float2 v = *reinterpret_cast<const float2*>(d + row * kPitch + col);
+                double2* o = reinterpret_cast<double2*>(y + (int64_t)row * R);
+                double2 w = *o;
+                w.x += coef * (double)v.x;
+                w.y += coef * (double)v.y;
+                *o = w;
             }
         }
     }
