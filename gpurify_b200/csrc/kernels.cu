@@ -72,9 +72,10 @@ __global__ void k_diag_inv(DevPlan p, const double* __restrict__ P, double* __re
 
 // FP64 near apply: per work item (target leaf, <= 64 rows) and chunk of 8 NT
 // right-hand sides, Y[rows][.] = P_t[rows][0:S] X[src(0:S)][.] on FP64 matrix
-// instructions.  KC source panels per stage go through a three-stage cp.async
-// ring: the item's P rows (contiguous along the contraction) and the gathered
-// X rows (contiguous along the right-hand sides).  Four warps: WN = NT / NTW of
+// instructions.  KC source panels per stage go through a cp.async ring of three
+// stages (two where four CTAs of 64 columns share an SM): the item's P rows
+// (contiguous along the contraction) and the gathered X rows (contiguous along
+// the right-hand sides).  Four warps: WN = NT / NTW of
 // them side by side over the columns, WM over the 8-row tiles (tile i belongs
 // to warp i % WM), so narrow chunks do not leave warps without work.  Row tiles
 // past the item's rows are skipped: a 12-row leaf costs 16 rows.  One warp runs
@@ -86,16 +87,20 @@ __global__ void k_diag_inv(DevPlan p, const double* __restrict__ P, double* __re
 // bank conflicts.  P rows are padded to a multiple of 4 entries and R is a
 // multiple of 4, so every 16-byte copy is aligned.
 // Bound: the FP64 rate from R = 32 up (2 R flop per 8-byte entry), below it
-// the stream of P and the gathers of X from L2.  Per apply, against 64 x 64
-// FMA tiles of 64 threads: 147.8 M entries, R = 64 1.01 ms (1.56 before; 0.51
-// at the FP64 rate); 7.5 M entries in 12-row leaves, R = 24 74 us (297);
-// 470 panels all pairs, R = 4 18 us (70).  The items run largest first: that
+// the stream of P and the gathers of X from L2.  At R = 64 the rest is the
+// copies' instructions (with a division, a range search and 64-bit products in
+// each they outnumbered the matrix instructions eight to one), padding to
+// whole 8-row tiles (11 %) and the last wave.  Per apply, against 64 x 64 FMA
+// tiles of 64 threads: 147.8 M entries, R = 64 0.76 ms (1.56 before, 1.01 with
+// the index arithmetic in every copy; 0.51 at the FP64 rate), R = 24 0.34 ms,
+// R = 8 0.24 (0.18 for the stream of P); 7.5 M entries in 12-row leaves, R =
+// 24 74 us (297); 470 panels all pairs, R = 4 18 us (70).  The items run largest first: that
 // alone took the 12-row leaves from 106 to 74 us.
 template <int NT>
 struct NearMma {
     static constexpr int NTW = NT % 3 == 0 ? 3 : NT == 1 ? 1 : 2;  // column tiles per warp
     static constexpr int WN = NT / NTW, WM = 4 / WN;
-    static constexpr int KC = NT <= 3 ? 32 : 16, S = NT == 8 ? 2 : 3;
+    static constexpr int KC = NT == 1 ? 32 : 16, S = NT == 8 ? 2 : 3;
     static constexpr int PP = KC + 4, XP = 8 * NT + 4;
     static constexpr int kMinCtas = NT == 8 ? 4 : 2;
 };
@@ -121,28 +126,41 @@ __global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(D
     if (warp == 0) near_ranges_warp(p, t, lane, s_beg, s_pre);
     __syncthreads();
     const int nst = (Sp + KC - 1) / KC, mt = (m + 7) >> 3;
-    int e = 0;  // near leaf of this thread's next X row (rows only grow)
-    auto issue = [&](int st) {
-        if (st < nst) {
-            const int k0 = st * KC;
-            double* ps = Ps + (st % S) * tile_rows * PP;
-            double* xs = Xs + (st % S) * KC * XP;
-            for (int id = tid; id < m * (KC / 2); id += 128) {
-                const int row = id / (KC / 2), k = 2 * (id % (KC / 2));
-                const bool ok = k0 + k < Sp;
-                cp_async_16(ps + row * PP + k, ok ? Pi + (int64_t)row * Sp + k0 + k : P, ok);
-            }
+    // Copies of one stage: P rows prow, prow + RS, .. from column pk on; X rows
+    // by panel number (rows only grow, so the near leaf they lie in is kept
+    // with its first row's address).
+    constexpr int TP = KC / 2, RS = 128 / TP;
+    const int prow = tid / TP, pk = 2 * (tid % TP);
+    const double* pp = Pi + (int64_t)prow * Sp + pk;
+    const int64_t pstep = (int64_t)RS * Sp;
+    const double* xe = X;
+    int e = -1, xend = 0, ist = 0, islot = 0;
+    auto issue = [&] {
+        if (ist < nst) {
+            const int k0 = ist * KC;
+            double* ps = Ps + islot * tile_rows * PP + prow * PP + pk;
+            double* xs = Xs + islot * KC * XP;
+            const bool pok = k0 + pk < Sp;
 #pragma unroll
-            for (int id = tid; id < KC * 4 * NT; id += 128) {
+            for (int i = 0; i < 64 / RS; ++i)
+                if (prow + RS * i < m) cp_async_16(ps + RS * i * PP, pok ? pp + i * pstep : P, pok);
+            pp += KC;
+#pragma unroll
+            for (int i = 0; i < (KC * NT + 31) / 32; ++i) {
+                const int id = tid + 128 * i;
+                if (KC * NT % 32 != 0 && id >= KC * 4 * NT) break;
                 const int kk = id / (4 * NT), c = 2 * (id % (4 * NT)), k = k0 + kk;
+                if (k < nsrc)
+                    while (k >= xend) {
+                        ++e;
+                        xend = s_pre[e + 1];
+                        xe = X + (s_beg[e] - s_pre[e]) * R + rc;
+                    }
                 const bool ok = k < nsrc && c < cols;
-                int64_t gid = 0;
-                if (k < nsrc) {
-                    while (s_pre[e + 1] <= k) ++e;
-                    gid = s_beg[e] + (k - s_pre[e]);
-                }
-                cp_async_16(xs + kk * XP + c, ok ? X + gid * R + rc + c : X, ok);
+                cp_async_16(xs + kk * XP + c, ok ? xe + (int64_t)k * R + c : X, ok);
             }
+            ++ist;
+            islot = islot + 1 == S ? 0 : islot + 1;
         }
         cp_async_fence();
     };
@@ -153,26 +171,32 @@ __global__ void __launch_bounds__(128, NearMma<NT>::kMinCtas) k_near_apply_mma(D
 #pragma unroll
         for (int j = 0; j < NTW; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-    for (int st = 0; st < S - 1; ++st) issue(st);
-    for (int st = 0; st < nst; ++st) {
+    for (int st = 0; st < S - 1; ++st) issue();
+    for (int st = 0, slot = 0; st < nst; ++st, slot = slot + 1 == S ? 0 : slot + 1) {
         cp_async_wait_for<S - 2>();
         __syncthreads();
-        issue(st + S - 1);
-        const double* ps = Ps + (st % S) * tile_rows * PP + (8 * wm + g) * PP + q;
-        const double* xs = Xs + (st % S) * KC * XP + q * XP + 8 * NTW * wn + g;
+        issue();
+        const double* ps = Ps + slot * tile_rows * PP + (8 * wm + g) * PP + q;
+        const double* xs = Xs + slot * KC * XP + q * XP + 8 * NTW * wn + g;
 #pragma unroll
-        for (int k = 0; k < KC; k += 4) {
-            double b[NTW];
+        for (int h = 0; h < KC; h += 16) {
+            double b[4][NTW];
 #pragma unroll
-            for (int j = 0; j < NTW; ++j) b[j] = xs[k * XP + 8 * j];
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int j = 0; j < NTW; ++j) b[k][j] = xs[(h + 4 * k) * XP + 8 * j];
 #pragma unroll
             for (int i = 0; i < MT; ++i)
                 if (wm + WM * i < mt) {
                     // rows m .. 8 mt - 1 of the last tile hold leftovers of
                     // other stages or items: their outputs are never stored
-                    const double a = ps[8 * WM * i * PP + k];
+                    double a[4];
 #pragma unroll
-                    for (int j = 0; j < NTW; ++j) dmma(acc[i][j], a, b[j]);
+                    for (int k = 0; k < 4; ++k) a[k] = ps[8 * WM * i * PP + h + 4 * k];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int j = 0; j < NTW; ++j) dmma(acc[i][j], a[k], b[k][j]);
                 }
         }
     }
