@@ -92,6 +92,7 @@ struct FacM2L {
     const int32_t* tgt_col = nullptr;   // per pair: its first column within the target
     const int64_t* tgt_col_off = nullptr;  // nbox + 1: summed ranks of the targets before
     const int64_t* tgt_base = nullptr;  // nbox: first T row (each target's columns rounded up to 4)
+    const int32_t* tgt_order = nullptr;  // nbox: each level's targets, most columns first
     T* Tm = nullptr;                    // target-major intermediate (R values per column)
     const double* box_scale = nullptr;  // per box: 1 / half-width of its level
 };

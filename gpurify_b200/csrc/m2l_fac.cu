@@ -15,10 +15,13 @@
 // the CUDA cores with 16-, 32- or 64-column tiles (31,940 box pairs, R = 16:
 // 0.22 ms per FP32 apply, 0.54 with 64 columns).  One FP64 apply (both phases), against the 64-column
 // FMA tiles it replaced:
-//   order 5, R = 64, 62,802 box pairs:  1.05 ms (1.98 before; 0.8 at the FP64 rate)
+//   order 5, R = 64, 62,802 box pairs:  0.96 ms (1.98 before; 0.8 at the FP64 rate)
 //   order 6, R = 24, 96,750 box pairs:  1.38 ms (6.23)
 //   order 5, R = 16, 31,940 box pairs:  0.22 ms (0.95)
 //   order 4, R = 4, 4,528 box pairs:    34 us (135)
+// Both phases start the items with most columns first (the host sorts them):
+// in the order of the boxes the first of these took 1.09 ms, 12 to 14 % of the
+// SM cycles idle behind the last long items.
 #include "dmma.cuh"
 #include "farfield.cuh"
 
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(NS, (FacU64<NT, NS>::kMinCtas))
     k_fac_u64(FacM2L<double> f, int b0, double* __restrict__ L, int R) {
     using C = FacU64<NT, NS>;
     constexpr int KC = C::KC, S = C::kStages, TP = C::TP, UP = C::UP, ns = NS;
-    const int t = b0 + blockIdx.x, rc = blockIdx.y * (8 * NT);
+    const int t = f.tgt_order[b0 + blockIdx.x], rc = blockIdx.y * (8 * NT);
     const int rows = min(8 * NT, R - rc);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
     const int K = (int)(f.tgt_col_off[t + 1] - f.tgt_col_off[t]);
@@ -334,7 +337,7 @@ template <int MW, int RI>
 __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* __restrict__ L, int R) {
     constexpr int V = 4, KC = 32, XP = MW + V, RW = 8 * RI, AP = RW + V, TXN = MW / 8;
     const int ns = f.ns;
-    const int t = b0 + blockIdx.x;
+    const int t = f.tgt_order[b0 + blockIdx.x];
     const int rc = blockIdx.y * RW;
     const int m0 = blockIdx.z * MW;
     const int K = (int)(f.tgt_col_off[t + 1] - f.tgt_col_off[t]);

@@ -20,8 +20,8 @@
 //     MN-major tile, so the gather is a plain copy: no transpose and no
 //     per-slice register work.
 // What bounds it: with 28 rows per leaf (bus) or 55 (window) the gather of X (8 NT bytes
-// a source panel against 4 per row of P) is most of what a CTA reads, from L2
-// at 55 to 60 bytes a clock and SM.  So the copies follow NT (a 12-column apply
+// a source panel against 4 per row of P) is most of what a CTA reads (2.2 GB
+// an apply of the window, 11 TB/s from L2).  So the copies follow NT (a 12-column apply
 // of a 21,195-panel bus: 97 us with 64 columns copied, 68 with 16, and four
 // stages), and four neighbouring threads read 64 contiguous bytes, whole
 // sectors (64-net window, 64 columns: 228 -> 202 us).  One arrival per warp

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <numeric>
 
 #include "adjoint.cuh"
 #include "farfield.cuh"
@@ -488,7 +489,7 @@ struct Operator {
     FacM2L<double> fac64;
     FacM2L<float> fac32;
     DBuf<int64_t> src_col, src_trow, tgt_col_off, tgt_base;
-    DBuf<int32_t> src_slot, tgt_col;
+    DBuf<int32_t> src_slot, tgt_col, tgt_order;
     DBuf<FacItem> fac_items;
     DBuf<double> T64;
     DBuf<float> T32;
@@ -751,8 +752,19 @@ struct Operator {
                 while (p < first[b + 1] && scol[p + 1] - scol[p0] <= cap) ++p;
                 items.push_back({(int32_t)b, (int32_t)p0, (int32_t)p});
             }
+        // Both phases start the work with most columns first: a last wave of
+        // long items would leave SMs idle.
+        std::stable_sort(items.begin(), items.end(), [&](const FacItem& a, const FacItem& b) {
+            return scol[a.p1] - scol[a.p0] > scol[b.p1] - scol[b.p0];
+        });
+        std::vector<int32_t> order(nb);
+        std::iota(order.begin(), order.end(), 0);
+        for (int l = 0; l <= pl.L; ++l)
+            std::stable_sort(order.begin() + pl.lvl_off[l], order.begin() + pl.lvl_off[l + 1],
+                             [&](int32_t a, int32_t b) { return tcol[a + 1] - tcol[a] > tcol[b + 1] - tcol[b]; });
         cudaStream_t s = ctx.stream;
         fac_items.upload(items, s);
+        tgt_order.upload(order, s);
         src_slot.upload(sslot, s);
         src_col.upload(scol, s);
         src_trow.upload(strow, s);
@@ -773,6 +785,7 @@ struct Operator {
             f.tgt_col = tgt_col.p;
             f.tgt_col_off = tgt_col_off.p;
             f.tgt_base = tgt_base.p;
+            f.tgt_order = tgt_order.p;
             f.box_scale = box_scale.p;
         };
         wire(fac64);
