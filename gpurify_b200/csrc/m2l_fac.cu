@@ -12,9 +12,10 @@
 // the plan's upload).
 //
 // FP64 runs on mma.sync (dmma.cuh) with column tiles that follow R, FP32 on
-// the CUDA cores with 16-, 32- or 64-column tiles (31,940 box pairs, R = 16:
-// 0.22 ms per FP32 apply, 0.54 with 64 columns).  One FP64 apply (both phases), against the 64-column
-// FMA tiles it replaced:
+// the CUDA cores with 16-, 32- or 64-column tiles (13,846 box pairs: 96, 137
+// and 216 us per FP32 apply; with operands read one at a time from shared
+// memory 113, 172 and 279).  One FP64 apply (both phases), against the
+// 64-column FMA tiles it replaced:
 //   order 5, R = 64, 62,802 box pairs:  0.96 ms (1.98 before; 0.8 at the FP64 rate)
 //   order 6, R = 24, 96,750 box pairs:  1.38 ms (6.23)
 //   order 5, R = 16, 31,940 box pairs:  0.22 ms (0.95)
@@ -28,6 +29,9 @@
 namespace gpx {
 
 namespace {
+
+// FP32: contraction steps per stage, and stages of phase 1 and phase 2
+constexpr int kFac32Chunk = 32, kV32Stages = 2, kU32Stages = 3;
 
 inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
@@ -237,26 +241,29 @@ __global__ void __launch_bounds__(NS, (FacU64<NT, NS>::kMinCtas))
     }
 }
 
-// Phase 1, FP32: a transposed GEMM per (source item, 8 RI right-hand sides),
-// C[c][r] = sum_l Vt_c[l] E_s[r][l].  E_s^T (B) is staged once per item; the
-// gathered Vt rows (A) of each CT-column sub-block stream through a cp.async
-// double buffer over the ns nodes.  CT threads, 8 x RI outputs per thread
-// (columns ty + (CT/8) i, rows tx + 8 j).
+// Phase 1, FP32: a GEMM per (source item, 8 RI right-hand sides), C[c][r] =
+// sum_l Vt_c[l] E_s[r][l].  E_s is staged once per item; the gathered Vt rows
+// of each CT-column sub-block stream through a cp.async ring over the ns
+// nodes.  CT threads, 8 x RI outputs per thread (columns ty + (CT/8) i, rows
+// tx + 8 j).  Both tiles are contiguous along the contraction, so a thread
+// reads four nodes of a row at once: 10 shared reads for 64 FMAs at RI = 2,
+// where one node at a time took 40 and bound the kernel.  Pitches of 4 more
+// than a multiple of 32 words keep the reads free of bank conflicts.  Nodes are
+// added in ascending order.
 template <int CT, int RI>
 __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* __restrict__ items,
                                                 const float* __restrict__ E, int R) {
-    constexpr int V = 4, KC = 32, PP = KC + V;
-    constexpr int BP = 8 * RI + 1;  // odd pitch: the transposed staging stores hit distinct banks
+    constexpr int V = 4, KC = kFac32Chunk, S = kV32Stages, PP = KC + V;
     constexpr int CS = CT / 8;  // column stride of a thread's tile
     const int ns = f.ns;
     const FacItem it = items[blockIdx.x];
     const int rc = blockIdx.y * (8 * RI);
-    const int rows = min(8 * RI, R - rc);
+    const int rows = min(8 * RI, R - rc), BP = ns + V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float(*As)[CT][PP] = reinterpret_cast<float(*)[CT][PP]>(smem_raw);  // [2][CT][PP]: [c][l]
-    int64_t* col_t = reinterpret_cast<int64_t*>(smem_raw + sizeof(float) * 2 * CT * PP);
+    float(*As)[CT][PP] = reinterpret_cast<float(*)[CT][PP]>(smem_raw);  // [S][CT][PP]: [c][l]
+    int64_t* col_t = reinterpret_cast<int64_t*>(smem_raw + sizeof(float) * S * CT * PP);
     int32_t* col_vt = reinterpret_cast<int32_t*>(col_t + kFacItemCols);
-    float(*Bs)[BP] = reinterpret_cast<float(*)[BP]>(col_vt + kFacItemCols);  // [ns][BP]: [l][r]
+    float* Bs = reinterpret_cast<float*>(col_vt + kFacItemCols);  // [8 RI][BP]: [r][l]
     expand_source(f, it, col_vt, col_t);
     const int ncols = (int)(f.src_col[it.p1] - f.src_col[it.p0]);
     __syncthreads();
@@ -265,23 +272,26 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
     const int nsub = (ncols + CT - 1) / CT;  // CT-column sub-blocks
     const int nsteps = nsub * nch;
     auto issue = [&](int step) {
-        const int sub = step / nch, ch = step % nch;
-        const int nc = min(CT, ncols - CT * sub);
-        const int k0 = ch * KC, buf = step & 1;
+        if (step < nsteps) {
+            const int sub = step / nch, ch = step % nch;
+            const int nc = min(CT, ncols - CT * sub);
+            const int k0 = ch * KC, buf = step % S;
 #pragma unroll
-        for (int q = 0; q < KC / V; ++q) {
-            const int id = tid + CT * q, row = id / (KC / V), kc = (id % (KC / V)) * V;
-            const bool ok = row < nc;
-            cp_async_16(&As[buf][row][kc], ok ? f.Vt + (int64_t)col_vt[CT * sub + row] * ns + k0 + kc : f.Vt, ok);
+            for (int q = 0; q < KC / V; ++q) {
+                const int id = tid + CT * q, row = id / (KC / V), kc = (id % (KC / V)) * V;
+                const bool ok = row < nc;
+                cp_async_16(&As[buf][row][kc], ok ? f.Vt + (int64_t)col_vt[CT * sub + row] * ns + k0 + kc : f.Vt, ok);
+            }
         }
         cp_async_fence();
     };
-    issue(0);
     const float* Es = E + ((int64_t)it.src * R + rc) * ns;
-    for (int e = tid; e < 8 * RI * ns; e += CT) {
-        const int r = e / ns, l = e % ns;
-        Bs[l][r] = r < rows ? Es[(int64_t)r * ns + l] : 0.f;
+    for (int e = tid; e < 8 * RI * (ns / V); e += CT) {
+        const int r = e / (ns / V), l = (e % (ns / V)) * V;
+        cp_async_16(Bs + r * BP + l, r < rows ? Es + (int64_t)r * ns + l : Es, r < rows);
     }
+#pragma unroll
+    for (int s = 0; s < S - 1; ++s) issue(s);
     float acc[8][RI];
     for (int step = 0; step < nsteps; ++step) {
         const int sub = step / nch, ch = step % nch;
@@ -291,26 +301,27 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
 #pragma unroll
                 for (int j = 0; j < RI; ++j) acc[i][j] = 0.f;
         }
+        cp_async_wait_for<S - 2>();
         __syncthreads();
-        if (step + 1 < nsteps) {
-            issue(step + 1);
-            cp_async_wait_for<1>();
-        } else {
-            cp_async_wait_for<0>();
-        }
-        __syncthreads();
-        const int buf = step & 1;
-#pragma unroll 4
-        for (int kk = 0; kk < KC; ++kk) {
-            float a[8], b[RI];
+        issue(step + S - 1);
+        const int buf = step % S;
+#pragma unroll 2
+        for (int kk = 0; kk < KC; kk += V) {
+            float4 b[RI];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = As[buf][ty + CS * i][kk];
+            for (int j = 0; j < RI; ++j)
+                b[j] = *reinterpret_cast<const float4*>(Bs + (tx + 8 * j) * BP + ch * KC + kk);
 #pragma unroll
-            for (int j = 0; j < RI; ++j) b[j] = Bs[ch * KC + kk][tx + 8 * j];
+            for (int i = 0; i < 8; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(&As[buf][ty + CS * i][kk]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < RI; ++j) acc[i][j] += a[i] * b[j];
+                for (int j = 0; j < RI; ++j) {
+                    acc[i][j] += a.x * b[j].x;
+                    acc[i][j] += a.y * b[j].y;
+                    acc[i][j] += a.z * b[j].z;
+                    acc[i][j] += a.w * b[j].w;
+                }
+            }
         }
         if (ch == nch - 1) {
             const int nc = min(CT, ncols - CT * sub);
@@ -329,13 +340,17 @@ __global__ void __launch_bounds__(CT) k_fac_v32(FacM2L<float> f, const FacItem* 
     }
 }
 
-// Phase 2, FP32: CTA per (target box, 8 RI rows r, MW nodes m), MW threads, RI x
-// 8 outputs per thread (rows ty + 8 i, nodes tx + (MW/8) j); the contraction
-// over the target's concatenated ranks streams A = T rows and B = gathered Ut
-// rows through a cp.async double buffer.  L is written, not added to.
+// Phase 2, FP32: CTA per (target box, 8 RI rows r, MW nodes m), a warp per 32
+// nodes and all rows, 2 RI x 4 outputs per thread (rows 16 h + 4 ry + {0..3},
+// nodes 32 warp + 4 nx + {0..3}); the contraction over the target's
+// concatenated ranks streams A = T rows and B = gathered Ut rows through a
+// cp.async ring, both contiguous along a thread's outputs, which it reads 16
+// bytes at a time.  Shared reads bound it at few rows: with warps of 128 nodes x
+// 4 rows five wavefronts fed 16 FMAs at RI = 2, with 32 x 16 two do.  L is
+// written, not added to.
 template <int MW, int RI>
 __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* __restrict__ L, int R) {
-    constexpr int V = 4, KC = 32, XP = MW + V, RW = 8 * RI, AP = RW + V, TXN = MW / 8;
+    constexpr int V = 4, KC = kFac32Chunk, S = kU32Stages, XP = MW + V, RW = 8 * RI, AP = RW + V, RT = RW / 4;
     const int ns = f.ns;
     const int t = f.tgt_order[b0 + blockIdx.x];
     const int rc = blockIdx.y * RW;
@@ -345,68 +360,67 @@ __global__ void __launch_bounds__(MW) k_fac_u32(FacM2L<float> f, int b0, float* 
     const float* A = f.Tm + f.tgt_base[t] * R + rc;  // column-major: A[c][r] at c * R + r
     const int m = min(RW, R - rc);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float(*As)[KC][AP] = reinterpret_cast<float(*)[KC][AP]>(smem_raw);                             // [2][KC][AP]: [c][r]
-    float(*Bs)[KC][XP] = reinterpret_cast<float(*)[KC][XP]>(smem_raw + sizeof(float) * 2 * KC * AP);  // [2][KC][XP]
-    uint16_t* col = reinterpret_cast<uint16_t*>(smem_raw + sizeof(float) * 2 * KC * (AP + XP));
-    const int tid = threadIdx.x, tx = tid % TXN, ty = tid / TXN;
+    float(*As)[KC][AP] = reinterpret_cast<float(*)[KC][AP]>(smem_raw);                             // [S][KC][AP]: [c][r]
+    float(*Bs)[KC][XP] = reinterpret_cast<float(*)[KC][XP]>(smem_raw + sizeof(float) * S * KC * AP);  // [S][KC][XP]
+    uint16_t* col = reinterpret_cast<uint16_t*>(smem_raw + sizeof(float) * S * KC * (AP + XP));
+    const int tid = threadIdx.x, nx = tid & 7, ry = (tid & 31) >> 3, node = 32 * (tid >> 5) + V * nx;
     const int nchunk = (K + KC - 1) / KC;
     auto issue = [&](int cch) {
-        const int k0 = cch * KC, buf = cch & 1;
-        for (int id = tid; id < KC * (RW / V); id += MW) {
-            const int kk = id / (RW / V), rr = (id % (RW / V)) * V;
-            const bool ok = k0 + kk < K && rr < m;
-            cp_async_16(&As[buf][kk][rr], ok ? A + (int64_t)(k0 + kk) * R + rr : f.Tm, ok);
-        }
-        for (int id = tid; id < KC * (MW / V); id += MW) {
-            const int kk = id / (MW / V), cc = (id % (MW / V)) * V;
-            const bool ok = k0 + kk < K && m0 + cc < ns;
-            cp_async_16(&Bs[buf][kk][cc], ok ? f.Ut + (int64_t)col[k0 + kk] * ns + m0 + cc : f.Ut, ok);
+        if (cch < nchunk) {
+            const int k0 = cch * KC, buf = cch % S;
+            for (int id = tid; id < KC * (RW / V); id += MW) {
+                const int kk = id / (RW / V), rr = (id % (RW / V)) * V;
+                const bool ok = k0 + kk < K && rr < m;
+                cp_async_16(&As[buf][kk][rr], ok ? A + (int64_t)(k0 + kk) * R + rr : f.Tm, ok);
+            }
+            for (int id = tid; id < KC * (MW / V); id += MW) {
+                const int kk = id / (MW / V), cc = (id % (MW / V)) * V;
+                const bool ok = k0 + kk < K && m0 + cc < ns;
+                cp_async_16(&Bs[buf][kk][cc], ok ? f.Ut + (int64_t)col[k0 + kk] * ns + m0 + cc : f.Ut, ok);
+            }
         }
         cp_async_fence();
     };
-    float acc[RI][8];
+    float acc[RT][4];
 #pragma unroll
-    for (int i = 0; i < RI; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
     if (K > 0) {
         expand_target(f, t, col);
         __syncthreads();
-        issue(0);
+#pragma unroll
+        for (int s = 0; s < S - 1; ++s) issue(s);
     }
     for (int cch = 0; cch < nchunk; ++cch) {
+        cp_async_wait_for<S - 2>();
         __syncthreads();
-        if (cch + 1 < nchunk) {
-            issue(cch + 1);
-            cp_async_wait_for<1>();
-        } else {
-            cp_async_wait_for<0>();
-        }
-        __syncthreads();
-        const int buf = cch & 1;
+        issue(cch + S - 1);
+        const int buf = cch % S;
 #pragma unroll 4
         for (int kk = 0; kk < KC; ++kk) {
-            float a[RI], b[8];
+            const float4 b = *reinterpret_cast<const float4*>(&Bs[buf][kk][node]);
 #pragma unroll
-            for (int i = 0; i < RI; ++i) a[i] = As[buf][kk][ty + 8 * i];
+            for (int i = 0; i < RT; i += 4) {
+                const float4 a4 = *reinterpret_cast<const float4*>(&As[buf][kk][4 * i + 4 * ry]);
+                const float a[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) b[j] = Bs[buf][kk][tx + TXN * j];
-#pragma unroll
-            for (int i = 0; i < RI; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
+                for (int q = 0; q < 4; ++q) {
+                    acc[i + q][0] += a[q] * b.x;
+                    acc[i + q][1] += a[q] * b.y;
+                    acc[i + q][2] += a[q] * b.z;
+                    acc[i + q][3] += a[q] * b.w;
+                }
+            }
         }
     }
+    if (m0 + node >= ns) return;  // ns is a multiple of 4
 #pragma unroll
-    for (int i = 0; i < RI; ++i) {
-        const int r = ty + 8 * i;
+    for (int i = 0; i < RT; ++i) {
+        const int r = 16 * (i / 4) + 4 * ry + i % 4;
         if (r >= m) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int mm = m0 + tx + TXN * j;
-            if (mm >= ns) continue;
-            L[((int64_t)t * R + rc + r) * ns + mm] = sc * acc[i][j];
-        }
+        *reinterpret_cast<float4*>(L + ((int64_t)t * R + rc + r) * ns + m0 + node) =
+            make_float4(sc * acc[i][0], sc * acc[i][1], sc * acc[i][2], sc * acc[i][3]);
     }
 }
 
@@ -438,9 +452,9 @@ void run_fac64(Ctx& c, const FacM2L<double>& f, int b0, int nb, double* L, const
 
 template <int RI>
 void run_fac32(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const float* E, int R) {
-    constexpr int V = 4, KC = 32, CT = 128, RW = 8 * RI;
+    constexpr int V = 4, KC = kFac32Chunk, CT = 128, RW = 8 * RI;
     if (f.nitems > 0) {
-        const int smem = (int)(sizeof(float) * (2 * CT * (KC + V) + f.ns * (RW + 1)) + 12 * kFacItemCols);
+        const int smem = (int)(sizeof(float) * (kV32Stages * CT * (KC + V) + RW * (f.ns + V)) + 12 * kFacItemCols);
         set_smem_once(k_fac_v32<CT, RI>, smem);
         k_fac_v32<CT, RI><<<dim3(f.nitems, cdiv(R, RW)), CT, smem, c.stream>>>(f, f.items, E, R);
         GPX_LAUNCH_CHECK();
@@ -448,12 +462,12 @@ void run_fac32(Ctx& c, const FacM2L<float>& f, int b0, int nb, float* L, const f
     const int cols = 2 * ((f.max_cols + 7) & ~7);
     if (f.ns >= 128) {
         constexpr int MW = 128;
-        const int smem = (int)(sizeof(float) * 2 * KC * (RW + V + MW + V)) + cols;
+        const int smem = (int)(sizeof(float) * kU32Stages * KC * (RW + V + MW + V)) + cols;
         set_smem_once(k_fac_u32<MW, RI>, smem);
         k_fac_u32<MW, RI><<<dim3(nb, cdiv(R, RW), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
     } else {
         constexpr int MW = 64;
-        const int smem = (int)(sizeof(float) * 2 * KC * (RW + V + MW + V)) + cols;
+        const int smem = (int)(sizeof(float) * kU32Stages * KC * (RW + V + MW + V)) + cols;
         set_smem_once(k_fac_u32<MW, RI>, smem);
         k_fac_u32<MW, RI><<<dim3(nb, cdiv(R, RW), cdiv(f.ns, MW)), MW, smem, c.stream>>>(f, b0, L, R);
     }
