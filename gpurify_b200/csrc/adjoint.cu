@@ -92,10 +92,11 @@ __global__ void k_panel_dprops(DevPlan p, const double* __restrict__ V, double* 
 // without evaluating the integral, and the others carry derivatives of the point
 // alone.  Bound: the FP64 pipe.  Bus of 21,038 panels, 51 M entries, 4
 // parameters (width, spacing, thickness, height): 56 ms with every moving pair
-// on dual numbers throughout, 32 now.
+// on dual numbers throughout, 32 with constant panels, 18 with the panels in
+// shared memory (255 registers before, one CTA an SM) and the items split.
 constexpr int kDThreads = 256;
 constexpr int kDTile = 64;
-__global__ void __launch_bounds__(kDThreads) k_near_assemble_dual(DevPlan p, const double* __restrict__ V,
+__global__ void __launch_bounds__(kDThreads, 3) k_near_assemble_dual(DevPlan p, const double* __restrict__ V,
                                                                   const double* __restrict__ dcent,
                                                                   double* __restrict__ dP, double coef) {
     const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
@@ -106,51 +107,57 @@ __global__ void __launch_bounds__(kDThreads) k_near_assemble_dual(DevPlan p, con
     const int64_t off = p.nval_off[t];
     __shared__ int64_t s_beg[28];
     __shared__ int32_t s_pre[29];
-    __shared__ int64_t s_gid[kDTile];
+    // A panel of constants (43 doubles) or of dual numbers (86) and the velocity
+    // of a rigid one; the odd pitch puts consecutive panels in distinct banks.
+    __shared__ double s_panel[kDTile][87];
+    __shared__ int32_t s_rigid[kDTile];
     if (threadIdx.x < 32) near_ranges_warp(p, t, threadIdx.x, s_beg, s_pre);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kDThreads / 32;
+    const int j = threadIdx.x % kDTile, row0 = r0 + threadIdx.x / kDTile;
     for (int base = kDTile * blockIdx.y; base < S; base += kDTile * gridDim.y) {
         const int cnt = min(kDTile, S - base);
         if (threadIdx.x < cnt) {
             int s = base + threadIdx.x, e = 0;
             while (s_pre[e + 1] <= s) ++e;
-            s_gid[threadIdx.x] = s_beg[e] + (s - s_pre[e]);
-        }
-        __syncthreads();
-        for (int j = lane; j < cnt; j += 32) {
-            const int64_t g = s_gid[j];
+            const int64_t g = s_beg[e] + (s - s_pre[e]);
             const double* vv = V + 12 * g;
+            double* sp = s_panel[threadIdx.x];
             bool rigid = true;
             for (int k = 3; k < 12; ++k) rigid &= vv[k] == vv[k % 3];
-            const double ux = vv[0], uy = vv[1], uz = vv[2];
-            auto write = [&](int row, double val) { dP[off + (int64_t)row * Sp + base + j] = val; };
+            s_rigid[threadIdx.x] = rigid;
             if (rigid) {
-                // only the point's motion relative to the panel counts
-                SrcPanel sp;
-                prep_source(p.verts + 12 * g, sp);
-                for (int row = r0 + warp; row < m; row += nw) {
-                    const double* c = p.cent + 3 * (tb + row);
-                    const double* dc = dcent + 3 * (tb + row);
+                prep_source(p.verts + 12 * g, *reinterpret_cast<SrcPanel*>(sp));
+                for (int k = 0; k < 3; ++k) sp[43 + k] = vv[k];
+            } else {
+                Dual gv[12];
+                for (int k = 0; k < 12; ++k) gv[k] = Dual(p.verts[12 * g + k], vv[k]);
+                prep_source_t<Dual>(gv, *reinterpret_cast<SrcPanelT<Dual>*>(sp));
+            }
+        }
+        __syncthreads();
+        if (j < cnt) {
+            const double* sp = s_panel[j];
+            const bool rigid = s_rigid[j];
+            for (int row = row0; row < m; row += kDThreads / kDTile) {
+                const double* c = p.cent + 3 * (tb + row);
+                const double* dc = dcent + 3 * (tb + row);
+                double val = 0.0;
+                if (rigid) {
+                    // only the point's motion relative to the panel counts
+                    const double ux = sp[43], uy = sp[44], uz = sp[45];
                     const double wx = dc[0] - ux, wy = dc[1] - uy, wz = dc[2] - uz;
                     // velocities of a common translation agree to rounding
                     // (the centroid's is an area-weighted mean)
                     const double same = 1e-14 * (fabs(ux) + fabs(uy) + fabs(uz));
-                    double val = 0.0;
                     if (fabs(wx) > same || fabs(wy) > same || fabs(wz) > same)
-                        val = coef * wilton_t<Dual, double>(sp, Dual(c[0], wx), Dual(c[1], wy), Dual(c[2], wz)).d;
-                    write(row, val);
+                        val = coef * wilton_t<Dual, double>(*reinterpret_cast<const SrcPanel*>(sp), Dual(c[0], wx),
+                                                            Dual(c[1], wy), Dual(c[2], wz)).d;
+                } else {
+                    val = coef * wilton_t<Dual>(*reinterpret_cast<const SrcPanelT<Dual>*>(sp), Dual(c[0], dc[0]),
+                                                Dual(c[1], dc[1]), Dual(c[2], dc[2])).d;
                 }
-            } else {
-                Dual gv[12];
-                for (int k = 0; k < 12; ++k) gv[k] = Dual(p.verts[12 * g + k], vv[k]);
-                SrcPanelT<Dual> sp;
-                prep_source_t<Dual>(gv, sp);
-                for (int row = r0 + warp; row < m; row += nw) {
-                    const double* c = p.cent + 3 * (tb + row);
-                    const double* dc = dcent + 3 * (tb + row);
-                    write(row, coef * wilton_t<Dual>(sp, Dual(c[0], dc[0]), Dual(c[1], dc[1]), Dual(c[2], dc[2])).d);
-                }
+                dP[off + (int64_t)row * Sp + base + j] = val;
+                asm volatile("" ::: "memory");  // the panel is read again per row, not kept in registers
             }
         }
         __syncthreads();

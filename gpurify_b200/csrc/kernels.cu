@@ -22,11 +22,14 @@ constexpr int kAsmThreads = 256;
 constexpr int kAsmTile = 64;
 
 // One CTA per work item (target leaf, <= 64 rows) and every gridDim.y-th tile
-// of 64 sources: rows of the leaf's P block m_t x S_t, row-major.  Bound: the
-// FP64 pipe (about 1,900 multiply-add slots per entry: 4 edges of 2 square
-// roots, log1p, 2 arc tangents and their divisions), so few items are split
-// over the sources until the chip is full (assembly_split).
-__global__ void __launch_bounds__(kAsmThreads, 2) k_near_assemble(DevPlan p, double* __restrict__ P, double coef) {
+// of 64 sources: rows of the leaf's P block m_t x S_t, row-major; a thread has
+// one source of the tile and every fourth row.  The tile's panels are prepared
+// once, in shared memory, and read from there for each row: with a panel in a
+// thread's registers (128) two CTAs shared an SM, now three do.
+// Bound: the FP64 pipe (about 1,900 multiply-add slots per entry: 4 edges of 2
+// square roots, log1p, 2 arc tangents and their divisions), at about half its
+// rate, since each entry is one chain of them.  147.8 M entries 12.9 -> 9.8 ms.
+__global__ void __launch_bounds__(kAsmThreads, 3) k_near_assemble(DevPlan p, double* __restrict__ P, double coef) {
     const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int64_t tb = p.leaf_begin[t];
     const int m = min((int)(p.leaf_begin[t + 1] - tb), r0 + 64);
@@ -35,26 +38,24 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_near_assemble(DevPlan p, dou
     const int64_t off = p.nval_off[t];
     __shared__ int64_t s_beg[28];
     __shared__ int32_t s_pre[29];
-    __shared__ int64_t s_gid[kAsmTile];
+    __shared__ SrcPanel s_panel[kAsmTile];  // 43 doubles each: lanes on consecutive panels hit distinct banks
     if (threadIdx.x < 32) near_ranges_warp(p, t, threadIdx.x, s_beg, s_pre);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kAsmThreads / 32;
+    const int j = threadIdx.x % kAsmTile, row0 = r0 + threadIdx.x / kAsmTile;
     for (int base = kAsmTile * blockIdx.y; base < S; base += kAsmTile * gridDim.y) {
         const int cnt = min(kAsmTile, S - base);
         if (threadIdx.x < cnt) {
             int s = base + threadIdx.x, e = 0;
             while (s_pre[e + 1] <= s) ++e;
-            s_gid[threadIdx.x] = s_beg[e] + (s - s_pre[e]);
+            prep_source(p.verts + 12 * (s_beg[e] + (s - s_pre[e])), s_panel[threadIdx.x]);
         }
         __syncthreads();
-        for (int j = lane; j < cnt; j += 32) {
-            SrcPanel sp;
-            prep_source(p.verts + 12 * s_gid[j], sp);
-            for (int row = r0 + warp; row < m; row += nw) {
+        if (j < cnt)
+            for (int row = row0; row < m; row += kAsmThreads / kAsmTile) {
                 const double* c = p.cent + 3 * (tb + row);
-                P[off + (int64_t)row * Sp + base + j] = coef * wilton(sp, c[0], c[1], c[2]);
+                P[off + (int64_t)row * Sp + base + j] = coef * wilton(s_panel[j], c[0], c[1], c[2]);
+                asm volatile("" ::: "memory");  // the panel is read again per row, not kept in 86 registers
             }
-        }
         __syncthreads();
     }
 }

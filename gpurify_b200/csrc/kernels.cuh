@@ -1,5 +1,7 @@
 // Device-side view of a plan and the launch wrappers of the FP64 kernels.
 #pragma once
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -69,10 +71,13 @@ __device__ __forceinline__ void near_ranges_warp(const DevPlan& p, int t, int la
 }
 
 // Blocks over the sources of each near item of the assembly and its derivative:
-// enough for about eight CTAs an SM in all (two are resident), at most 16.
-// 470 panels (8 items): assembly 0.69 ms with one block per item, 0.11 with 16;
-// 466 items 1.04 ms with one, 0.59 with two; above 592 items one block each.
-inline int assembly_split(int nitems) { return nitems > 592 ? 1 : nitems < 74 ? 16 : 1184 / nitems; }
+// about 16,000 in all, at most 64 per item (of a tile of 64 sources each where
+// that is fewer).  An item of 64 rows can hold most of what an SM should do in
+// all, so it is cut until the pieces even out: 970 items (21,195-panel bus, 51 M
+// entries, the assembly and four derivatives) 39.5 ms with one block per item,
+// 26.6 with 2,400 blocks, 24.7 with 4,800, 22.5 with 19,200; 2,091 items 10.1 ms
+// and 9.8; 8 items (470 panels) 0.69 ms and 0.1.
+inline int assembly_split(int nitems) { return std::clamp(16384 / nitems, 1, 64); }
 // Wilton near-field block assembly: P (nnz doubles).
 void launch_near_assemble(Ctx& c, const DevPlan& p, int64_t nnz, double* P, double coef);
 // inv_diag[i] = 1 / P_ii (|P_ii| > 1e-30 else 1), the reference's DiagJacobi.
