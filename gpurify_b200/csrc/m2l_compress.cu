@@ -14,13 +14,21 @@
 // both operands are split into TF32 hi and lo parts and D = A_hi B_hi +
 // A_hi B_lo + A_lo B_hi (about 2^-21): B (the basis, K-major, one row per
 // output column) is split once per process; A (the expansion rows) is split
-// in shared memory once a slice has landed.
-// One CTA per (128 rows, 64 output columns): D = 128 x 64 FP32 in TMEM.  The
-// contraction runs in slices of 32 through a 2-stage ring: all 128 threads
-// copy a slice with cp.async, split their A chunks, and one thread issues the
-// slice's MMAs and commits them to the stage's mbarrier, which the copies of
-// the slice two ahead wait on (bounded).  The epilogue stores each row's 64
-// FP32 values (rows past nrows are neither loaded nor stored).
+// on the way to shared memory.
+// One CTA per (64 rows, 64 output columns): D = 64 of the 128 rows of an
+// accumulator x 64 FP32 in TMEM (the MMA reads 128 A rows from a tile's start,
+// the other 64 from the tile behind it, into rows nobody reads).  The
+// contraction runs in slices of 32 through a 2-stage ring: all 128 threads copy
+// the slice's B rows with cp.async and its A rows through registers, read a
+// slice ahead, and one thread issues the slice's MMAs and commits them to the
+// stage's mbarrier, which the copies of the slice two ahead wait on (bounded).
+// The epilogue stores D through shared memory, whole rows of 64 at a time (rows
+// past nrows are neither loaded nor stored).
+// What bounds it: two to seven short slices per CTA, a chain of latencies, so
+// what counts is CTAs per SM (three, of 64 KB) and an even last wave.  115,200
+// rows (64-net window, 64 columns): compress 38 us and decompress 42, against 47
+// and 53 with 128 rows per CTA in two stages of 48 KB (900 CTAs for 296
+// places), split in place between two barriers and stored by one thread per row.
 #include "farfield.cuh"
 
 namespace gpx {
@@ -28,10 +36,12 @@ namespace gpx {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr uint32_t kATile = 128 * 128;                  // 128 rows x 32 FP32 (128 B)
+constexpr int kRows = 64;                               // rows per CTA
+constexpr uint32_t kATile = kRows * 128;                // rows x 32 FP32 (128 B)
 constexpr uint32_t kBTile = 64 * 128;                   // 64 rows x 32 FP32
-constexpr uint32_t kStage = 2 * kATile + 2 * kBTile;    // A_hi, A_lo, B_hi, B_lo: 48 KB
-constexpr uint32_t kSmemBytes = 2 * kStage + 1024 + 64 + 4096;
+constexpr uint32_t kStage = 2 * kATile + 2 * kBTile;    // A_hi, A_lo, B_hi, B_lo: 32 KB
+constexpr uint32_t kSmemBytes = 2 * kStage + 1024 + 64;
+constexpr int kPitch = 68;                              // floats per row of the staged result
 constexpr uint32_t kTmemCols = 64;
 constexpr int kWaitLimit = 1 << 22;
 // Instruction descriptor: D F32, A/B TF32, both K-major, N = 64, M = 128.
@@ -104,9 +114,9 @@ __global__ void __launch_bounds__(kThreads) k_rows_tc(const float* __restrict__ 
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
     __shared__ int s_bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t r0 = (int64_t)blockIdx.x * 128;
+    const int64_t r0 = (int64_t)blockIdx.x * kRows;
     const int col0 = blockIdx.y * 64;
-    const int cnt = (int)min((int64_t)128, nrows - r0);
+    const int cnt = (int)min((int64_t)kRows, nrows - r0);
     if (tid == 0) {
         for (int k = 0; k < 2; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[k])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -121,57 +131,63 @@ __global__ void __launch_bounds__(kThreads) k_rows_tc(const float* __restrict__ 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
-    // copies of slice q into stage q % 2: A rows [r0, r0 + cnt) (rows past
-    // cnt are not loaded: their D rows are never stored), B rows col0 .. +63
+    // B rows col0 .. +63 of slice q into stage q % 2
     auto issue = [&](int q) {
-        const uint32_t a = base + (uint32_t)(q & 1) * kStage;
-        for (int e = tid; e < 128 * 8; e += kThreads) {
-            const int row = e >> 3, c = e & 7;
-            if (row < cnt) cp16(a + swz(row, c), In + (r0 + row) * (int64_t)ldi + 32 * q + 4 * c, true);
-        }
-        for (int e = tid; e < 64 * 8; e += kThreads) {
-            const int row = e >> 3, c = e & 7;
+        const uint32_t b = base + (uint32_t)(q & 1) * kStage + 2 * kATile;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 3) + 16 * i, c = tid & 7;
             const int64_t off = (int64_t)(col0 + row) * KD + 32 * q + 4 * c;
-            cp16(a + 2 * kATile + swz(row, c), Bhi + off, true);
-            cp16(a + 2 * kATile + kBTile + swz(row, c), Blo + off, true);
+            cp16(b + swz(row, c), Bhi + off, true);
+            cp16(b + kBTile + swz(row, c), Blo + off, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // A rows [r0, r0 + cnt) of slice q, into registers while slice q - 1 is
+    // multiplied
+    float4 ar[4];
+    auto fetch = [&](int q) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 3) + 16 * i;
+            ar[i] = row < cnt ? *reinterpret_cast<const float4*>(In + (r0 + row) * (int64_t)ldi + 32 * q + 4 * (tid & 7))
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     };
     bool bad = false;
     int committed = 0;  // slices whose MMAs thread 0 committed (uniform across the CTA)
     issue(0);
+    fetch(0);
     for (int q = 0; q < nsl; ++q) {
         const int st = q & 1;
+        // A_hi and A_lo of this slice; the stage's last MMAs were waited for before its B rows were requested
+        {
+            uint8_t* at = sbase + (size_t)st * kStage;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t o = swz((uint32_t)((tid >> 3) + 16 * i), (uint32_t)(tid & 7));
+                const float4 v = ar[i];
+                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+                *reinterpret_cast<float4*>(at + kATile + o) =
+                    make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z), to_tf32(v.w - h.w));
+                *reinterpret_cast<float4*>(at + o) = h;
+            }
+        }
         if (q + 1 < nsl) {
             // stage (q+1)&1 last held slice q-1: its MMAs must be done
             if (q >= 1 && !mbar_wait(smem_u32(&bars[(q + 1) & 1]), (uint32_t)(((q - 1) >> 1) & 1))) bad = true;
-            if (__syncthreads_or(bad)) {
-                bad = true;
-                break;
-            }
-            issue(q + 1);
+            if (!bad) issue(q + 1);
+            fetch(q + 1);
+        }
+        if (q + 1 < nsl && !bad)
             asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
+        else
             asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        // split the A tile of this slice: A_hi in place, A_lo beside it
-        {
-            uint8_t* at = sbase + (size_t)st * kStage;
-            for (int e = tid; e < 128 * 8; e += kThreads) {
-                const int row = e >> 3;
-                if (row >= cnt) continue;
-                const uint32_t o = swz((uint32_t)row, (uint32_t)(e & 7));
-                float4* hp = reinterpret_cast<float4*>(at + o);
-                float4* lp = reinterpret_cast<float4*>(at + kATile + o);
-                const float4 v = *hp;
-                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-                *lp = make_float4(to_tf32(v.x - h.x), to_tf32(v.y - h.y), to_tf32(v.z - h.z), to_tf32(v.w - h.w));
-                *hp = h;
-            }
-        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
+        if (__syncthreads_or(bad)) {
+            bad = true;
+            break;
+        }
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t ah = base + (uint32_t)st * kStage, al = ah + kATile;
@@ -209,22 +225,27 @@ __global__ void __launch_bounds__(kThreads) k_rows_tc(const float* __restrict__ 
     }
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!bad) {
-        const int row = warp * 32 + lane;
-        float* o = row < cnt ? Out + (r0 + row) * (int64_t)ldo + col0 : nullptr;
+        float* d = reinterpret_cast<float*>(sbase);  // the stages are idle
+        if (warp * 32 < cnt) {
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (o) {
+            for (int cb = 0; cb < 4; ++cb) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float4* o = reinterpret_cast<float4*>(d + (warp * 32 + lane) * kPitch + cb * 16);
 #pragma unroll
-                for (int k = 0; k < 16; k += 4)
-                    if (col0 + cb * 16 + k < ncols)
-                        *reinterpret_cast<float4*>(o + cb * 16 + k) =
-                        make_float4(__uint_as_float(v[k]), __uint_as_float(v[k + 1]), __uint_as_float(v[k + 2]),
-                                    __uint_as_float(v[k + 3]));
+                for (int k = 0; k < 4; ++k)
+                    o[k] = make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
+                                       __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3]));
             }
         }
+        __syncthreads();
+        const int col = 4 * (tid & 15);
+        if (col0 + col < ncols)
+#pragma unroll 4
+            for (int row = tid >> 4; row < cnt; row += kThreads / 16)
+                *reinterpret_cast<float4*>(Out + (r0 + row) * (int64_t)ldo + col0 + col) =
+                    *reinterpret_cast<const float4*>(d + row * kPitch + col);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -239,7 +260,7 @@ void launch_rows_tc(Ctx& c, const float* In, int ldi, const float* Bhi, const fl
     if (ncols % 4 != 0 || ldi % 4 != 0 || ldo % 4 != 0 || ldo < ncols)
         throw Error(GPX_ERR_INTERNAL, "tensor-core row GEMM needs 16-byte rows");
     set_smem_once(k_rows_tc<KD>, (int)kSmemBytes);
-    const dim3 grid((unsigned)((nrows + 127) / 128), (unsigned)((ncols + 63) / 64));
+    const dim3 grid((unsigned)((nrows + kRows - 1) / kRows), (unsigned)((ncols + 63) / 64));
     k_rows_tc<KD><<<grid, kThreads, kSmemBytes, c.stream>>>(In, ldi, Bhi, Blo, ncols, Out, ldo, nrows, err);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
