@@ -278,16 +278,48 @@ __global__ void k_givens_loop(GmresDev g, cudaGraphConditionalHandle h, int32_t*
 }
 
 // Back substitution H y = g per column (krylov.rs:144-152); y[i][r].
-__global__ void k_trisolve(GmresDev g) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= g.R) return;
+// One block per column: its threads bring rows of H to shared memory, as many
+// as fit, and one of them runs the chain of multiply-adds, which is all that
+// is serial, in the order of the rows' columns.  A thread per column with
+// everything in global memory waited for each entry: 58 columns of H 212 us.
+// Columns past kTriCols (longer than a restart) are read from global memory.
+constexpr int kTriThreads = 128, kTriBuf = 4096, kTriCols = 1024;
+__global__ void __launch_bounds__(kTriThreads) k_trisolve(GmresDev g) {
+    __shared__ double s_h[kTriBuf], s_y[kTriCols];
+    const int r = blockIdx.x, tid = threadIdx.x;
     const int m = g.m, R = g.R, ku = g.done[r] ? 0 : g.kused[r];
-    for (int i = 0; i < m; ++i) g.y[i * R + r] = 0.0;
-    for (int i = ku - 1; i >= 0; --i) {
-        double sum = g.g[i * R + r];
-        for (int j = i + 1; j < ku; ++j) sum -= g.H[((int64_t)i * m + j) * R + r] * g.y[j * R + r];
-        g.y[i * R + r] = sum / g.H[((int64_t)i * m + i) * R + r];
+    for (int i = tid; i < m; i += kTriThreads)
+        if (i >= ku || ku > kTriCols) g.y[i * R + r] = 0.0;
+    if (ku > kTriCols) {
+        __syncthreads();
+        if (tid == 0)
+            for (int i = ku - 1; i >= 0; --i) {
+                double sum = g.g[i * R + r];
+                for (int j = i + 1; j < ku; ++j) sum -= g.H[((int64_t)i * m + j) * R + r] * g.y[j * R + r];
+                g.y[i * R + r] = sum / g.H[((int64_t)i * m + i) * R + r];
+            }
+        return;
     }
+    for (int i1 = ku; i1 > 0;) {
+        const int i0 = max(0, i1 - kTriBuf / ku), n = (i1 - i0) * ku;
+        for (int e = tid; e < n; e += kTriThreads) {
+            const int i = i0 + e / ku, j = e % ku;
+            if (j >= i) s_h[e] = g.H[((int64_t)i * m + j) * R + r];
+        }
+        for (int i = i0 + tid; i < i1; i += kTriThreads) s_y[i] = g.g[i * R + r];
+        __syncthreads();
+        if (tid == 0)
+            for (int i = i1 - 1; i >= i0; --i) {
+                const double* h = s_h + (i - i0) * ku;
+                double sum = s_y[i];
+#pragma unroll 8
+                for (int j = i + 1; j < ku; ++j) sum -= h[j] * s_y[j];
+                s_y[i] = sum / h[i];
+            }
+        __syncthreads();
+        i1 = i0;
+    }
+    for (int i = tid; i < ku; i += kTriThreads) g.y[i * R + r] = s_y[i];
 }
 
 // Start of a cycle: beta = ||res||, converged-at-start test, V_0 = res/beta,
@@ -510,7 +542,7 @@ void launch_givens_loop(Ctx& c, const GmresDev& g, cudaGraphConditionalHandle h,
 
 void launch_trisolve(Ctx& c, const GmresDev& g) {
     KTimer t(c, K_SMALL);
-    k_trisolve<<<blocks_for(g.R, 64), 64, 0, c.stream>>>(g);
+    k_trisolve<<<g.R, kTriThreads, 0, c.stream>>>(g);
     GPX_LAUNCH_CHECK();
     c.launches += 1;
 }

@@ -923,22 +923,76 @@ struct Operator {
     }
 };
 
+// part[y][i][r] = sum of X[n][r] area[n] over the panels n of conductor i in
+// slice y of the rows.  A block has to walk its rows in order, each a wait for
+// its conductor and then for the row, so eight rows are read ahead and the rows
+// are cut into slices: 73,011 rows of 64 columns, 65 conductors, one slice per
+// conductor 1.58 ms, now 0.34; 1,759 rows of 12 columns 14.5 us, now 8.
 __global__ void k_accum_c(const int32_t* __restrict__ cond, const double* __restrict__ area,
-                          const double* __restrict__ X, int64_t N, int R, double* __restrict__ C) {
+                          const double* __restrict__ X, int64_t N, int R, double* __restrict__ part) {
+    constexpr int kAhead = 8;
     const int i = blockIdx.x;
     const int nsub = 256 / R;
     const int r = threadIdx.x % R, sub = threadIdx.x / R;
+    const int64_t per = (N + gridDim.y - 1) / gridDim.y, n1 = min(N, (blockIdx.y + 1) * per);
     double acc = 0.0;
     if (sub < nsub)
-        for (int64_t n = sub; n < N; n += nsub)
-            if (cond[n] == i) acc += X[n * R + r] * area[n];
+        for (int64_t n0 = blockIdx.y * per + sub; n0 < n1; n0 += kAhead * nsub) {
+            bool mine[kAhead];
+            double x[kAhead], a[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int64_t n = n0 + u * nsub;
+                mine[u] = n < n1 && cond[n] == i;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int64_t n = n0 + u * nsub;
+                x[u] = mine[u] ? X[n * R + r] : 0.0;
+                a[u] = mine[u] ? area[n] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (mine[u]) acc += x[u] * a[u];
+        }
     __shared__ double red[256];
     red[threadIdx.x] = acc;
     __syncthreads();
     if (sub == 0) {
         double s = red[r];
         for (int k = 1; k < nsub; ++k) s += red[k * R + r];
-        C[(int64_t)i * R + r] = s;
+        part[((int64_t)blockIdx.y * gridDim.x + i) * R + r] = s;
+    }
+}
+
+// C[v] = sum over the slices of part[y][v]
+__global__ void k_accum_slices(const double* __restrict__ part, int slices, int nv, double* __restrict__ C) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nv) return;
+    double s = part[v];
+#pragma unroll 8
+    for (int y = 1; y < slices; ++y) s += part[(int64_t)y * nv + v];
+    C[v] = s;
+}
+
+// C (ncond x R) of the densities X; C has room for accum_slices more of it, the
+// partial sums.  At most 64 slices of 256 rows or more, and no more blocks
+// than 16,384: many conductors fill the chip by themselves.
+int accum_slices(int64_t N, int ncond) {
+    return (int)std::clamp<int64_t>(std::min<int64_t>(N / 256, 16384 / ncond), 1, 64);
+}
+void launch_accum_c(Ctx& c, const int32_t* cond, const double* area, const double* X, int64_t N, int R, int ncond,
+                    double* C) {
+    KTimer kt(c, K_VEC, (8.0 * R + 12.0) * (double)N, 2.0 * (double)N * R);
+    const int slices = accum_slices(N, ncond), nv = ncond * R;
+    double* part = slices > 1 ? C + nv : C;
+    k_accum_c<<<dim3(ncond, slices), 256, 0, c.stream>>>(cond, area, X, N, R, part);
+    GPX_LAUNCH_CHECK();
+    c.launches += 1;
+    if (slices > 1) {
+        k_accum_slices<<<(nv + 127) / 128, 128, 0, c.stream>>>(part, slices, nv, C);
+        GPX_LAUNCH_CHECK();
+        c.launches += 1;
     }
 }
 
@@ -1537,13 +1591,8 @@ void cap_solve(Ctx& ctx, int64_t n, const double* verts, const int32_t* cond, in
         st.converged = st.converged && sc.converged;
         outer = std::max(outer, oc);
         DBuf<double> dC;
-        dC.alloc((size_t)ncond * R, ctx.stream);
-        {
-            KTimer kt(ctx, K_VEC, (8.0 * R + 12.0) * (double)n, 2.0 * (double)n * R);
-            k_accum_c<<<ncond, 256, 0, ctx.stream>>>(pr.dp.cond.p, d_weight, X.p, n, R, dC.p);
-            GPX_LAUNCH_CHECK();
-            ctx.launches += 1;
-        }
+        dC.alloc((size_t)(1 + accum_slices(n, ncond)) * ncond * R, ctx.stream);
+        launch_accum_c(ctx, pr.dp.cond.p, d_weight, X.p, n, R, ncond, dC.p);
         std::vector<double> part((size_t)ncond * R);
         dC.download(part.data(), part.size());
         GPX_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -1693,7 +1742,7 @@ void cap_sensitivity(Ctx& ctx, int64_t n, const double* verts, const int32_t* co
     {
         DBuf<int32_t> d_rhs;
         DBuf<double> dC;
-        dC.alloc((size_t)ncond * R, s);
+        dC.alloc((size_t)(1 + accum_slices(n, ncond)) * ncond * R, s);
         std::vector<double> part((size_t)ncond * R);
         for (int c0 = 0; c0 < Rn; c0 += R) {
             const int nc = std::min(R, Rn - c0);
@@ -1709,12 +1758,7 @@ void cap_sensitivity(Ctx& ctx, int64_t n, const double* verts, const int32_t* co
                                                      std::to_string(st.max_resid));
             its = std::max(its, st.iterations);
             outer = std::max(outer, oc);
-            {
-                KTimer kt(ctx, K_VEC, (8.0 * R + 12.0) * (double)n, 2.0 * (double)n * R);
-                k_accum_c<<<ncond, 256, 0, s>>>(pr.dp.cond.p, pr.dp.area.p, Xs.back().p, n, R, dC.p);
-                GPX_LAUNCH_CHECK();
-                ctx.launches += 1;
-            }
+            launch_accum_c(ctx, pr.dp.cond.p, pr.dp.area.p, Xs.back().p, n, R, ncond, dC.p);
             dC.download(part.data(), part.size());
             GPX_CUDA(cudaStreamSynchronize(s));
             for (int i = 0; i < ncond; ++i)

@@ -82,3 +82,22 @@ def test_mixed_near_apply_at_column_tile_edges(ctx, near, cols):
     wide, _ = ctx.operator_apply(p["verts"], sig, **kw)
     few, _ = ctx.operator_apply(p["verts"], np.ascontiguousarray(sig[:, :cols]), **kw)
     assert np.isfinite(few).all() and np.array_equal(few, wide[:, :cols])
+
+
+@pytest.mark.parametrize("n", [255, 512, 513, 770])
+def test_capacitance_sums_over_row_slices(ctx, orc, n):
+    """The capacitance sums run over slices of 256 rows or more: one slice up to
+    511 panels, then two and three, the last one ragged, with a conductor whose
+    panels all lie in one slice, against the oracle's dense solve (1e-9, the bar
+    of the parity tests at this solver tolerance)."""
+    lay = layouts.two_wires(length_nm=6000)
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, mesh_max_edge_m=0.15e-6,
+                             max_panels=-1)
+    verts = np.ascontiguousarray(p["verts"][:n])
+    assert len(verts) == n
+    cond = (np.arange(n) % 2).astype(np.int32)
+    cond[-5:] = 2
+    C, rep = ctx.cap_solve(verts, cond, 3, tol=1e-12, dense_below=2**31 - 1)  # every pair near: the oracle's matrix
+    assert rep["dense"] == 1
+    ref = orc.cap_dense(verts, cond, 3)
+    assert np.abs(C - ref).max() / np.abs(ref).max() < 1e-9
