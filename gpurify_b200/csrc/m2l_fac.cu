@@ -159,7 +159,8 @@ struct FacU64 {
     static constexpr int TP = 8 * NT + 4, UP = NS + 4;
     static constexpr int kSmem = (int)sizeof(double) * kStages * KC * (TP + UP);  // + the column list
     // 64-column tiles would take 183 registers and leave two CTAs an SM at
-    // order 5; three need at most 168 (707 us of phase 2 down to 540)
+    // order 5; three need at most 168 (phase 2 of the 64-net window 707 us with
+    // two, 540 with three, 490 with the longest boxes first)
     static constexpr int kMinCtas = NS == 128 ? 3 : NS < 128 ? 4 : 1;
 };
 template <int NT, int NS>
