@@ -36,7 +36,7 @@ struct DevPlan {
     const int64_t* m2l_off;
     const int32_t* m2l_src;
     const int32_t* m2l_slot;
-    const double* m2l_K;      // 343 n3 x n3 (FP64 table)
+    const double* m2l_K;      // 343 n3 x n3 (FP64 table; null where the factored form runs)
     const double* leaf_ctr;   // 3 per leaf: box centre
     const int32_t* leaf_of;   // per panel: its leaf
     double leaf_half;

@@ -29,8 +29,7 @@ namespace gpx {
 
 struct DevM2L {
     int n = 0, mode = 0;
-    DBuf<double> K;   // FP64 operators
-    DBuf<double> U, Vt;  // low-rank factors (compressed mode), stride n3
+    DBuf<double> K;   // FP64 operators, for the dense form: only where the factored one does not exist
     DBuf<double> Ut64, Vt64;  // factored-M2L tables: Vt rows and transposed U rows, 343 x 32 x ns
     DBuf<float> Ut32, Vt32;
     bool factored_ok = false;
@@ -133,11 +132,6 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
     d->n = n;
     d->mode = mode;
     d->rank = host.rank;
-    d->K.upload(host.K, stream);
-    if (mode == GPX_M2L_COMPRESSED) {
-        d->U.upload(host.U, stream);
-        d->Vt.upload(host.Vt, stream);
-    }
     d->d_rank.upload(host.rank, stream);
     for (int32_t r : host.rank) d->max_rank = std::max(d->max_rank, (int)r);
     if (mode == GPX_M2L_COMPRESSED && d->max_rank <= kFacMaxRank) {
@@ -163,6 +157,8 @@ std::shared_ptr<DevM2L> get_m2l(Ctx& ctx, int n, int mode) {
             d->Vt32.upload(vt32, stream);
         }
         d->factored_ok = true;
+    } else {
+        d->K.upload(host.K, stream);
     }
     if (n == 4 || n == 5) {
         // TF32-rounded (nearest, ties away) operators for the tensor-core M2L,
