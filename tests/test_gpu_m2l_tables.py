@@ -1,5 +1,6 @@
 """The device M2L tables a context keeps: what a first call of an order uploads
-beyond a second one."""
+beyond a second one, and the tables the workers of a batch share."""
+import numpy as np
 import pytest
 
 from gpurify_b200 import _lib, layouts
@@ -33,3 +34,27 @@ def test_first_call_uploads_only_tables_some_kernel_reads(order):
     finally:
         ctx.close()
     assert up[0] - up[1] <= tables
+
+
+@pytest.mark.parametrize("order", [5, 6])
+def test_batch_on_a_fresh_context_equals_separate_solves(order):
+    """Eight workers meet no table of the order: one builds it while the others
+    wait, and with mixed_m2l 3 one of them adds the shared basis to the table
+    the others already hold.  Window by window the matrices have the bits of
+    separate calls on a context of their own."""
+    probs = [panels(n, 8.0, 7 + n) for n in (2, 3, 4, 5, 3, 4, 2, 5)]
+    kw = dict(order=order, max_level=3, dense_below=-1, precision=_lib.PREC_MIXED, mixed_m2l=3, far_quad=1, precond=1)
+    for _ in range(2):
+        ctx = _lib.Context(0)
+        try:
+            res = ctx.cap_solve_batched(probs, batch_streams=8, **kw)
+        finally:
+            ctx.close()
+        one = _lib.Context(0)
+        try:
+            for (v, c, nc), (C, rep) in zip(probs, res):
+                C1, rep1 = one.cap_solve(v, c, nc, **kw)
+                assert rep["m2l_pairs"] > 0 and rep["converged"] == 1 and rep["iterations"] == rep1["iterations"]
+                assert np.array_equal(C, C1)
+        finally:
+            one.close()

@@ -101,3 +101,83 @@ def test_capacitance_sums_over_row_slices(ctx, orc, n):
     assert rep["dense"] == 1
     ref = orc.cap_dense(verts, cond, 3)
     assert np.abs(C - ref).max() / np.abs(ref).max() < 1e-9
+
+
+@pytest.mark.parametrize("tol,above", [(1e-7, False), (1e-8, True)])
+def test_back_substitution_of_a_long_cycle(ctx, tol, above):
+    """A restart may be longer than the 1,024 columns of H whose solution the
+    back substitution keeps in shared memory; longer ones are solved in global
+    memory.  Nearly touching plates take some 980 and 1,080 steps in one cycle;
+    the residual is formed from the solution, so that the cycle converges only
+    with the right one."""
+    k = np.arange(1300)
+    x, y, gap = (k % 37) * 1.2e-6, (k // 37) * 1.2e-6, 1e-6 * 10 ** np.linspace(-4.2, -0.7, 1300)
+    verts = np.concatenate([np.stack([x, y, z, x + 1e-6, y, z, x + 1e-6, y + 1e-6, z, x, y + 1e-6, z], axis=1)
+                            for z in (0 * gap, gap)])
+    cond = np.random.default_rng(0).integers(0, 2, 2600).astype(np.int32)
+    _, rep = ctx.cap_solve(verts, cond, 2, tol=tol, restart=1400, max_restarts=1, max_level=2, dense_below=-1)
+    assert rep["converged"] == 1 and rep["max_rel_residual"] <= tol and rep["restart_used"] == 1400
+    assert (rep["iterations"] > 1024) == above
+
+
+def _squares(n, seed):
+    """n separate horizontal squares, one per micron of a 3-D grid, in random order."""
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(n ** (1 / 3)))
+    cell = rng.permutation(side**3)[:n]
+    x, y, z = (1e-6 * (cell // d % side) for d in (1, side, side * side))
+    s = rng.uniform(0.05, 0.35, n) * 1e-6
+    return np.stack([x, y, z, x + s, y, z, x + s, y + s, z, x, y + s, z], axis=1)
+
+
+# work items of the near assembly: below 256 they are split over 64 blocks of
+# their sources, above 16,384 not at all
+@pytest.mark.parametrize("n,depth", [(1, 1), (65, 1), (4097, 1), (2500, 3), (20000, 6)])
+def test_near_assembly_at_item_splits(ctx, orc, n, depth):
+    v = _squares(n, n)
+    sig = np.random.default_rng(n).standard_normal((n, 1))
+    far = dict(order=2, max_level=depth, dense_below=-1) if depth > 1 else dict(dense_below=2**31 - 1)
+    y, rep = ctx.operator_apply(v, sig, **far)
+    if depth > 1:
+        yo, _ = orc.fmm_cap_apply(v, sig[:, 0], 2, depth)
+    else:  # the library's own kernel for single potentials: the oracle's form of the integral cancels at far pairs
+        yo = ctx.potential_matrix(v, v.reshape(n, 4, 3).mean(axis=1)) @ sig[:, 0]
+    assert rep["dense"] == (depth == 1)
+    assert np.linalg.norm(y[:, 0] - yo) / np.linalg.norm(yo) < 1e-11
+
+
+@pytest.mark.parametrize("n,depth", [(64, 1), (65, 1), (300, 1), (2500, 3), (18000, 6)])
+def test_near_derivative_at_item_splits(ctx, n, depth):
+    """Capacitance scales with length: along the velocity field x (panels that
+    grow) dC = C, and along a common translation dC = 0.  With every pair
+    exact that holds to the solver's tolerance of 1e-10; with a far field, whose
+    boxes do not move, to its truncation, about 1e-3 at order 5 of panels a
+    leaf's size (a block of sources left out is an error of its share of C)."""
+    v = _squares(n, n)
+    cond = np.where(v[:, 0] > np.median(v[:, 0]), 1, 0).astype(np.int32)
+    vel = np.stack([v * 1e6, np.tile([1.0, -2.0, 0.5], (n, 4))])  # per um; translation
+    far = dict(order=5, max_level=depth, dense_below=-1, far_quad=1) if depth > 1 else dict(dense_below=2**31 - 1)
+    C, dC, rep = ctx.cap_sensitivity(v, cond, 2, vel, tol=1e-10, **far)
+    assert rep["dense"] == (depth == 1) and rep["converged"] == 1
+    bar = 5e-3 if depth > 1 else 1e-8
+    assert np.abs(dC[0] * 1e-6 - C).max() < bar * np.abs(C).max()
+    assert np.abs(dC[1] * 1e-6).max() < bar * np.abs(C).max()
+
+
+@pytest.mark.parametrize("order,m2l", [(4, 1), (4, 2), (5, 1), (5, 2), (5, 3), (6, 1), (6, 3)])
+@pytest.mark.parametrize("cols", [4, 16, 20, 32])
+def test_mixed_apply_of_few_columns_close_to_fp64(ctx, order, m2l, cols):
+    """The FP32 operator at 16 and 32 rows per box, column by column against
+    FP64, at the bars of the 64-column tests: 1e-3 with TF32 products, 2e-3 in
+    the shared basis, 5e-5 with the FP32 near apply and the factored M2L."""
+    lay = layouts.two_wires(length_nm=6000)
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, mesh_max_edge_m=0.3e-6,
+                             max_panels=-1)
+    sig = np.random.default_rng(order + cols).standard_normal((len(p["verts"]), cols))
+    kw = dict(order=order, max_level=4, dense_below=-1)
+    ref, rep = ctx.operator_apply(p["verts"], sig, **kw)
+    y, _ = ctx.operator_apply(p["verts"], sig, precision=_lib.PREC_MIXED, mixed_m2l=m2l, mixed_near=1 if m2l == 1 else 0,
+                              **kw)
+    assert rep["m2l_pairs"] > 0
+    err = np.linalg.norm(y - ref, axis=0) / np.linalg.norm(ref, axis=0)
+    assert err.max() < {1: 5e-5, 2: 1e-3, 3: 2e-3}[m2l]
