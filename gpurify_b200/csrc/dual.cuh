@@ -21,7 +21,6 @@ struct Dual {
         return {s, s > 0.0 ? a.d / (2.0 * s) : 0.0};
     }
     friend __host__ __device__ inline Dual log1p(Dual a) { return {::log1p(a.v), a.d / (1.0 + a.v)}; }
-    friend __host__ __device__ inline Dual atan(Dual a) { return {::atan(a.v), a.d / (1.0 + a.v * a.v)}; }
     friend __host__ __device__ inline Dual fabs(Dual a) { return a.v < 0.0 ? Dual{-a.v, -a.d} : a; }
 };
 

@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
     uint8_t* sbase = smem_raw + (base - raw);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sbase + 2 * kStage);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    __shared__ int s_bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int it = blockIdx.x;
     const int t = p.item_leaf[it], r0 = p.item_row0[it];
@@ -115,7 +114,6 @@ __global__ void __launch_bounds__(kThreads) k_l2p_tc(DevPlan p, const float* __r
     if (tid == 0) {
         for (int k = 0; k < 2; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[k])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_bad = 0;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),

@@ -112,7 +112,6 @@ __global__ void __launch_bounds__(kThreads) k_rows_tc(const float* __restrict__ 
     uint8_t* sbase = smem_raw + (base - raw);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sbase + 2 * kStage);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    __shared__ int s_bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t r0 = (int64_t)blockIdx.x * kRows;
     const int col0 = blockIdx.y * 64;
@@ -120,7 +119,6 @@ __global__ void __launch_bounds__(kThreads) k_rows_tc(const float* __restrict__ 
     if (tid == 0) {
         for (int k = 0; k < 2; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[k])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_bad = 0;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
