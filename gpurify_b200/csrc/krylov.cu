@@ -383,6 +383,7 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 
 }  // namespace
 
+// Row blocks of the column reductions: fixed, not by the device's SMs, since they set the order of every sum.
 int reduce_blocks_for(int64_t N) { return (int)std::min<int64_t>(592, std::max<int64_t>(1, N / 64)); }
 
 void DotScratch::alloc(int64_t N, int max_vectors, int R, cudaStream_t s) {
@@ -394,8 +395,8 @@ void DotScratch::alloc(int64_t N, int max_vectors, int R, cudaStream_t s) {
 
 // Blocks y of a dot of ni vectors: as many as bring the grid to four blocks an
 // SM, at most one per eight vectors.
-static int dot_grid_y(int nblk, int ni) {
-    return std::max(1, std::min({(ni + 7) / 8, 592 / nblk, DotScratch::kMaxY}));
+static int dot_grid_y(const Ctx& c, int nblk, int ni) {
+    return std::max(1, std::min({(ni + 7) / 8, 4 * c.sm_count / nblk, DotScratch::kMaxY}));
 }
 
 // Up to 32 row blocks (about 2,000 rows) the last block of a y adds the
@@ -411,7 +412,7 @@ void multidot_t(Ctx& c, const TA* A, int64_t strideA, int ni, const double* B, i
     const bool fuse = d.nblk <= kFuseBlocks;
     {
         KTimer t(c, tag, ((double)sizeof(TA) * ni + 8.0) * (double)N * R, 2.0 * ni * (double)N * R);
-        k_multidot<<<dim3(d.nblk, dot_grid_y(d.nblk, ni)), kRedThreads, 0, c.stream>>>(
+        k_multidot<<<dim3(d.nblk, dot_grid_y(c, d.nblk, ni)), kRedThreads, 0, c.stream>>>(
             A, strideA, ni, kdev, B, N, R, d.partial.p, fuse ? d.ctr.p : nullptr, out, root ? 1 : 0);
         GPX_LAUNCH_CHECK();
     }

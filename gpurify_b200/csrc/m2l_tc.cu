@@ -266,7 +266,7 @@ void launch_rb(Ctx& c, const TcLevel& lv, const float* E, int64_t nbox, float* L
               float scale, const double* box_scale, int* err) {
     using Cf = TcCfg<NS, RB>;
     const int64_t ctas = (int64_t)lv.nitems * (R / RB);
-    const int per_sm = (int)std::min<int64_t>(4, (ctas + 147) / 148);
+    const int per_sm = (int)std::min<int64_t>(4, (ctas + c.sm_count - 1) / c.sm_count);
     const int room = 227 * 1024 / per_sm - 1024;
     int S = Cf::kMaxStages;
     while (S > 2 && (int)Cf::smem(S) > room) --S;

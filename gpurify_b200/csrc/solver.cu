@@ -740,7 +740,7 @@ struct Operator {
         // run of 512 stages the source's expansion once for 16 blocks of 32
         // columns; where that would leave SMs idle (fewer than eight CTAs
         // each), shorter runs spread the work.
-        const int64_t cap = scol[np] / kFacItemCols >= 8 * 148 ? kFacItemCols : 128;
+        const int64_t cap = scol[np] / kFacItemCols >= 8 * ctx.sm_count ? kFacItemCols : 128;
         std::vector<FacItem> items;
         for (int64_t b = 0; b < nb; ++b)
             for (int64_t p = first[b]; p < first[b + 1];) {
