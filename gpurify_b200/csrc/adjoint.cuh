@@ -14,10 +14,11 @@ void launch_panel_dprops(Ctx& c, const DevPlan& p, const double* V, double* dcen
 // blocks along V (sources) and dcent (collocation points).
 void launch_near_assemble_dual(Ctx& c, const DevPlan& p, int64_t nnz, const double* V, const double* dcent,
                                double* dP, double coef);
-// dW (N x n3) = derivative of (area * far-field source weights) along V.
+// dW (N x ns: node stride, padding written as zero) = derivative of (area *
+// far-field source weights) along V.
 void launch_dsrc_weights(Ctx& c, const DevPlan& p, int quad, const double* V, double* dW);
-// out (N x n3) = Chebyshev weights of each centroid in its leaf (dcent null)
-// or their derivative along dcent.
+// out (N x ns: node stride, padding written as zero) = Chebyshev weights of
+// each centroid in its leaf (dcent null) or their derivative along dcent.
 void launch_centroid_weights(Ctx& c, const DevPlan& p, const double* dcent, double* out);
 // PT = transposed near blocks of P (same block layout).
 void launch_near_transpose(Ctx& c, const DevPlan& p, const int32_t* near_rev, const int32_t* near_pre,

@@ -26,8 +26,8 @@ struct FarWeights {
 
 // Y += coef * far-field potential of X (N x R, type T).  Expansions E and L:
 // nbox x Rb x ns each (Rb >= R rows per box, node stride ns); E is written in
-// full by P2M and M2M (zero padding rows and nodes), L is zeroed here.  M2L is
-// supplied per level.
+// full by P2M and M2M (zero padding rows and nodes), L is zeroed here unless
+// l_written.  M2L is supplied per level.
 // m2l_all_levels: the M2L callback runs once for every level (level -1,
 // first box of level 2, box count of levels 2..L) instead of once per level.
 // Inputs of the tensor-core P2M (p2m_tc.cu): the source weights (area
@@ -49,8 +49,8 @@ void launch_far_field(Ctx& c, const DevPlan& p, const FarLaunch& f, const T* X, 
                       int R, int Rb, T* E, T* L, double coef, const M2LLevelFn<T>& m2l, bool m2l_all_levels = false,
                       const P2MSplit* p2m_tc = nullptr, bool l_written = false);
 // l_written: the M2L callback overwrites every local-expansion row of levels
-// 2 and deeper (the shared-basis decompression does), and L's rows of levels
-// 0 and 1 are zero: L is then not cleared before the M2L.
+// 2 and deeper (the factored form and the shared-basis decompression do; no
+// kernel reads those of levels 0 and 1): L is then not cleared before the M2L.
 // Whi / Wlo [N][128] = TF32 split of (area if mul_area) x W[N][ns] (ns <= 128).
 void launch_split_weights(Ctx& c, const double* W, int ns, const double* area, bool mul_area, float* Whi, float* Wlo,
                           int64_t N);
@@ -113,8 +113,10 @@ void launch_m2l_fac<float>(Ctx& c, const FacM2L<float>& f, int b0, int nb, float
 // the union of their offsets and leave fewer, longer items: at 16 columns an
 // apply of a 21,195-panel bus (depth 5) takes 66 us with two or four boxes and
 // 158 us with eight, the 64-net window 71, 48 and 64 us; at 32 columns the
-// window takes 75 us with two and 66 us with four.  Four boxes of 64 with two
-// accumulators measured slower on the window (0.385 against 0.309 ms).
+// window takes 75 us with two and 66 us with four (64 x 64 cores all of them).
+// At 64 columns two boxes fill the accumulator's 128 rows; four with two
+// accumulators were slower when tiles were copied with cp.async (full order-5
+// operators, node stride 128: 385 against 309 us, 233 with two boxes now).
 constexpr int tc_group(int Rb) { return Rb >= 64 ? 2 : 4; }
 struct TcLevel {
     int nitems = 0;

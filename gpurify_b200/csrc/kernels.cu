@@ -1,9 +1,8 @@
 // FP64 kernels of the potential-coefficient operator.
 //
 //  * near-field assembly: closed-form Wilton integral of 1/|p - r'| over each
-//    source panel (integrals/panel.rs:147-208), one CTA per target leaf, one
-//    warp per group of target rows, lanes over source panels staged in shared
-//    memory (source geometry is prepared once per lane and reused across rows);
+//    source panel (integrals/panel.rs:147-208), CTAs over <= 64 rows of a target
+//    leaf and a share of its sources, whose prepared panels lie in shared memory;
 //  * near-field apply: dense leaf blocks times R right-hand sides on FP64
 //    matrix instructions (FP32 on the CUDA cores);
 //  * far field: Chebyshev P2M, M2M, M2L, L2L, L2P (fmm/bbfmm.rs:209-448).
@@ -29,6 +28,9 @@ constexpr int kAsmTile = 64;
 // Bound: the FP64 pipe (about 1,900 multiply-add slots per entry: 4 edges of 2
 // square roots, log1p, 2 arc tangents and their divisions), at about half its
 // rate, since each entry is one chain of them.  147.8 M entries 12.9 -> 9.8 ms.
+// Three CTAs leave 80 registers a thread, two fewer than the kernel would take:
+// 28 bytes of spill stores and 36 of loads.  143.2 M entries take 9.5 ms so, and
+// 10.8 with two CTAs and no spills.
 __global__ void __launch_bounds__(kAsmThreads, 3) k_near_assemble(DevPlan p, double* __restrict__ P, double coef) {
     const int it = p.item_order[blockIdx.x], t = p.item_leaf[it], r0 = p.item_row0[it];
     const int64_t tb = p.leaf_begin[t];

@@ -282,7 +282,8 @@ __global__ void k_givens_loop(GmresDev g, cudaGraphConditionalHandle h, int32_t*
 // as fit, and one of them runs the chain of multiply-adds, which is all that
 // is serial, in the order of the rows' columns.  A thread per column with
 // everything in global memory waited for each entry: 58 columns of H 212 us.
-// Columns past kTriCols (longer than a restart) are read from global memory.
+// kTriCols is what the shared memory holds of y.  A restart has no such bound:
+// a longer cycle is solved by one thread with everything in global memory.
 constexpr int kTriThreads = 128, kTriBuf = 4096, kTriCols = 1024;
 __global__ void __launch_bounds__(kTriThreads) k_trisolve(GmresDev g) {
     __shared__ double s_h[kTriBuf], s_y[kTriCols];

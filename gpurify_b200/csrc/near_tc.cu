@@ -1,10 +1,10 @@
 // Near-field apply on the 5th-generation tensor cores (tcgen05, kind::tf32,
 // FP32 accumulation in tensor memory) for the mixed path:
-//     Y[rows of item][rc : rc+64] = P_t[rows][0:S] X[near sources of t][rc : rc+64]
+//     Y[rows of item][rc : rc+NT] = P_t[rows][0:S] X[near sources of t][rc : rc+NT]
 // With 64 right-hand sides the near product does 32 flop per streamed FP32
 // matrix byte, above what the FP32 CUDA cores sustain per HBM byte, so on the
-// CUDA cores it is compute bound; on the tensor cores it is bound by streaming
-// the near blocks from HBM.
+// CUDA cores it is compute bound; on the tensor cores the gathers of X from L2
+// and the stream of the near blocks from HBM bound it (figures below).
 //
 // One CTA per (work item = target leaf and <= 128 of its rows, NT-wide chunk
 // of right-hand sides, NT = 16, 32 or 64), D = 128 x NT FP32 in TMEM (16
@@ -15,8 +15,8 @@
 //     HBM;
 //   B_hi, B_lo (32 x NT each, MN-major, 128-byte swizzle on a 32-byte base) = the 32 source
 //     panels' rows of X_hi = tf32(x) and X_lo = tf32(x - x_hi), gathered from
-//     the L2-resident split copies written by k_split_tf32.  A source row of
-//     X is 64 contiguous FP32 values, which is exactly one K row of an
+//     the L2-resident split copies written by k_split_tf32.  A source row's
+//     NT columns are contiguous FP32 values, which is exactly one K row of an
 //     MN-major tile, so the gather is a plain copy: no transpose and no
 //     per-slice register work.
 // What bounds it: with 28 rows per leaf (bus) or 55 (window) the gather of X (8 NT bytes
@@ -24,7 +24,8 @@
 // an apply of the window, 11 TB/s from L2).  So the copies follow NT (a 12-column apply
 // of a 21,195-panel bus: 97 us with 64 columns copied, 68 with 16, and four
 // stages), and four neighbouring threads read 64 contiguous bytes, whole
-// sectors (64-net window, 64 columns: 228 -> 202 us).  One arrival per warp
+// sectors (64-net window, 64 columns: 228 -> 202 us; at 69,253 panels 184 us,
+// 693 MB of DRAM traffic, half of the L2's and of the DRAM's throughput each).  One arrival per warp
 // after a lagging wait for its copies, in place of one per thread when they
 // land, was slower (300 and 104 us).
 // D += A B_hi + A B_lo represents X to about 2^-21, so the operator stays
