@@ -435,15 +435,15 @@ def time_solves(ctx, verts, cond, ncond, solve_kw, steps, warmup, stream, dist, 
 
 
 # DRAM bytes per launch measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum, one --set full capture of two launches of each
-# kernel on this bench window, cold cache) divided by the launch's
-# algorithmic bytes as this bench counts them (near apply: 4 B per stored
-# near entry plus 16 B per panel and right-hand side; M2L: each box's
-# expansion read once and its local expansion written once).  bench scales
-# the ratio by the algorithmic bytes of the launches it times.
-TRAFFIC_PER_ALGO_BYTE = {"near_apply": 1.163, "m2l": 0.968,
+# dram__bytes_write.sum, one launch of each kernel in an operator apply of this
+# bench window with 64 columns, cold cache) divided by the launch's algorithmic
+# bytes as this bench counts them (near apply: 4 B per stored near entry plus
+# 16 B per panel and right-hand side; M2L: each box's expansion read once and
+# its local expansion written once).  bench scales the ratio by the algorithmic
+# bytes of the launches it times.
+TRAFFIC_PER_ALGO_BYTE = {"near_apply": 1.158, "m2l": 0.811,
                          # shared-basis M2L: compress + 64 x 64 cores + decompress per apply
-                         "m2l_shared": 1.151}
+                         "m2l_shared": 1.166}
 
 
 def roofline_of(ks, ms_total, m2l_engine, shared_m2l=False):
