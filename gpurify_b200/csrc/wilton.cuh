@@ -73,21 +73,49 @@ __device__ __forceinline__ void prep_source_t(const S* g, SrcPanelT<S>& s) {
 // stable form needs no fallback, and a point on the edge line (r0 = 0)
 // contributes 0 exactly as the reference's fallback does.
 //
-// The arc-tangent term of one edge, ad (atan(tp) - atan(tm)).
-__device__ __forceinline__ double edge_angle(double ad, double tp, double tm) { return ad * (::atan(tp) - ::atan(tm)); }
-// On dual numbers the derivative alone (wilton_t<Dual> is used for nothing
-// else): the angle itself counts only where the height over the panel changes.
-__device__ __forceinline__ Dual edge_angle(Dual ad, Dual tp, Dual tm) {
+// The logarithm's term of one edge, pp log(num / den).
+__device__ __forceinline__ double edge_log(double pp, double sp, double sm, double rp, double rm, double r0sq,
+                                           double el) {
+    const double num = sp >= 0.0 ? rp + sp : r0sq / (rp - sp);
+    const double den = sm >= 0.0 ? rm + sm : r0sq / (rm - sm);
+    return num > 0.0 && den > 0.0 ? pp * ::log1p(el * (num + den) / ((rp + rm) * den)) : 0.0;
+}
+// The arc-tangent term of one edge, ad (atan(tp) - atan(tm)), which is zero
+// over the edge's line (pp = 0) and in the panel's plane (ad = 0).
+__device__ __forceinline__ double edge_angle(double ad, double pp, double sp, double sm, double rp, double rm,
+                                             double r0sq) {
+    if (!(ad > 0.0 && pp != 0.0)) return 0.0;
+    const double tp = (pp * sp) / (r0sq + ad * rp), tm = (pp * sm) / (r0sq + ad * rm);
+    return ad * (::atan(tp) - ::atan(tm));
+}
+
+// On dual numbers (wilton_t<Dual> serves the derivative and nothing else) both
+// terms have one where their value is zero.  Over the edge's line pp still
+// changes, and points over it are common: panels of one grid share their lines.
+// The logarithm then stays finite before and behind the edge; behind it
+// (sp, sm < 0) num / den = (rm - sm) / (rp - sp), without the r0^2 both lose.
+// On the edge itself the derivative diverges and counts as zero.
+template <class P>
+__device__ __forceinline__ Dual edge_log(Dual pp, Dual sp, Dual sm, Dual rp, Dual rm, Dual r0sq, P el) {
+    const bool behind = sp < 0.0 && sm < 0.0;
+    const Dual num = behind ? rm - sm : sp >= 0.0 ? rp + sp : r0sq / (rp - sp);
+    const Dual den = behind ? rp - sp : sm >= 0.0 ? rm + sm : r0sq / (rm - sm);
+    return num > 0.0 && den > 0.0 ? pp * log1p(el * (num + den) / ((rp + rm) * den)) : Dual(0.0);
+}
+// In the panel's plane the term is even in the height, so its derivative is
+// zero; over the plane the angle itself counts only where the height changes.
+__device__ __forceinline__ Dual edge_angle(Dual ad, Dual pp, Dual sp, Dual sm, Dual rp, Dual rm, Dual r0sq) {
+    if (!(ad > 0.0)) return 0.0;
+    const Dual tp = (pp * sp) / (r0sq + ad * rp), tm = (pp * sm) / (r0sq + ad * rm);
     const double angle = ad.d != 0.0 ? ::atan(tp.v) - ::atan(tm.v) : 0.0;
-    const double pp = 1.0 + tp.v * tp.v, mm = 1.0 + tm.v * tm.v;
-    return {0.0, ad.d * angle + ad.v * ((tp.d * mm - tm.d * pp) / (pp * mm))};
+    const double tpp = 1.0 + tp.v * tp.v, tmm = 1.0 + tm.v * tm.v;
+    return {0.0, ad.d * angle + ad.v * ((tp.d * tmm - tm.d * tpp) / (tpp * tmm))};
 }
 
 // P: scalar of the panel, S: scalar of the point (and of the result).
 template <class S, class P = S>
 __device__ __forceinline__ S wilton_t(const SrcPanelT<P>& s, S px, S py, S pz) {
     using ::fabs;
-    using ::log1p;
     using ::sqrt;
     const S d = (px - s.v[0][0]) * s.n[0] + (py - s.v[0][1]) * s.n[1] + (pz - s.v[0][2]) * s.n[2];
     const S p0[3] = {px - s.n[0] * d, py - s.n[1] * d, pz - s.n[2] * d};
@@ -106,17 +134,7 @@ __device__ __forceinline__ S wilton_t(const SrcPanelT<P>& s, S px, S py, S pz) {
         const S r0sq = pp * pp + d * d;
         const S rp = sqrt(sp * sp + r0sq);
         const S rm = sqrt(sm * sm + r0sq);
-        const S num = sp >= 0.0 ? rp + sp : r0sq / (rp - sp);
-        const S den = sm >= 0.0 ? rm + sm : r0sq / (rm - sm);
-        S lt = 0.0;
-        if (num > 0.0 && den > 0.0) lt = pp * log1p(s.el[i] * (num + den) / ((rp + rm) * den));
-        S at = 0.0;
-        if (ad > 0.0 && pp != 0.0) {
-            const S tp = (pp * sp) / (r0sq + ad * rp);
-            const S tm = (pp * sm) / (r0sq + ad * rm);
-            at = edge_angle(ad, tp, tm);
-        }
-        total += lt - at;
+        total += edge_log(pp, sp, sm, rp, rm, r0sq, s.el[i]) - edge_angle(ad, pp, sp, sm, rp, rm, r0sq);
     }
     return total;
 }

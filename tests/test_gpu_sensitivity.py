@@ -145,3 +145,18 @@ def test_row_subset_and_chunked_columns(ctx, orc):
     assert err < 1e-5, err
     with pytest.raises(_lib.GpxError, match="gradient row"):
         ctx.cap_sensitivity(verts, cond, nc, V, grad_rows=[5, 5], **kw)
+
+
+@pytest.mark.parametrize("param", [("width", 1), ("spacing", 0)])
+def test_panels_on_one_grid_match_oracle_differences(ctx, orc, param):
+    """Panels of a window's mesh share grid lines: many collocation points lie
+    straight over the line of another panel's edge, in its plane or not, where
+    the terms of the panel integral are zero and their derivatives are not."""
+    lay = layouts.routing_window(3, 6.0, seed=5, len_um=(0.5, 3.0))
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, max_panels=-1)
+    nc = len(p["nets"]) + 1
+    V = sensitivity.velocity_fields(p["verts"], p["cond"], p["nets"], [param])
+    _, dC, rep = ctx.cap_sensitivity(p["verts"], p["cond"], nc, V, **DENSE)
+    assert rep["dense"] == 1
+    ref = fd(lambda v: orc.cap_dense(v, p["cond"], nc), p["verts"], V[0], 1e-10)
+    assert np.abs(dC[0] - ref).max() / np.abs(ref).max() < 1e-5
