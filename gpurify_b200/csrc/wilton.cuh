@@ -112,14 +112,24 @@ __device__ __forceinline__ Dual edge_angle(Dual ad, Dual pp, Dual sp, Dual sm, D
     return {0.0, ad.d * angle + ad.v * ((tp.d * tmm - tm.d * tpp) / (tpp * tmm))};
 }
 
+// Height of a point at distance d from the panel's plane.  A dual height below
+// the rounding of the coordinates (16 units in their last place) is in the
+// plane: the arc tangents' sum is even in the height, and where the motion
+// bends a panel, so that its own centroid leaves the plane, the sign of a
+// rounding error would decide on a derivative of +-2 pi.
+__device__ __forceinline__ double height(double d, double, double, double) { return ::fabs(d); }
+__device__ __forceinline__ Dual height(Dual d, Dual px, Dual py, Dual pz) {
+    const double ulps = 16.0 * 2.220446049250313e-16;
+    return ::fabs(d.v) <= ulps * (::fabs(px.v) + ::fabs(py.v) + ::fabs(pz.v)) ? Dual(0.0) : fabs(d);
+}
+
 // P: scalar of the panel, S: scalar of the point (and of the result).
 template <class S, class P = S>
 __device__ __forceinline__ S wilton_t(const SrcPanelT<P>& s, S px, S py, S pz) {
-    using ::fabs;
     using ::sqrt;
     const S d = (px - s.v[0][0]) * s.n[0] + (py - s.v[0][1]) * s.n[1] + (pz - s.v[0][2]) * s.n[2];
     const S p0[3] = {px - s.n[0] * d, py - s.n[1] * d, pz - s.n[2] * d};
-    const S ad = fabs(d);
+    const S ad = height(d, px, py, pz);
     S total = 0.0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

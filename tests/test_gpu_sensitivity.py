@@ -160,3 +160,18 @@ def test_panels_on_one_grid_match_oracle_differences(ctx, orc, param):
     assert rep["dense"] == 1
     ref = fd(lambda v: orc.cap_dense(v, p["cond"], nc), p["verts"], V[0], 1e-10)
     assert np.abs(dC[0] - ref).max() / np.abs(ref).max() < 1e-5
+
+
+def test_velocities_that_bend_panels_match_oracle_differences(ctx, orc):
+    """Independent motion of every vertex takes a panel's centroid out of its
+    plane.  The self term is even in that height, a cusp, so its derivative is
+    zero, whatever the rounding error the height starts from.  The central
+    difference at this step is 7e-6 off (it halves with the step until rounding
+    takes over), hence 1e-4."""
+    lay = layouts.routing_window(3, 6.0, seed=5, len_um=(0.5, 3.0))
+    p = _lib.bridge_panelize(lay.store.arrays(), lay.deck.layer_table(), 1.0, lay.net_of_poly, max_panels=-1)
+    nc = len(p["nets"]) + 1
+    V = np.random.default_rng(0).standard_normal((1,) + p["verts"].shape)
+    _, dC, _ = ctx.cap_sensitivity(p["verts"], p["cond"], nc, V, **DENSE)
+    ref = fd(lambda v: orc.cap_dense(v, p["cond"], nc), p["verts"], V[0], 1e-12)
+    assert np.abs(dC[0] - ref).max() / np.abs(ref).max() < 1e-4
