@@ -95,8 +95,8 @@ __global__ void k_panel_dprops(DevPlan p, const double* __restrict__ V, double* 
 // on dual numbers throughout, 32 with constant panels, 18 with the panels in
 // shared memory (255 registers before, one CTA an SM) and the items split.
 // Three CTAs an SM leave 80 registers of the 126 it would take (148 bytes of
-// spill stores, 252 of loads): four derivatives of 52.4 M entries take 19.5 ms
-// so, and 20.6 with two CTAs and no spills.
+// spill stores, 252 of loads): four derivatives of 52.4 M entries take 18.9 ms
+// so, and 20.3 with two CTAs and no spills.
 constexpr int kDThreads = 256;
 constexpr int kDTile = 64;
 __global__ void __launch_bounds__(kDThreads, 3) k_near_assemble_dual(DevPlan p, const double* __restrict__ V,
